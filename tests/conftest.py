@@ -33,7 +33,7 @@ def golden():
 @pytest.fixture(scope="session")
 def reference_available():
     from refsupport import REF_SRC, ORACLE_DIR
-    return REF_SRC.exists() or (ORACLE_DIR / "_ref" / "libref_harness3d.so").exists()
+    return (REF_SRC / "src").exists() or (ORACLE_DIR / "_ref" / "libref_harness3d.so").exists()
 
 
 @pytest.fixture(scope="session")
@@ -44,3 +44,21 @@ def rgpu_lib():
     if not rgpu.LIB_PATH.exists():
         rgbuild.build()
     return rgpu.lib()
+
+
+def _skip_without_reference(item):
+    from refsupport import ReferenceUnavailable
+    try:
+        return (yield)
+    except ReferenceUnavailable as e:
+        pytest.skip(str(e))
+
+
+@pytest.hookimpl(wrapper=True)
+def pytest_runtest_setup(item):
+    return (yield from _skip_without_reference(item))
+
+
+@pytest.hookimpl(wrapper=True)
+def pytest_runtest_call(item):
+    return (yield from _skip_without_reference(item))

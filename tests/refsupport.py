@@ -53,7 +53,7 @@ def ensure_built(target):
            "dropin": ORACLE_DIR / "_ref" / "libref_harness_gpu3d.so"}[target]
     if lib.exists():
         return True
-    if target in ("ref", "dropin") and not REF_SRC.exists():
+    if target in ("ref", "dropin") and not (REF_SRC / "src").exists():
         return False
     subprocess.run(["make", "-s", "-C", str(ORACLE_DIR), target, f"REF={REF_SRC}", "-j8"], check=True)
     return lib.exists()
@@ -91,13 +91,18 @@ class GridArrays:
         return (self.ncoarse + (ic[None, :] - 1) * self.ngridmax + octs[:, None]).reshape(-1)
 
 
+class ReferenceUnavailable(RuntimeError):
+    """Neither the reference's sources nor a harness built from them are here (conftest.py skips the test)."""
+
+
 class RefHarness:
     """The reference driven through its own API.  variant="gpu" loads the
     drop-in build whose HydroSolver is the GpuHydroSolver patch."""
 
     def __init__(self, ndim, variant="cpu"):
         target = "dropin" if variant == "gpu" else "ref"
-        assert ensure_built(target), "reference sources unavailable"
+        if not ensure_built(target):
+            raise ReferenceUnavailable("reference sources not present")
         self.ndim = ndim
         name = f"libref_harness_gpu{ndim}d.so" if variant == "gpu" else f"libref_harness{ndim}d.so"
         self.lib = C.CDLL(str(ORACLE_DIR / "_ref" / name))

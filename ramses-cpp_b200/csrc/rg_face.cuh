@@ -7,6 +7,7 @@
 // boundary (:130-145) branch, and the Riemann solver selected at :456-461.
 #pragma once
 
+#include "rg_fast.cuh"
 #include "rg_internal.cuh"
 #include "rg_mlp.cuh"
 #include "rg_physics.cuh"
@@ -18,6 +19,11 @@ struct StepK {
     int slope_type, interpol_type, interpol_var, exact_niter;
     double exact_tol;
     const float* mlp;  // learned Newton start of the exact solver, or nullptr
+    // branch-free forms (rg_fast.cuh): usable with these slope and
+    // interpolation types and this gamma; their limiters and gas constants
+    int fast;
+    Limiter own, ghost;
+    FastGas gas;
 };
 
 __device__ __forceinline__ int cell_of(const TreeView& T, const PlanView& P, int p) {
@@ -90,26 +96,11 @@ __device__ __forceinline__ void ghost_trace(const double* qc, const double* ql, 
 
 // Ghost face state of the 1D build (HydroSolver.cpp:219-356): the coarse
 // neighbour's child states, then a slope_type slope against the active cell.
-__device__ __forceinline__ void ghost_1d(const double* __restrict__ uold, size_t ncell, const TreeView& T, int n, int nl, int nr,
-                         int side, const double* q_act, double dt, const DxDiv& D, const StepK& K, double* qm,
-                         double* qp) {
+// uc, ul, ur: conservative states of the neighbour and of its two neighbours.
+__device__ __forceinline__ void ghost_1d_states(const double* uc, const double* ul, const double* ur, int side,
+                                                const double* q_act, double dt, const DxDiv& D, const StepK& K,
+                                                double* qm, double* qp) {
     constexpr int NV = 3;
-    double uc[NV], ul[NV], ur[NV];
-#pragma unroll
-    for (int iv = 0; iv < NV; ++iv) uc[iv] = uold[(size_t)iv * ncell + n - 1];
-    for (int k = 0; k < 2; ++k) {
-        int id = k ? nr : nl;
-        double* uo = k ? ur : ul;
-        if (id > 0) {
-#pragma unroll
-            for (int iv = 0; iv < NV; ++iv) uo[iv] = uold[(size_t)iv * ncell + id - 1];
-        } else {
-#pragma unroll
-            for (int iv = 0; iv < NV; ++iv) uo[iv] = uc[iv];
-            int ib = -id;
-            if (ib > 0 && ib <= T.nbound_type && T.bound_type[ib - 1] == 1) uo[1] *= -1.0;
-        }
-    }
     const double gamma = K.gamma;
     const int ivar = K.interpol_var, itp = K.interpol_type;
     double q1[3][NV];
@@ -186,6 +177,29 @@ __device__ __forceinline__ void ghost_1d(const double* __restrict__ uold, size_t
     trace<1>(qg, dq, dt, D.dx, qm, qp, gamma);
 }
 
+__device__ __forceinline__ void ghost_1d(const double* __restrict__ uold, size_t ncell, const TreeView& T, int n, int nl, int nr,
+                         int side, const double* q_act, double dt, const DxDiv& D, const StepK& K, double* qm,
+                         double* qp) {
+    constexpr int NV = 3;
+    double uc[NV], ul[NV], ur[NV];
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) uc[iv] = uold[(size_t)iv * ncell + n - 1];
+    for (int k = 0; k < 2; ++k) {
+        int id = k ? nr : nl;
+        double* uo = k ? ur : ul;
+        if (id > 0) {
+#pragma unroll
+            for (int iv = 0; iv < NV; ++iv) uo[iv] = uold[(size_t)iv * ncell + id - 1];
+        } else {
+#pragma unroll
+            for (int iv = 0; iv < NV; ++iv) uo[iv] = uc[iv];
+            int ib = -id;
+            if (ib > 0 && ib <= T.nbound_type && T.bound_type[ib - 1] == 1) uo[1] *= -1.0;
+        }
+    }
+    ghost_1d_states(uc, ul, ur, side, q_act, dt, D, K, qm, qp);
+}
+
 // Step values of the box of level cell p (ensemble levels).
 __device__ __forceinline__ void step_of_box(const PlanView& P, int p, double& dt, DxDiv& D) {
     const BoxStep& B = P.boxes[box_of(P, p)];
@@ -203,6 +217,17 @@ __device__ __forceinline__ int riemann(const double* ql, const double* qr, doubl
                                  mlp_guess<NDIM>(K.mlp, ql, qr, K.gamma, K.smallp));
     else solve_llf<NDIM>(ql, qr, f, K.gamma);
     return 0;
+}
+
+// The branch-free solvers; the exact solver iterates, so it has its plain form only.
+template <int NDIM, int RS>
+__device__ __forceinline__ bool riemann_fast(const double* ql, const double* qr, double* f, const StepK& K,
+                                             unsigned& iters) {
+    if constexpr (RS == RG_RIEMANN_HLLC) return hllc_fast<NDIM>(ql, qr, f, K.gas);
+    else if constexpr (RS == RG_RIEMANN_HLL) return hll_fast<NDIM>(ql, qr, f, K.gas);
+    else if constexpr (RS == RG_RIEMANN_LLF) return llf_fast<NDIM>(ql, qr, f, K.gas);
+    iters += riemann<NDIM, RS>(ql, qr, f, K);
+    return true;
 }
 
 // Face state of the neighbour across slot (idim, side), rotated.  Writes the
@@ -299,12 +324,110 @@ __device__ __forceinline__ void neighbour_face(const TreeView& T, const PlanView
 // the next launch (nothing ever waits on another block).
 constexpr int TILE = 32;
 
+// The two fluxes of level cell p (cell id c) along idim in the plain forms, to
+// the scratch.  LEVEL0 as in k_face_tiles.  Returns the Newton updates and
+// adds the Riemann problems solved to *calls.
+template <int NDIM, int RS, bool LEVEL0>
+__device__ __noinline__ unsigned tile_dir_plain(const TreeView& T, const PlanView& P, const double* __restrict__ prim,
+                                                const double* __restrict__ uold, int p, int c, int idim, int kd0,
+                                                int kd1, double dt, const DxDiv& D, const StepK& K, double* flux,
+                                                unsigned* calls) {
+    constexpr int NV = Dims<NDIM>::NV;
+    const size_t ncell = (size_t)T.ncell;
+    const int nc = P.ncells, s0 = 2 * idim;
+    unsigned iters = 0;
+    double qc[NV], qmo[NV], qpo[NV];
+    load_rot<NDIM>(prim, ncell, c, idim, qc);
+    if constexpr (LEVEL0) {
+        double qn[NV], dq0[NV];
+        load_rot<NDIM>(prim, ncell, c, 0, qn);
+#pragma unroll
+        for (int iv = 0; iv < NV; ++iv) dq0[iv] = 0.0;
+        trace<NDIM>(qn, dq0, dt, D.dx, qmo, qpo, K.gamma);
+        rot_swap<NDIM>(qmo, idim);
+        rot_swap<NDIM>(qpo, idim);
+    } else {
+        const int l = P.icn[(size_t)s0 * nc + p], rr = P.icn[(size_t)(s0 + 1) * nc + p];
+        double ql[NV], qr[NV];
+        load_nb_rot<NDIM>(T, prim, ncell, l, idim, qc, ql);
+        load_nb_rot<NDIM>(T, prim, ncell, rr, idim, qc, qr);
+        own_trace<NDIM>(qc, ql, qr, dt, D, K, qmo, qpo);
+    }
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        const int kd = side ? kd1 : kd0;
+        const int s = s0 + side;
+        double f[NV];
+        if ((kd & KIND_MASK) == K_ZERO) {
+#pragma unroll
+            for (int iv = 0; iv < NV; ++iv) f[iv] = 0.0;
+        } else {
+            const int n = P.icn[(size_t)s * nc + p];
+            double qf[NV];
+            neighbour_face<NDIM, LEVEL0 ? 1 : 0>(T, P, prim, uold, ncell, p, c, idim, side, kd, n, qc, nullptr, dt, D, K,
+                                                 qf);
+            if (side == 0) iters += riemann<NDIM, RS>(qf, qpo, f, K);
+            else iters += riemann<NDIM, RS>(qmo, qf, f, K);
+            ++*calls;
+            rot_swap<NDIM>(f, idim);
+        }
+#pragma unroll
+        for (int iv = 0; iv < NV; ++iv) flux[((size_t)s * NV + iv) * nc + p] = f[iv];
+    }
+    return iters;
+}
+
+// The same in the branch-free forms, for cells whose two interfaces are ghost
+// or zero ones; the fluxes in f.  False: not covered, take the plain forms.
+template <int NDIM, int RS, bool POW2>
+__device__ __forceinline__ bool tile_dir_fast(const TreeView& T, const PlanView& P, const double* __restrict__ prim,
+                                              int p, int c, int idim, bool z0, bool z1, double dt, const DxDiv& D,
+                                              const StepK& K, double (*f)[Dims<NDIM>::NV], unsigned& iters) {
+    constexpr int NV = Dims<NDIM>::NV;
+    const size_t ncell = (size_t)T.ncell, nc = (size_t)P.ncells, s0 = 2 * (size_t)idim;
+    const int l = P.icn[s0 * nc + p], r = P.icn[(s0 + 1) * nc + p];
+    // stencils of the two neighbours (the cell itself stands in where no problem is solved)
+    const int ll = z0 ? c : P.stc[(s0 * 2 + 0) * nc + p], lr = z0 ? c : P.stc[(s0 * 2 + 1) * nc + p];
+    const int rl = z1 ? c : P.stc[((s0 + 1) * 2 + 0) * nc + p], rr = z1 ? c : P.stc[((s0 + 1) * 2 + 1) * nc + p];
+    if (min(min(min(l, r), min(ll, lr)), min(rl, rr)) <= 0) return false;
+    double qc[NV], ql[NV], qr[NV], qf[NV], qn[NV], qmo[NV], qpo[NV], qm[NV], qp[NV];
+    load_rot<NDIM>(prim, ncell, c, idim, qc);
+    load_rot<NDIM>(prim, ncell, l, idim, ql);
+    load_rot<NDIM>(prim, ncell, r, idim, qr);
+    const FastStep S = fast_step(dt, D.dx, D.inv), Sc = fast_step(dt, 2.0 * D.dx, 0.5 * D.inv);
+    Check C;
+    load_rot<NDIM>(prim, ncell, ll, idim, qf);
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) qn[iv] = qc[iv];
+    if (lr != c) load_rot<NDIM>(prim, ncell, lr, idim, qn);
+    trace_fast<NDIM, POW2, true, true, false>(ql, qf, qn, K.ghost, Sc, K.gamma, qm, nullptr, C);
+    load_rot<NDIM>(prim, ncell, rr, idim, qf);
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) qn[iv] = qc[iv];
+    if (rl != c) load_rot<NDIM>(prim, ncell, rl, idim, qn);
+    trace_fast<NDIM, POW2, true, false, true>(qr, qn, qf, K.ghost, Sc, K.gamma, nullptr, qp, C);
+    trace_fast<NDIM, POW2, true, true, true>(qc, ql, qr, K.own, S, K.gamma, qmo, qpo, C);
+    const bool ok = C.num_ok() && C.top_ok();
+    unsigned i0 = 0, i1 = 0;
+    const bool a = riemann_fast<NDIM, RS>(qm, qpo, f[0], K, i0), b = riemann_fast<NDIM, RS>(qmo, qp, f[1], K, i1);
+    iters = (z0 ? 0 : i0) + (z1 ? 0 : i1);
+    rot_swap<NDIM>(f[0], idim);
+    rot_swap<NDIM>(f[1], idim);
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) {
+        f[0][iv] = z0 ? 0.0 : f[0][iv];
+        f[1][iv] = z1 ? 0.0 : f[1][iv];
+    }
+    return ok && (a || z0) && (b || z1);
+}
+
 // LEVEL0: instantiated for level 0 (the coarse cells, first-order traces) or
 // for the other levels, so neither instance carries the other's code
 template <int NDIM, int RS, int R, int MINB, bool BOXED, bool LEVEL0 = false>
 __global__ void __launch_bounds__(TILE * NDIM * R, MINB)
-    k_face_tiles(TreeView T, PlanView P, const double* __restrict__ prim, const double* __restrict__ uold,
-                 double* __restrict__ flux, double* __restrict__ fsum, DevStatus* st, StepK K, int batch) {
+    k_face_tiles(const __grid_constant__ TreeView T, const __grid_constant__ PlanView P, const double* __restrict__ prim, const double* __restrict__ uold,
+                 double* __restrict__ flux, double* __restrict__ fsum, DevStatus* st,
+                 const __grid_constant__ StepK K, int batch) {
     constexpr int NV = Dims<NDIM>::NV, NS = Dims<NDIM>::NS;
     __shared__ double sf[R][NS][NV][TILE];
     __shared__ int s_base;
@@ -315,7 +438,7 @@ __global__ void __launch_bounds__(TILE * NDIM * R, MINB)
     const int ntiles = (nc + TILE - 1) / TILE;
     const double dt0 = st->dt;
     const DxDiv D0{st->dx, st->inv_dx, st->dx_pow2 != 0};
-    unsigned long long iters = 0, calls = 0;
+    unsigned iters = 0, calls = 0;
     for (;;) {
         if (threadIdx.x == 0) s_base = (int)atomicAdd(&st->face_next, (unsigned)(batch * R));
         __syncthreads();
@@ -337,47 +460,35 @@ __global__ void __launch_bounds__(TILE * NDIM * R, MINB)
                     double dt = dt0;
                     DxDiv D = D0;
                     if constexpr (BOXED) step_of_box(P, p, dt, D);
-                    double qc[NV], qmo[NV], qpo[NV];
-                    load_rot<NDIM>(prim, ncell, c, idim, qc);
-                    if constexpr (LEVEL0) {
-                        double qn[NV], dq0[NV];
-                        load_rot<NDIM>(prim, ncell, c, 0, qn);
+                    const int k0 = kd0 & KIND_MASK, k1 = kd1 & KIND_MASK;
+                    double f[2][NV];
+                    double* out = flux + (size_t)s0 * NV * nc + p;
+                    unsigned it = 0;
+                    bool ok = false;
+                    if constexpr (NDIM == 3 && !LEVEL0) {
+                        if (K.fast && (k0 == K_GHOST || k0 == K_ZERO) && (k1 == K_GHOST || k1 == K_ZERO) &&
+                            D.dx > 0x1p-60 && D.dx < 0x1p60) {
+                            if (D.pow2)
+                                ok = tile_dir_fast<NDIM, RS, true>(T, P, prim, p, c, idim, k0 == K_ZERO, k1 == K_ZERO, dt,
+                                                                   D, K, f, it);
+                            else
+                                ok = tile_dir_fast<NDIM, RS, false>(T, P, prim, p, c, idim, k0 == K_ZERO, k1 == K_ZERO,
+                                                                    dt, D, K, f, it);
+                        }
+                    }
+                    if (ok) {
 #pragma unroll
-                        for (int iv = 0; iv < NV; ++iv) dq0[iv] = 0.0;
-                        trace<NDIM>(qn, dq0, dt, D.dx, qmo, qpo, K.gamma);
-                        rot_swap<NDIM>(qmo, idim);
-                        rot_swap<NDIM>(qpo, idim);
+                        for (int k = 0; k < 2 * NV; ++k) out[(size_t)k * nc] = f[k / NV][k % NV];
+                        calls += (k0 != K_ZERO) + (k1 != K_ZERO);
                     } else {
-                        const int l = P.icn[(size_t)s0 * nc + p], rr = P.icn[(size_t)(s0 + 1) * nc + p];
-                        double ql[NV], qr[NV];
-                        load_nb_rot<NDIM>(T, prim, ncell, l, idim, qc, ql);
-                        load_nb_rot<NDIM>(T, prim, ncell, rr, idim, qc, qr);
-                        own_trace<NDIM>(qc, ql, qr, dt, D, K, qmo, qpo);
+                        it = tile_dir_plain<NDIM, RS, LEVEL0>(T, P, prim, uold, p, c, idim, kd0, kd1, dt, D, K, flux,
+                                                              &calls);
+#pragma unroll
+                        for (int k = 0; k < 2 * NV; ++k) f[k / NV][k % NV] = out[(size_t)k * nc];
                     }
+                    iters += it;
 #pragma unroll
-                    for (int side = 0; side < 2; ++side) {
-                        const int kd = side ? kd1 : kd0;
-                        const int s = s0 + side;
-                        double f[NV];
-                        if ((kd & KIND_MASK) == K_ZERO) {
-#pragma unroll
-                            for (int iv = 0; iv < NV; ++iv) f[iv] = 0.0;
-                        } else {
-                            const int n = P.icn[(size_t)s * nc + p];
-                            double qf[NV];
-                            neighbour_face<NDIM, LEVEL0 ? 1 : 0>(T, P, prim, uold, ncell, p, c, idim, side, kd, n, qc, nullptr,
-                                                 dt, D, K, qf);
-                            if (side == 0) iters += riemann<NDIM, RS>(qf, qpo, f, K);
-                            else iters += riemann<NDIM, RS>(qmo, qf, f, K);
-                            ++calls;
-                            rot_swap<NDIM>(f, idim);
-                        }
-#pragma unroll
-                        for (int iv = 0; iv < NV; ++iv) {
-                            flux[((size_t)s * NV + iv) * nc + p] = f[iv];
-                            sf[r][s][iv][lane] = f[iv];
-                        }
-                    }
+                    for (int k = 0; k < 2 * NV; ++k) sf[r][s0 + k / NV][k % NV][lane] = f[k / NV][k % NV];
                 }
             }
             __syncthreads();
@@ -397,13 +508,14 @@ __global__ void __launch_bounds__(TILE * NDIM * R, MINB)
         }
     }
     if (RS == RG_RIEMANN_EXACT) {
+        unsigned long long wi = iters, wc = calls;
         for (int o = 16; o > 0; o >>= 1) {
-            iters += __shfl_xor_sync(0xffffffffu, iters, o);
-            calls += __shfl_xor_sync(0xffffffffu, calls, o);
+            wi += __shfl_xor_sync(0xffffffffu, wi, o);
+            wc += __shfl_xor_sync(0xffffffffu, wc, o);
         }
-        if (lane == 0 && calls) {
-            atomicAdd(&st->exact_iters, iters);
-            atomicAdd(&st->exact_calls, calls);
+        if (lane == 0 && wc) {
+            atomicAdd(&st->exact_iters, wi);
+            atomicAdd(&st->exact_calls, wc);
         }
     }
     // the last block out resets the work counter for the next launch

@@ -57,10 +57,110 @@ struct BrickGeom {
     const int* brick_off;
 };
 
+// Fluxes of one cell and direction in the plain forms, to the scratch.
+template <int RS>
+__device__ __noinline__ unsigned brick_dir_plain(const double* sq, int site, int idim, bool ghost, double dt,
+                                                 const DxDiv& D, const StepK& K, double* flux, int nc, int p) {
+    constexpr int NV = 5;
+    const int stride = idim == 0 ? 1 : (idim == 1 ? BSIDE : BSIDE * BSIDE);
+    int o1, o2, o3;
+    unsigned iters = 0;
+    brick_planes(idim, o1, o2, o3);
+    double qc[NV], ql[NV], qr[NV], qmo[NV], qpo[NV];
+    brick_state(sq, site, o1, o2, o3, qc);
+    brick_state(sq, site - stride, o1, o2, o3, ql);
+    brick_state(sq, site + stride, o1, o2, o3, qr);
+    own_trace<3>(qc, ql, qr, dt, D, K, qmo, qpo);
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        // neighbour n = c -/+ e, its stencil (n - e, n + e) = (c - 2e, c) / (c, c + 2e)
+        double qfar[NV], qm[NV], qp[NV], f[NV];
+        brick_state(sq, side ? site + 2 * stride : site - 2 * stride, o1, o2, o3, qfar);
+        const double* qn = side ? qr : ql;
+        const double* qnl = side ? qc : qfar;
+        const double* qnr = side ? qfar : qc;
+        if (ghost) ghost_trace<3>(qn, qnl, qnr, dt, D, K, qm, qp);
+        else own_trace<3>(qn, qnl, qnr, dt, D, K, qm, qp);
+        if (side == 0) iters += riemann<3, RS>(qm, qpo, f, K);
+        else iters += riemann<3, RS>(qmo, qp, f, K);
+        rot_swap<3>(f, idim);
+#pragma unroll
+        for (int iv = 0; iv < NV; ++iv) flux[((size_t)(2 * idim + side) * NV + iv) * nc + p] = f[iv];
+    }
+    return iters;
+}
+
+// The two fluxes of one cell and direction in the branch-free forms (a ghost
+// neighbour on both sides); false: not covered, take the plain forms.
+template <int RS, bool POW2>
+__device__ __forceinline__ bool brick_dir_fast(const double* __restrict__ sq, int site, int idim, const FastStep& S,
+                                               const FastStep& Sc, const StepK& K, double* f0, double* f1,
+                                               unsigned& iters) {
+    constexpr int NV = 5;
+    const int stride = idim == 0 ? 1 : (idim == 1 ? BSIDE : BSIDE * BSIDE);
+    int o1, o2, o3;
+    brick_planes(idim, o1, o2, o3);
+    double qc[NV], ql[NV], qr[NV], qfl[NV], qfr[NV], qmo[NV], qpo[NV], qm[NV], qp[NV];
+    brick_state(sq, site, o1, o2, o3, qc);
+    brick_state(sq, site - stride, o1, o2, o3, ql);
+    brick_state(sq, site + stride, o1, o2, o3, qr);
+    brick_state(sq, site - 2 * stride, o1, o2, o3, qfl);
+    brick_state(sq, site + 2 * stride, o1, o2, o3, qfr);
+    Check C;
+    trace_fast<3, POW2, false, true, true>(qc, ql, qr, K.own, S, K.gamma, qmo, qpo, C);
+    trace_fast<3, POW2, false, true, false>(ql, qfl, qc, K.ghost, Sc, K.gamma, qm, nullptr, C);
+    trace_fast<3, POW2, false, false, true>(qr, qc, qfr, K.ghost, Sc, K.gamma, nullptr, qp, C);
+    const bool ok = C.num_ok();
+    const bool a = riemann_fast<3, RS>(qm, qpo, f0, K, iters), b = riemann_fast<3, RS>(qmo, qp, f1, K, iters);
+    rot_swap<3>(f0, idim);
+    rot_swap<3>(f1, idim);
+    return ok && a && b;
+}
+
+// One cell of a brick: its fluxes in the three directions to the scratch, its
+// own flux sum in slot order.
+template <int RS, bool FAST, bool POW2>
+__device__ __forceinline__ void brick_cell(const double* sq, int site, int p, int nc, bool ghost, double dt,
+                                           const DxDiv& D, const FastStep& S, const FastStep& Sc, const StepK& K,
+                                           double* __restrict__ flux, double* __restrict__ fsum, unsigned& iters) {
+    constexpr int NV = 5;
+    double fs[NV];
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) fs[iv] = 0.0;
+#pragma unroll 1
+    for (int idim = 0; idim < 3; ++idim) {
+        double f[2][NV];
+        double* out = flux + (size_t)(2 * idim * NV) * nc + p;
+        unsigned it = 0;
+        bool ok = false;
+        if (FAST) ok = brick_dir_fast<RS, POW2>(sq, site, idim, S, Sc, K, f[0], f[1], it);
+        if (FAST && ok) {
+#pragma unroll
+            for (int k = 0; k < 2 * NV; ++k) out[(size_t)k * nc] = f[k / NV][k % NV];
+        } else {
+            it = brick_dir_plain<RS>(sq, site, idim, ghost, dt, D, K, flux, nc, p);
+#pragma unroll
+            for (int k = 0; k < 2 * NV; ++k) f[k / NV][k % NV] = out[(size_t)k * nc];
+        }
+        iters += it;
+#pragma unroll
+        for (int iv = 0; iv < NV; ++iv) fs[iv] = (fs[iv] + f[0][iv]) - f[1][iv];
+    }
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) fsum[(size_t)iv * nc + p] = fs[iv];
+}
+
 // The face work of one brick (index `brick` in the level's brick order), by
 // the whole block: stage the brick and its halo in sq (shared, [NV][BSITES]),
 // then every cell's fluxes and own flux sum.  Newton statistics of the exact
 // solver are added to iters / calls.
+//
+// The cells go through the branch-free forms where the solver's types, the
+// cell size and the brick's values allow (one vote of the block over the
+// staged states: finite, below 2^170); they keep every lane of a warp on one
+// straight line, so the two Riemann problems of a direction overlap.  Lanes
+// of a half-warp take rows y and y + 2 of the brick: rows are 12 doubles
+// apart, so the 16 lanes meet 16 different 8-byte banks.
 template <int RS, bool BOXED>
 __device__ __forceinline__ void brick_face(const PlanView& P, const BrickGeom& G, const int* __restrict__ lat_id,
                                            const int* __restrict__ lat_p, int kind, const double* __restrict__ prim,
@@ -91,6 +191,7 @@ __device__ __forceinline__ void brick_face(const PlanView& P, const BrickGeom& G
     const int nbx = ex / BRICK, nby = ey / BRICK;
     const int bx = local % nbx, by = (local / nbx) % nby, bz = local / (nbx * nby);
     const int x0 = bx * BRICK - BHALO, y0 = by * BRICK - BHALO, z0 = bz * BRICK - BHALO;
+    Check C;
     for (int t = threadIdx.x; t < BSITES; t += blockDim.x) {
         const int a = t % BSIDE, b = (t / BSIDE) % BSIDE, cz = t / (BSIDE * BSIDE);
         int x = x0 + a, y = y0 + b, z = z0 + cz;
@@ -99,61 +200,37 @@ __device__ __forceinline__ void brick_face(const PlanView& P, const BrickGeom& G
         z = z < 0 ? z + ez : (z >= ez ? z - ez : z);
         const size_t id = (size_t)lat_id[(size_t)x + (size_t)ex * ((size_t)y + (size_t)ey * z)] - 1;
 #pragma unroll
-        for (int iv = 0; iv < NV; ++iv) sq[iv * BSITES + t] = __ldg(prim + iv * ncell + id);
+        for (int iv = 0; iv < NV; ++iv) {
+            const double v = __ldg(prim + iv * ncell + id);
+            C.up(v);
+            sq[iv * BSITES + t] = v;
+        }
     }
-    __syncthreads();
     const int nc = P.ncells;
     const bool ghost = (kind & KIND_MASK) == K_GHOST;
+    // cell sizes of 2^-60 .. 2^60 keep the slopes' quotients in range
+    const bool fast = __syncthreads_and(C.top_ok()) && ghost && K.fast && D.dx > 0x1p-60 && D.dx < 0x1p60;
+    const FastStep S = fast_step(dt, D.dx, D.inv), Sc = fast_step(dt, 2.0 * D.dx, 0.5 * D.inv);
+    unsigned it = 0, done = 0;
     for (int u = threadIdx.x; u < BRICK * BRICK * BRICK; u += blockDim.x) {
-        const int x = u % BRICK, y = (u / BRICK) % BRICK, z = u / (BRICK * BRICK);
+        const int x = u % BRICK, z = u / (BRICK * BRICK);
+        const int y = ((u >> 4) & 1) | ((u >> 2) & 2) | ((u >> 3) & 4);
         const int site = (x + BHALO) + BSIDE * ((y + BHALO) + BSIDE * (z + BHALO));
         const int p = lat_p[(size_t)(bx * BRICK + x) + (size_t)ex * ((size_t)(by * BRICK + y) + (size_t)ey * (bz * BRICK + z))];
-        double fs[NV];
-#pragma unroll
-        for (int iv = 0; iv < NV; ++iv) fs[iv] = 0.0;
-#pragma unroll 1
-        for (int idim = 0; idim < 3; ++idim) {
-            const int stride = idim == 0 ? 1 : (idim == 1 ? BSIDE : BSIDE * BSIDE);
-            int o1, o2, o3;
-            brick_planes(idim, o1, o2, o3);
-            double qc[NV], ql[NV], qr[NV], qmo[NV], qpo[NV];
-            brick_state(sq, site, o1, o2, o3, qc);
-            brick_state(sq, site - stride, o1, o2, o3, ql);
-            brick_state(sq, site + stride, o1, o2, o3, qr);
-            own_trace<3>(qc, ql, qr, dt, D, K, qmo, qpo);
-#pragma unroll
-            for (int side = 0; side < 2; ++side) {
-                // neighbour n = c -/+ e, its stencil (n - e, n + e) = (c - 2e, c) / (c, c + 2e)
-                double qn[NV], qfar[NV], qm[NV], qp[NV], f[NV];
-                brick_state(sq, side ? site + stride : site - stride, o1, o2, o3, qn);
-                brick_state(sq, side ? site + 2 * stride : site - 2 * stride, o1, o2, o3, qfar);
-                const double* qnl = side ? qc : qfar;
-                const double* qnr = side ? qfar : qc;
-                if (ghost) ghost_trace<3>(qn, qnl, qnr, dt, D, K, qm, qp);
-                else own_trace<3>(qn, qnl, qnr, dt, D, K, qm, qp);
-                if (side == 0) iters += riemann<3, RS>(qm, qpo, f, K);
-                else iters += riemann<3, RS>(qmo, qp, f, K);
-                ++calls;
-                rot_swap<3>(f, idim);
-                const int s = 2 * idim + side;
-                const double sign = side ? -1.0 : 1.0;
-#pragma unroll
-                for (int iv = 0; iv < NV; ++iv) {
-                    flux[((size_t)s * NV + iv) * nc + p] = f[iv];
-                    fs[iv] = fs[iv] + sign * f[iv];
-                }
-            }
-        }
-#pragma unroll
-        for (int iv = 0; iv < NV; ++iv) fsum[(size_t)iv * nc + p] = fs[iv];
+        if (!fast) brick_cell<RS, false, false>(sq, site, p, nc, ghost, dt, D, S, Sc, K, flux, fsum, it);
+        else if (D.pow2) brick_cell<RS, true, true>(sq, site, p, nc, ghost, dt, D, S, Sc, K, flux, fsum, it);
+        else brick_cell<RS, true, false>(sq, site, p, nc, ghost, dt, D, S, Sc, K, flux, fsum, it);
+        done += 6;
     }
+    iters += it;
+    calls += done;
 }
 
 template <int RS, int MINB, bool BOXED>
 __global__ void __launch_bounds__(BRICK_THREADS, MINB)
     k_face_brick(PlanView P, BrickGeom G, const int* __restrict__ lat_id, const int* __restrict__ lat_p, int kind,
                  const double* __restrict__ prim, size_t ncell, double* __restrict__ flux,
-                 double* __restrict__ fsum, DevStatus* st, StepK K) {
+                 double* __restrict__ fsum, DevStatus* st, const __grid_constant__ StepK K) {
     extern __shared__ __align__(16) double sq[];  // [NV][BSITES]
     unsigned long long iters = 0, calls = 0;
     brick_face<RS, BOXED>(P, G, lat_id, lat_p, kind, prim, ncell, flux, fsum, st, K, (int)blockIdx.x, sq, iters,

@@ -1,0 +1,260 @@
+// rg_fast.cuh -- branch-free forms of the face step's arithmetic with the same bits.
+//
+// What bounds the face kernels is the latency of the FP64 chains and the
+// instructions around them, not the FP64 pipe (36 % busy in the brick kernel
+// at 16 warps per SM): every IEEE division and square root of the compiler
+// carries a branch to its slow path, and every early return of a Riemann
+// solver another, so nothing of a cell's two problems overlaps.  The forms
+// here have no branch: quotients and roots come from a Newton iteration and a
+// final correction that is correctly rounded for operands away from the ends
+// of the exponent range, one reciprocal serves every quotient by the same
+// divisor, selects replace the early returns, and what a form assumes about
+// its operands is gathered in a Check that the caller looks at once per cell
+// and direction; where it fails (ranges, floors, rare branches of the
+// reference) the caller takes the plain form instead, so every result has the
+// bits of the plain form.
+//
+// Division: y = RN(1/b) by Newton's iteration, q = RN(a y), r = RN(a - b q)
+// (exact), q' = RN(q + r y) is RN(a/b) -- P. Markstein, IBM J. Res. Dev. 34
+// (1990); with y known in advance: Brisebarre, Muller, Raina, IEEE Trans.
+// Comput. 53 (2004).  Square root: Goldschmidt's iteration and the same kind
+// of correction (Markstein; Cornea, Harrison, Tang, "Scientific Computing on
+// Itanium-based Systems", ch. 7-8).  The seeds are the PTX approximations
+// (2^-19.9 and 2^-19.0 relative, measured), so one cubic step reaches 2^-57.
+// Against the IEEE operations: no difference on 3e10 pairs and roots,
+// divisors and quotients next to the hard cases among them, nor on the 844
+// roots within 2^-43 ulp of a rounding boundary.  The results do not carry the sign
+// of a negative zero numerator over a positive divisor; no numerator here can be one.
+#pragma once
+
+#include "rg_physics.cuh"
+
+namespace rg {
+
+__device__ __forceinline__ double rcp_fast(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = fma(-b, y, 1.0);
+    y = fma(y, fma(e, e, e), y);
+    return fma(y, fma(-b, y, 1.0), y);
+}
+// a / b with y = rcp_fast(b) (or the correctly rounded 1 / b)
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+__device__ __forceinline__ double sqrt_fast(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = x * y, h = 0.5 * y;
+    const double r = fma(-g, h, 0.5), t = fma(1.5 * r, r, r);
+    g = fma(g, t, g);
+    h = fma(h, t, h);
+    return fma(fma(-g, g, x), h, g);
+}
+
+// Operand checks, gathered: magnitudes below 2^170 (finite with them) by the
+// largest high word, numerators zero or above 2^-800 by the smallest (0 wraps
+// to the top; a nonzero low word counts), so that with divisors in [2^-140,
+// 2^700] no step of a quotient over- or underflows.
+struct Check {
+    static constexpr unsigned kTop = (1023u + 170u) << 20, kBottom = (1023u - 800u) << 20;
+    unsigned mx = 0, mn = 0xffffffffu;
+    __device__ __forceinline__ void up(double x) { mx = max(mx, (unsigned)__double2hiint(x) & 0x7fffffffu); }
+    __device__ __forceinline__ void num(double a) {
+        const unsigned h = ((unsigned)__double2hiint(a) & 0x7fffffffu) | min((unsigned)__double2loint(a), 1u);
+        mn = min(mn, h - 1u);
+    }
+    __device__ __forceinline__ bool top_ok() const { return mx < kTop; }
+    __device__ __forceinline__ bool num_ok() const { return mn >= kBottom; }
+};
+
+// Limited slope parameters: the slope types 1, 2, 3 and 8 (and those the
+// reference treats as 1) are min(th |l|, th |r|, cf |l + r|) with the sign of
+// l where l r > 0, and so are the interpolation types 1..3 of the ghost
+// branch: |l + r| >= max(|l|, |r|) there, so cf = 1 leaves a minmod as it is,
+// and th = infinity the centred slope.
+struct Limiter {
+    double th, cf;
+};
+// CHK: the caller has not looked at the states, so the difference is checked
+// (finite, not huge) here
+template <bool CHK>
+__device__ __forceinline__ double limited(double ql, double qc, double qr, const Limiter& L, Check& C) {
+    const double l = qc - ql, r = qr - qc;
+    const double c = L.cf * fabs(l + r);
+    if (CHK) C.up(c);
+    double m = L.th * fabs(l);
+    const double b = L.th * fabs(r);
+    m = b < m ? b : m;
+    m = c < m ? c : m;
+    m = copysign(m, l);
+    return l * r > 0.0 ? m : 0.0;
+}
+
+// Values of a step the branch-free forms share (per cell size).
+struct FastStep {
+    double hdt, hdt0;       // dt / 2, and times zero: the tangential source term
+    double dx, inv;         // cell size of the slope, its reciprocal
+    double hdx;             // half the cell size
+};
+__device__ __forceinline__ FastStep fast_step(double dt, double dx, double inv) {
+    return FastStep{0.5 * dt, 0.5 * dt * 0.0, dx, inv, 0.5 * dx};
+}
+
+// compute_slopes / ghost slopes and trace of a rotated state: the upper face
+// state in qm, the lower in qp (either may be left out).  Primitive states:
+// their density is at least 1e-10 (ctoprim).
+template <int NDIM, bool POW2, bool CHK, bool QM, bool QP>
+__device__ __forceinline__ void trace_fast(const double* q, const double* ql, const double* qr, const Limiter& L,
+                                           const FastStep& S, double gamma, double* qm, double* qp, Check& C) {
+    constexpr int NV = Dims<NDIM>::NV, IP = Dims<NDIM>::IP;
+    double dq[NV];
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) {
+        const double s = limited<CHK>(ql[iv], q[iv], qr[iv], L, C);
+        if (POW2) {
+            dq[iv] = s * S.inv;
+        } else {
+            C.num(s);
+            dq[iv] = div_by(s, S.dx, S.inv);
+        }
+    }
+    const double r = q[0], u = q[1], p = smax(q[IP], r * 1e-20);
+    const double y = rcp_fast(r);
+    if (CHK) {
+        C.up(r);
+        C.up(p);
+        C.up(dq[IP]);
+    }
+    C.num(dq[IP]);
+    const double cs2 = smax(div_by(gamma * p, r, y), 1e-20);
+    const double ru = dq[1] * r;
+    const double b[3] = {S.hdt * (-u * dq[0] - ru), S.hdt * (-u * dq[1] - div_by(dq[IP], r, y)),
+                         S.hdt * (-u * dq[IP] - ru * cs2)};
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) {
+        const double a = S.hdx * dq[iv];
+        const double bb = iv == 0 ? b[0] : (iv == 1 ? b[1] : (iv == IP ? b[2] : S.hdt0));
+        if (QP) qp[iv] = q[iv] - a + bb;
+        if (QM) qm[iv] = q[iv] + a + bb;
+    }
+    if (QP && qp[0] < 1e-10) qp[0] = r;
+    if (QM && qm[0] < 1e-10) qm[0] = r;
+}
+
+// The solvers' constants: gamma, gamma - 1 and its reciprocal, the pressure floor's factor.
+struct FastGas {
+    double gamma, gm1, rgm1, smallp;
+};
+
+// compute_flux and prim_to_cons of one state
+template <int NDIM>
+__device__ __forceinline__ void flux_cons(const double* q, const FastGas& G, double* f, double* u, Check& C) {
+    constexpr int IP = Dims<NDIM>::IP;
+    double v2 = q[1] * q[1];
+#pragma unroll
+    for (int i = 2; i <= NDIM; ++i) v2 = v2 + q[i] * q[i];
+    C.num(q[IP]);
+    const double E = 0.5 * q[0] * v2 + div_by(q[IP], G.gm1, G.rgm1);
+    C.up(E);
+    const double m = q[0] * q[1];
+    f[0] = m;
+    f[1] = m * q[1] + q[IP];
+    u[0] = q[0];
+    u[1] = m;
+#pragma unroll
+    for (int i = 2; i <= NDIM; ++i) {
+        f[i] = m * q[i];
+        u[i] = q[0] * q[i];
+    }
+    f[IP] = (E + q[IP]) * q[1];
+    u[IP] = E;
+}
+
+template <int NDIM>
+__device__ __forceinline__ double cs2_fast(const double* q, const FastGas& G, Check& C) {
+    constexpr int IP = Dims<NDIM>::IP;
+    C.up(q[0]);
+    C.up(q[1]);
+    C.up(q[IP]);
+    return smax(div_by(G.gamma * q[IP], q[0], rcp_fast(q[0])), 1e-20);
+}
+
+// The Riemann solvers on traced states (their density is at least 1e-10 by
+// the trace's floor).  False: take the plain form.
+template <int NDIM>
+__device__ __forceinline__ bool hllc_fast(const double* ql, const double* qr, double* f, const FastGas& G) {
+    constexpr int NV = Dims<NDIM>::NV, IP = Dims<NDIM>::IP;
+    Check C;
+    const double rl = ql[0], ul = ql[1], pl = ql[IP], rr = qr[0], ur = qr[1], pr = qr[IP];
+    // the larger of two roots is the root of the larger: one root, same bits
+    const double c2l = cs2_fast<NDIM>(ql, G, C), c2r = cs2_fast<NDIM>(qr, G, C);
+    const double cmax = sqrt_fast(smax(c2l, c2r));
+    const double sl = smin(ul, ur) - cmax, sr = smax(ul, ur) + cmax;
+    const double rcl = rl * (ul - sl), rcr = rr * (sr - ur), div = rcr + rcl;
+    const double nu = rcr * ur + rcl * ul + (pl - pr), np = rcr * pl + rcl * pr + rcl * rcr * (ul - ur);
+    const double yd = rcp_fast(div);
+    const double ustar = smax(-1e6, smin(1e6, div_by(nu, div, yd)));
+    const double pstar = smax(div_by(np, div, yd), 0.0);
+    const bool supl = sl > 0.0, supr = sr < 0.0, star = !(supl || supr);
+    const bool left = supl || (!supr && ustar > 0.0);
+    double q[NV], u0[NV];
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) q[iv] = left ? ql[iv] : qr[iv];
+    flux_cons<NDIM>(q, G, f, u0, C);
+    const bool base_ok = C.top_ok() && C.num_ok() && !(pl < rl * G.smallp) && !(pr < rr * G.smallp);
+    Check D;
+    D.num(nu);
+    D.num(np);
+    const double so = left ? sl : sr;
+    const double den = left ? smin(so - ustar, -1e-10) : smax(so - ustar, 1e-10);
+    const double yn = rcp_fast(den);
+    const double w = so - q[1];
+    const double rstar = div_by(q[0] * w, den, yn);
+    const double ne = w * u0[IP] - q[IP] * q[1] + pstar * ustar;
+    D.num(ne);
+    double us[NV];
+    us[0] = rstar;
+    us[1] = rstar * ustar;
+#pragma unroll
+    for (int i = 2; i <= NDIM; ++i) us[i] = rstar * q[i];
+    us[IP] = div_by(ne, den, yn);
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) {
+        const double fs = f[iv] + so * (us[iv] - u0[iv]);
+        f[iv] = star ? fs : f[iv];
+    }
+    return base_ok && (!star || (D.num_ok() && !(div < 1e-5)));
+}
+
+template <int NDIM>
+__device__ __forceinline__ bool llf_fast(const double* ql, const double* qr, double* f, const FastGas& G) {
+    constexpr int NV = Dims<NDIM>::NV;
+    Check C;
+    double fl[NV], fr[NV], ul[NV], ur[NV];
+    flux_cons<NDIM>(ql, G, fl, ul, C);
+    flux_cons<NDIM>(qr, G, fr, ur, C);
+    const double al = sqrt_fast(cs2_fast<NDIM>(ql, G, C)), ar = sqrt_fast(cs2_fast<NDIM>(qr, G, C));
+    const double ha = 0.5 * smax(fabs(ql[1]) + al, fabs(qr[1]) + ar);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) f[i] = 0.5 * (fl[i] + fr[i]) - ha * (ur[i] - ul[i]);
+    return C.top_ok() && C.num_ok();
+}
+
+template <int NDIM>
+__device__ __forceinline__ bool hll_fast(const double* ql, const double* qr, double* f, const FastGas& G) {
+    constexpr int NV = Dims<NDIM>::NV;
+    Check C;
+    double fl[NV], fr[NV], ul[NV], ur[NV];
+    flux_cons<NDIM>(ql, G, fl, ul, C);
+    flux_cons<NDIM>(qr, G, fr, ur, C);
+    const double al = sqrt_fast(cs2_fast<NDIM>(ql, G, C)), ar = sqrt_fast(cs2_fast<NDIM>(qr, G, C));
+    const double sl = smin(0.0, smin(ql[1] - al, qr[1] - ar)), sr = smax(0.0, smax(ql[1] + al, qr[1] + ar));
+    const double w = sr - sl, inv = div_by(1.0, w, rcp_fast(w));
+#pragma unroll
+    for (int i = 0; i < NV; ++i) f[i] = (sr * fl[i] - sl * fr[i] + sr * sl * (ur[i] - ul[i])) * inv;
+    return C.top_ok() && C.num_ok() && !(w < 1e-20);
+}
+
+}  // namespace rg

@@ -1,0 +1,153 @@
+"""The branch-free forms of the face kernels (csrc/rg_fast.cuh): quotients and
+roots against the IEEE operations, and level steps against the oracle on
+states that reach each of their limits (operands outside the checked ranges,
+floors, zero and tiny numerators, supersonic faces, NaN), in the tiled and the
+brick kernel.  Same bits everywhere."""
+import ctypes
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+import rg_tree
+import rgpu
+from refsupport import make_params
+from test_gpu_level import ga_of
+
+pytestmark = pytest.mark.gpu
+
+CSRC = Path(rgpu.__file__).resolve().parent / "csrc"
+
+SOURCE = r"""
+#include "rg_fast.cuh"
+#include <cstdint>
+__device__ uint64_t rnd(uint64_t& s) {
+    s += 0x9E3779B97F4A7C15ull;
+    uint64_t z = s;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return z ^ (z >> 31);
+}
+__device__ double make(uint64_t m, int e) { return __longlong_as_double((long long)((m & 0xfffffffffffffull) | ((uint64_t)(1023 + e) << 52))); }
+__global__ void k(int mode, int n, unsigned long long* bad) {
+    uint64_t s = (blockIdx.x * blockDim.x + threadIdx.x) * 1000003ull + mode * 77777ull;
+    unsigned long long b0 = 0, b1 = 0;
+    for (int i = 0; i < n; ++i) {
+        uint64_t ra = rnd(s), rb = rnd(s);
+        const int ea = (int)(rnd(s) % 1200) - 600, eb = (int)(rnd(s) % 700) - 130;
+        if (mode == 1) rb = ~(rb % 64);                       // divisors just below a power of two
+        if (mode == 2) { ra = ~(ra % 4096); rb = ~(rb % 4096); }
+        if (mode == 3) { ra = ra & 1 ? ~(ra % 4096) : ra % 4096; rb = rb % 4096; }
+        const double b = make(rb, eb);
+        double a = make(ra, ea);
+        if (mode == 4) {                                      // quotients next to a rounding boundary
+            const double q = make(ra, 0);
+            a = fma(b, q * 0x1p-53, b * q);
+        }
+        if (rb >> 63) a = -a;
+        if (rg::div_by(a, b, rg::rcp_fast(b)) != a / b) ++b0;
+        const double x = make(ra, (ea & 1 ? 1 : 0) + 2 * (ea / 8));
+        if (rg::sqrt_fast(x) != sqrt(x)) ++b1;
+    }
+    atomicAdd(bad, b0);
+    atomicAdd(bad + 1, b1);
+}
+__global__ void kz(unsigned long long* bad) {                 // zero numerators keep their sign's result
+    if (rg::div_by(0.0, 3.0, rg::rcp_fast(3.0)) != 0.0 || signbit(rg::div_by(0.0, 3.0, rg::rcp_fast(3.0)))) ++bad[0];
+    if (!signbit(rg::div_by(0.0, -3.0, rg::rcp_fast(-3.0)))) ++bad[0];
+}
+extern "C" int check(int mode, int n, unsigned long long* out) {
+    unsigned long long* d;
+    if (cudaMalloc(&d, 16) != cudaSuccess) return 1;
+    cudaMemset(d, 0, 16);
+    k<<<592, 256>>>(mode, n, d);
+    kz<<<1, 1>>>(d);
+    const int rc = cudaMemcpy(out, d, 16, cudaMemcpyDeviceToHost) != cudaSuccess;
+    cudaFree(d);
+    return rc;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def forms(tmp_path_factory):
+    d = tmp_path_factory.mktemp("fast_forms")
+    (d / "t.cu").write_text(SOURCE)
+    subprocess.run(["/usr/local/cuda/bin/nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17",
+                    "-fmad=false", "-shared", "-Xcompiler", "-fPIC", f"-I{CSRC}", "-o", str(d / "t.so"),
+                    str(d / "t.cu")], check=True)
+    return ctypes.CDLL(str(d / "t.so"))
+
+
+@pytest.mark.parametrize("mode", range(5))
+def test_quotients_and_roots_are_the_ieee_ones(forms, mode):
+    bad = (ctypes.c_ulonglong * 2)()
+    assert forms.check(mode, 2000, bad) == 0
+    assert list(bad) == [0, 0]
+
+
+def odd_states(g, level, seed, nan):
+    """Random states with patches that reach every limit of the forms."""
+    u = rg_tree.random_state(g, level, seed=seed).reshape(5, g.ncell)
+    ids = g.cell_ids(level) - 1
+    n = len(ids)
+    rng = np.random.default_rng(seed)
+
+    def patch(k, m=0.04):
+        lo = int(n * k / 12)
+        return ids[lo:lo + max(8, int(n * m))]
+
+    def put(cells, rho, v, p):
+        u[0, cells] = rho
+        for d in range(3):
+            u[1 + d, cells] = rho * v[d]
+        u[4, cells] = p / 0.4 + 0.5 * rho * sum(x * x for x in v)
+    put(patch(0), 1.0, (0.0, 0.0, 0.0), 1.0)                      # at rest: zero slopes, zero numerators
+    put(patch(1), 1.0, (0.0, -0.0, 0.0), 1e-5)
+    put(patch(2), 2.0, (60.0, -70.0, 80.0), 0.5)                  # supersonic faces
+    put(patch(3), 1e-12, (1.0, 0.0, 0.0), 1e-14)                  # below the density floor
+    put(patch(4), 1.0, (0.0, 0.0, 0.0), 1e55)                     # above the checked range
+    put(patch(5), 1e53, (1e-3, 0.0, 0.0), 1.0)
+    put(patch(6), 1.0, (0.0, 0.0, 0.0), 1e-300)                   # pressure floor
+    c = patch(7)
+    put(c, 1.0, (1e-260, 0.0, 0.0), 1.0)                          # numerators under the checked range
+    u[1, c] = rng.uniform(-1e-260, 1e-260, len(c))
+    put(patch(8), 1e-7, (0.0, 0.0, 0.0), 1e-9)                    # rc_l + rc_r < 1e-5
+    c = patch(9)
+    u[4, c] = -u[4, c]                                            # negative energy
+    if nan:
+        u[rng.integers(0, 5), ids[n // 2]] = np.nan
+    return u.reshape(-1)
+
+
+def same(a, b):
+    na, nb = np.isnan(a), np.isnan(b)
+    return np.array_equal(na, nb) and np.array_equal(a[~na].view(np.int64), b[~nb].view(np.int64))
+
+
+@pytest.mark.parametrize("nan", [False, True])
+@pytest.mark.parametrize("variant", [1, 4, 10])
+@pytest.mark.parametrize("nx,level,riem,slope,itype", [(1, 5, "hllc", 2, 1), (1, 5, "llf", 1, 2), (3, 4, "hllc", 8, 3),
+                                                       (3, 4, "hll", 3, 1), (1, 4, "acoustic", 1, 3),
+                                                       (3, 4, "hllc", 2, 0), (1, 4, "hllc", 7, 1)])
+def test_level_step_at_the_limits_matches_the_oracle(rgpu_lib, oracle, nx, level, riem, slope, itype, variant, nan):
+    g = rg_tree.build_uniform(3, level, nx=nx, ny=nx, nz=nx)
+    ga = ga_of(g)
+    params = make_params(3, slope_type=slope, riemann=riem, interpol_type=itype)
+    ctx = rgpu.Context(params, 0)
+    try:
+        ctx.sync_topology(g)
+        ctx.set_face_config(level, variant, 1)
+        dx = 1.0 / (nx * 2 ** level)
+        for seed in (1, 2):
+            uold = odd_states(g, level, seed, nan)
+            unew = uold.copy()
+            ctx.upload_state(uold, unew)
+            oracle.godunov_fine(ga, params, level, 1e-4, dx, uold.copy(), unew)
+            ctx.godunov_level(level, 1e-4, dx)
+            got = np.empty_like(unew)
+            ctx.download_state(unew=got)
+            assert same(got, unew), f"{np.count_nonzero(got != unew)} values differ"
+    finally:
+        ctx.close()

@@ -10,6 +10,7 @@
 #include <cstdint>
 
 #include "rg_face.cuh"
+#include "rg_fast.cuh"
 #include "rg_mlp.cuh"
 
 namespace rg {
@@ -68,6 +69,12 @@ __global__ void k_stress_states(int n, unsigned long long seed, double* ql, doub
     }
 }
 
+template <int NDIM>
+__device__ __noinline__ int solve_exact_plain(const double* a, const double* b, double* f, double gamma, int niter,
+                                              double tol, double guess, double* ps) {
+    return solve_exact_p<NDIM>(a, b, f, gamma, 1e-10 * 1e-10 / gamma, niter, tol, guess, ps);
+}
+
 // Exact solves of a batch; guess_in: per-interface Newton starts (-1: the
 // two-shock start; k_mlp_guess_tc writes them), or null for the two-shock
 // start everywhere.
@@ -85,10 +92,30 @@ __global__ void __launch_bounds__(256, 4) k_exact_batch(int n, const double* __r
             b[v] = qr[(size_t)v * n + i];
         }
         double gamma = gam ? gam[i] : gamma0;
-        double smallp = 1e-10 * 1e-10 / gamma;
         double guess = guess_in ? guess_in[i] : -1.0;
         double ps;
-        int it = solve_exact_p<NDIM>(a, b, f, gamma, smallp, niter, tol, guess, &ps);
+        int it = 0;
+        bool ok = false;
+        if (gamma > 1.0 + 0x1p-20 && gamma < 0x1p20) {
+            // one reciprocal of gamma for the solver's three quotients by it
+            const double y = rcp_fast(gamma), gm1 = gamma - 1.0;
+            const FastGas G{gamma, gm1, rcp_fast(gm1), div_by(1e-10 * 1e-10, gamma, y),
+                            div_by(gamma + 1.0, 2.0 * gamma, 0.5 * y), div_by(1.0, gamma, y)};
+            ok = exact_fast<NDIM>(a, b, f, G, niter, tol, guess, &ps, &it);
+        }
+        if (!ok) {
+            // (copies: the call's arrays live in memory, the loop's in registers)
+            double a2[NV], b2[NV], f2[NV], p2;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                a2[v] = a[v];
+                b2[v] = b[v];
+            }
+            it = solve_exact_plain<NDIM>(a2, b2, f2, gamma, niter, tol, guess, &p2);
+            ps = p2;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) f[v] = f2[v];
+        }
         if (flux) {
 #pragma unroll
             for (int v = 0; v < NV; ++v) flux[(size_t)v * n + i] = f[v];

@@ -219,13 +219,21 @@ __device__ __forceinline__ int riemann(const double* ql, const double* qr, doubl
     return 0;
 }
 
-// The branch-free solvers; the exact solver iterates, so it has its plain form only.
+// The branch-free solvers (the exact one loops, its updates are branch-free;
+// the acoustic one has its plain form only).
 template <int NDIM, int RS>
 __device__ __forceinline__ bool riemann_fast(const double* ql, const double* qr, double* f, const StepK& K,
                                              unsigned& iters) {
     if constexpr (RS == RG_RIEMANN_HLLC) return hllc_fast<NDIM>(ql, qr, f, K.gas);
     else if constexpr (RS == RG_RIEMANN_HLL) return hll_fast<NDIM>(ql, qr, f, K.gas);
     else if constexpr (RS == RG_RIEMANN_LLF) return llf_fast<NDIM>(ql, qr, f, K.gas);
+    else if constexpr (RS == RG_RIEMANN_EXACT) {
+        int it;
+        const bool ok = exact_fast<NDIM>(ql, qr, f, K.gas, K.exact_niter, K.exact_tol,
+                                         mlp_guess<NDIM>(K.mlp, ql, qr, K.gamma, K.smallp), nullptr, &it);
+        iters += it;
+        return ok;
+    }
     iters += riemann<NDIM, RS>(ql, qr, f, K);
     return true;
 }

@@ -146,6 +146,7 @@ __device__ __forceinline__ void trace_fast(const double* q, const double* ql, co
 // The solvers' constants: gamma, gamma - 1 and its reciprocal, the pressure floor's factor.
 struct FastGas {
     double gamma, gm1, rgm1, smallp;
+    double g6, rg;  // (gamma + 1) / (2 gamma) and 1 / gamma: the exact solver's
 };
 
 // compute_flux and prim_to_cons of one state
@@ -255,6 +256,150 @@ __device__ __forceinline__ bool hll_fast(const double* ql, const double* qr, dou
 #pragma unroll
     for (int i = 0; i < NV; ++i) f[i] = (sr * fl[i] - sl * fr[i] + sr * sl * (ur[i] - ul[i])) * inv;
     return C.top_ok() && C.num_ok() && !(w < 1e-20);
+}
+
+// One Newton update of the two-shock solver (RiemannSolver.cpp:221-233).
+struct NewtonSide {
+    double u, p, c, b, y;  // velocity, pressure, gamma p rho, p + 1e-20 and its reciprocal
+};
+__device__ __forceinline__ double newton_mass(const NewtonSide& s, double p, double g6) {
+    return sqrt_fast(s.c * (1.0 + div_by(g6 * (p - s.p), s.b, s.y)));
+}
+__device__ __forceinline__ double newton_drop(const NewtonSide& s, double p, double w) {
+    const double d = w + 1e-20;
+    return div_by(p - s.p, d, rcp_fast(d));
+}
+__device__ __forceinline__ double newton_slope(const NewtonSide& s, double w) {
+    const double w2 = w * w, d = w2 + s.c + 1e-20;
+    return div_by(2.0 * (w2 * w), d, rcp_fast(d));
+}
+__device__ __forceinline__ double newton_update(const NewtonSide& l, const NewtonSide& r, double p, double g6, double* gap) {
+    const double wl = newton_mass(l, p, g6), wr = newton_mass(r, p, g6);
+    const double ql = newton_slope(l, wl), qr = newton_slope(r, wr);
+    *gap = (l.u - newton_drop(l, p, wl)) - (r.u + newton_drop(r, p, wr));
+    const double d = qr + ql + 1e-20;
+    return smax(div_by(qr * ql, d, rcp_fast(d)) * *gap, -p);
+}
+// |d / p| < tol as the division gives it: the product decides unless it is
+// within 2^-50 of the limit
+__device__ __forceinline__ bool newton_done(double d, double p, double tol) {
+    const double a = fabs(d), c = tol * p;
+    if (fabs(a - c) <= c * 0x1p-50) return a / p < tol;
+    return a < c;
+}
+
+// solve_exact_p (rg_physics.cuh) with the quotients and roots above, the same
+// iteration, stop, polish and sampling.  gamma > 1; false: take the plain form.
+template <int NDIM>
+__device__ __forceinline__ bool exact_fast(const double* ql, const double* qr, double* flux, const FastGas& G, int niter,
+                                           double tol, double p_guess, double* pstar_out, int* it_out) {
+    constexpr int IP = Dims<NDIM>::IP;
+    Check C;
+    const double gamma = G.gamma, g6 = G.g6;
+    const double rl = smax(ql[0], 1e-10), rr = smax(qr[0], 1e-10);
+    NewtonSide L, R;
+    L.u = ql[1];
+    R.u = qr[1];
+    L.p = smax(ql[IP], rl * G.smallp);
+    R.p = smax(qr[IP], rr * G.smallp);
+    L.c = gamma * L.p * rl;
+    R.c = gamma * R.p * rr;
+    L.b = L.p + 1e-20;
+    R.b = R.p + 1e-20;
+    L.y = rcp_fast(L.b);
+    R.y = rcp_fast(R.b);
+    C.up(rl);
+    C.up(rr);
+    C.up(L.u);
+    C.up(R.u);
+    C.up(L.p);
+    C.up(R.p);
+    const double wl = sqrt_fast(L.c), wr = sqrt_fast(R.c);
+    const double ws = wl + wr + 1e-20, ns = wr * L.p + wl * R.p + wl * wr * (L.u - R.u);
+    C.num(ns);
+    double pstar = smax(div_by(ns, ws, rcp_fast(ws)), 0.0);
+    if (p_guess > 0.0) pstar = p_guess;
+    double pold = pstar;
+    int it = 0;
+    const bool safe = tol < 1e-6;
+    double lo = 0.0, hi = CUDART_INF;
+    for (int iter = 0; iter < niter; ++iter) {
+        double gv;
+        C.up(pold);
+        const double delp = newton_update(L, R, pold, g6, &gv);
+        ++it;
+        if (safe) {
+            if (gv > 0.0) lo = smax(lo, pold);
+            else if (gv < 0.0) hi = smin(hi, pold);
+            else break;
+            double pn = pold + delp;
+            if (newton_done(delp, pn + 1e-10, tol)) {
+                pold = pn;
+                break;
+            }
+            if (!((pn > lo || pn == 0.0) && pn < hi)) pn = hi < CUDART_INF ? 0.5 * (lo + hi) : 2.0 * lo + 1e-300;
+            pold = pn;
+            if (hi - lo <= tol * (lo + 1e-10)) break;
+            continue;
+        }
+        pold = pold + delp;
+        if (newton_done(delp, pold + 1e-10, tol)) break;
+    }
+    C.up(pold);
+    if (safe) {
+        pold = __longlong_as_double(__double_as_longlong(pold) & ~((1LL << 22) - 1));
+        for (int k = 0; k < 2; ++k) {
+            double gv;
+            pold = pold + newton_update(L, R, pold, g6, &gv);
+            C.up(pold);
+        }
+    }
+    pstar = pold;
+    if (pstar_out) *pstar_out = pstar;
+    const double dl = newton_mass(L, pstar, g6) + 1e-20, dr = newton_mass(R, pstar, g6) + 1e-20;
+    const double ustar = 0.5 * (L.u + div_by(L.p - pstar, dl, rcp_fast(dl)) + R.u - div_by(R.p - pstar, dr, rcp_fast(dr)));
+    const bool left = ustar > 0;
+    double ro = left ? rl : rr, po = left ? L.p : R.p;
+    double rstar;
+    C.num(pstar);
+    if (pstar >= po) {
+        const double d = G.gm1 * pstar + (gamma + 1.0) * po;
+        rstar = div_by(ro * ((gamma + 1.0) * pstar + G.gm1 * po), d, rcp_fast(d));
+    } else {
+        rstar = ro * pow(div_by(pstar, left ? L.b : R.b, left ? L.y : R.y), G.rg);
+    }
+    rstar = smax(rstar, 1e-10);
+    const double c2l = smax(div_by(gamma * L.p, rl, rcp_fast(rl)), 1e-20);
+    const double c2r = smax(div_by(gamma * R.p, rr, rcp_fast(rr)), 1e-20);
+    const double cm = sqrt_fast(smax(c2l, c2r));
+    double uo;
+    if (smin(L.u, R.u) - cm > 0.0) {
+        ro = rl;
+        uo = L.u;
+        po = L.p;
+    } else if (smax(L.u, R.u) + cm < 0.0) {
+        ro = rr;
+        uo = R.u;
+        po = R.p;
+    } else {
+        ro = rstar;
+        uo = ustar;
+        po = pstar;
+    }
+    double e_kin = 0.5 * ro * uo * uo;
+#pragma unroll
+    for (int i = 2; i <= NDIM; ++i) {
+        const double vt = left ? ql[i] : qr[i];
+        e_kin = e_kin + 0.5 * ro * vt * vt;
+    }
+    const double E = div_by(po, G.gm1, G.rgm1) + e_kin;
+    flux[0] = ro * uo;
+    flux[1] = ro * uo * uo + po;
+#pragma unroll
+    for (int i = 2; i <= NDIM; ++i) flux[i] = flux[0] * (left ? ql[i] : qr[i]);
+    flux[IP] = (E + po) * uo;
+    *it_out = it;
+    return C.top_ok() && C.num_ok();
 }
 
 }  // namespace rg

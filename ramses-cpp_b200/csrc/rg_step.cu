@@ -623,7 +623,8 @@ StepK step_consts(const rg_ctx* c) {
     const int st = p.slope_type, it = p.interpol_type;
     K.own = st == 2 || st == 3 ? Limiter{2.0, 0.5} : (st == 8 ? Limiter{1.5, 0.5} : Limiter{1.0, 1.0});
     K.ghost = it == 1 ? Limiter{0.5, 1.0} : (it == 2 ? Limiter{1.0, 0.25} : Limiter{HUGE_VAL, 0.25});
-    K.gas = FastGas{p.gamma, p.gamma - 1.0, 1.0 / (p.gamma - 1.0), K.smallp};
+    K.gas = FastGas{p.gamma, p.gamma - 1.0, 1.0 / (p.gamma - 1.0), K.smallp, (p.gamma + 1.0) / (2.0 * p.gamma),
+                    1.0 / p.gamma};
     K.fast = st != 0 && !(st >= 4 && st <= 7) && it >= 1 && it <= 3 && K.gas.gm1 > 0x1p-20 && K.gas.gm1 < 0x1p20;
     return K;
 }

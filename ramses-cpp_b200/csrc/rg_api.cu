@@ -794,11 +794,14 @@ int rg_level_run(rg_ctx* c, int ilevel, double dx, int pressure_cap, double t_st
         n = c->h_status->run_steps;
         return c->h_status->err ? check_device_status(c) : RG_OK;
     };
-    if (P->ncells <= kRunBlockCells) {
-        // small level: the loop in a single-block kernel
+    if (int rc = line_check(c, *P)) return rc;
+    if (P->line || P->ncells <= kRunBlockCells) {
+        // small level: the loop in one kernel, a 1D line over a cluster, else a single block
         while (t < t_end && n < max_steps) {
             const long long limit = std::min<long long>(max_steps, n + kRunChunk);
-            if (int rc = launch_run_block(c, *P, dx, pressure_cap, t_end, limit)) return rc;
+            if (int rc = P->line ? launch_run_line(c, *P, dx, pressure_cap, t_end, limit)
+                                 : launch_run_block(c, *P, dx, pressure_cap, t_end, limit))
+                return rc;
             if (int rc = read_clock()) return rc;
         }
         c->next_level = ilevel;

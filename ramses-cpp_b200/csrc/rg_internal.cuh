@@ -154,6 +154,7 @@ struct Plan {
     int face_variant = -1, face_batch = 4;  // autotuned face-kernel shape (-1: not tuned yet)
     float face_ms = 0.f;
     int substeps_run = 0;
+    int line = -1;             // 1D: one periodic line in list order (-1: not looked at; rg_run1d.cu)
     int lattice = 0;           // the level is one complete periodic lattice (rg_lattice.cu)
     int lat_e[3] = {0, 0, 0};  // its extent
     int lat_kind = 0;          // the (single) interface kind of its faces
@@ -364,6 +365,11 @@ int refresh_tree(rg_ctx* c);
 // the block): the whole loop in one single-block kernel (rg_step.cu); the clock
 // in DevStatus run_t/run_steps.  Larger levels are faster spread over the GPU.
 constexpr int kRunBlockCells = 1024;
+// rg_level_run on a 1D level of at most kLineCells cells that is one periodic
+// line (line_check looks once per plan): one cluster launch (rg_run1d.cu)
+constexpr int kLineCells = 8192;
+int line_check(rg_ctx* c, Plan& P);
+int launch_run_line(rg_ctx* c, const Plan& P, double dx, int pressure_cap, double t_end, long long max_steps);
 int launch_run_block(rg_ctx* c, const Plan& P, double dx, int pressure_cap, double t_end, long long max_steps);
 // TreeUpdater operations on the device-resident tree (rg_tree.cu)
 int tree_flag_fine(rg_ctx* c, int ilevel, double ed, double ep, double ev, double eb2, int nexp, int icount,

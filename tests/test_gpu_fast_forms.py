@@ -57,6 +57,51 @@ __global__ void kz(unsigned long long* bad) {                 // zero numerators
     if (rg::div_by(0.0, 3.0, rg::rcp_fast(3.0)) != 0.0 || signbit(rg::div_by(0.0, 3.0, rg::rcp_fast(3.0)))) ++bad[0];
     if (!signbit(rg::div_by(0.0, -3.0, rg::rcp_fast(-3.0)))) ++bad[0];
 }
+// the exact solver's two forms on random pairs, odd ones among them
+__global__ void ke(int n, int niter, double tol, unsigned long long* bad) {
+    uint64_t s = (blockIdx.x * blockDim.x + threadIdx.x) * 99991ull + niter;
+    auto uni = [&](double a, double b) { return a + (b - a) * ((rnd(s) >> 11) * 0x1p-53); };
+    unsigned long long b0 = 0, plain = 0;
+    for (int i = 0; i < n; ++i) {
+        double l[5], r[5], f[5], g[5], ps, pg;
+        const int odd = rnd(s) % 16;
+        for (double* q : {l, r}) {
+            q[0] = exp(uni(-12.0, 12.0));
+            q[1] = uni(-3.0, 3.0);
+            q[2] = uni(-1.0, 1.0);
+            q[3] = uni(-1.0, 1.0);
+            q[4] = exp(uni(-16.0, 16.0));
+        }
+        if (odd == 0) for (int k = 0; k < 5; ++k) r[k] = l[k];
+        if (odd == 1) { l[1] = -40.0; r[1] = 40.0; }
+        if (odd == 2) r[4] = 0.0;
+        if (odd == 3) l[4] = -1.0;
+        if (odd == 4) r[0] = 1e-13;
+        if (odd == 5) l[4] = 1e60;
+        if (odd == 6) { l[1] = 50.0; r[1] = 45.0; }
+        if (odd == 7) { for (int k = 0; k < 5; ++k) r[k] = l[k]; r[1] += 1e-9; }
+        const double gamma = rnd(s) & 1 ? 1.4 : 5.0 / 3.0, smallp = 1e-10 * 1e-10 / gamma;
+        const double guess = odd == 8 ? l[4] * 1.1 : -1.0;
+        const rg::FastGas G{gamma, gamma - 1.0, 1.0 / (gamma - 1.0), smallp, (gamma + 1.0) / (2.0 * gamma), 1.0 / gamma};
+        int it;
+        if (!rg::exact_fast<3>(l, r, f, G, niter, tol, guess, &ps, &it)) { ++plain; continue; }
+        const int jt = rg::solve_exact_p<3>(l, r, g, gamma, smallp, niter, tol, guess, &pg);
+        bool same = it == jt && ps == pg;
+        for (int k = 0; k < 5; ++k) same = same && f[k] == g[k];
+        if (!same) ++b0;
+    }
+    atomicAdd(bad, b0);
+    atomicAdd(bad + 1, plain);
+}
+extern "C" int check_exact(int n, int niter, double tol, unsigned long long* out) {
+    unsigned long long* d;
+    if (cudaMalloc(&d, 16) != cudaSuccess) return 1;
+    cudaMemset(d, 0, 16);
+    ke<<<592, 128>>>(n, niter, tol, d);
+    const int rc = cudaMemcpy(out, d, 16, cudaMemcpyDeviceToHost) != cudaSuccess;
+    cudaFree(d);
+    return rc;
+}
 extern "C" int check(int mode, int n, unsigned long long* out) {
     unsigned long long* d;
     if (cudaMalloc(&d, 16) != cudaSuccess) return 1;
@@ -85,6 +130,14 @@ def test_quotients_and_roots_are_the_ieee_ones(forms, mode):
     bad = (ctypes.c_ulonglong * 2)()
     assert forms.check(mode, 2000, bad) == 0
     assert list(bad) == [0, 0]
+
+
+@pytest.mark.parametrize("niter,tol", [(10, 1e-6), (100, 1e-14), (1, 1e-6)])
+def test_exact_solver_forms_agree(forms, niter, tol):
+    """Same iterations, pressure and flux; only the pairs above the checked range take the plain form."""
+    out = (ctypes.c_ulonglong * 2)()
+    assert forms.check_exact(60, niter, ctypes.c_double(tol), out) == 0
+    assert out[0] == 0 and 0 < out[1] < 592 * 128 * 60 // 12
 
 
 def odd_states(g, level, seed, nan):
@@ -119,6 +172,38 @@ def odd_states(g, level, seed, nan):
     if nan:
         u[rng.integers(0, 5), ids[n // 2]] = np.nan
     return u.reshape(-1)
+
+
+@pytest.mark.parametrize("level,riem,slope,itype", [(5, "hllc", 1, 1), (6, "hllc", 2, 2), (7, "exact", 1, 1),
+                                                    (11, "llf", 8, 3), (13, "hll", 1, 1), (14, "acoustic", 2, 1)])
+def test_run_of_a_line_matches_single_substeps(rgpu_lib, level, riem, slope, itype):
+    """rg_level_run over a cluster (32 .. 8192 cells; 16 cells and fewer take one block) against the substeps one by
+    one: state, primitives' successor step, time and count."""
+    g = rg_tree.build_uniform(1, level)
+    u = rg_tree.random_state(g, level, seed=level, rho_range=(-0.3, 0.3), p_range=(-0.3, 0.3))
+    dx = 1.0 / 2 ** level
+    outs = []
+    for whole in (True, False):
+        ctx = rgpu.Context(make_params(1, slope_type=slope, riemann=riem, interpol_type=itype), 0)
+        ctx.sync_topology(g)
+        ctx.upload_state(u, u)
+        if whole:
+            t, n = ctx.level_run(level, dx, 1.0, pressure_cap=True, max_steps=7)
+            t, m = ctx.level_run(level, dx, 1.0, t_start=t, pressure_cap=True, max_steps=5)
+            n += m
+        else:
+            t, n = 0.0, 0
+            for _ in range(12):
+                t += ctx.level_substep(level, dx, pressure_cap=True, use_graph=False, want_dt=True)
+                n += 1
+        dt = ctx.level_substep(level, dx, pressure_cap=True, use_graph=False, want_dt=True)
+        a, b = np.empty_like(u), np.empty_like(u)
+        ctx.download_state(a, b)
+        outs.append((t, n, dt, a, b))
+        ctx.close()
+    (t, n, dt, a, b), (t1, n1, dt1, a1, b1) = outs
+    assert (t, n, dt) == (t1, n1, dt1)
+    assert np.array_equal(a.view(np.int64), a1.view(np.int64)) and np.array_equal(b.view(np.int64), b1.view(np.int64))
 
 
 def same(a, b):

@@ -137,6 +137,7 @@ int get_plan(rg_ctx* c, int ilevel, Plan** out) {
                 p.face_variant = t.variant;
                 p.face_batch = t.batch;
                 p.face_ms = t.ms;
+                p.pinned = t.pinned;
             }
         }
     }
@@ -156,6 +157,16 @@ int ensure_flux(rg_ctx* c, const Plan& P) {
             p.graph = nullptr;
         }
     return grow(c, &c->d_flux, &c->cap_flux, need, "flux scratch");
+}
+
+// What a leaf substep of the level needs: the brick step's second primitive
+// array, or the flux scratch (also the brick step's first call, which times
+// the face shapes for rg_godunov_level as every level's first step does).
+int ensure_leaf(rg_ctx* c, const Plan& P) {
+    if (!brick_step_on(c, P) || P.face_variant < 0)
+        if (int rc = ensure_flux(c, P)) return rc;
+    if (!brick_step_on(c, P) || c->d_prim2) return RG_OK;
+    return check_cuda(c, dev_alloc(c, &c->d_prim2, sizeof(double) * (size_t)c->nvar * c->ncell), "second primitives");
 }
 
 // rg_level_run's clock: start values, then after each substep t += dt, one
@@ -316,6 +327,7 @@ void rg_destroy(rg_ctx* c) {
     dev_free(c, c->d_uold);
     dev_free(c, c->d_unew);
     dev_free(c, c->d_prim);
+    dev_free(c, c->d_prim2);
     dev_free(c, c->d_flux);
     dev_free(c, c->d_mlp);
     dev_free(c, c->d_stage);
@@ -442,6 +454,8 @@ int rg_sync_topology(rg_ctx* c, const rg_grid_view* g) {
         if (int rc = grow(c, &c->d_unew, &cap, ns, "unew")) return rc;
         cap = c->cap_state;
         if (int rc = grow(c, &c->d_prim, &cap, ns, "prim")) return rc;
+        dev_free(c, c->d_prim2);
+        c->d_prim2 = nullptr;
         c->cap_state = std::max(c->cap_state, ns);
         c->have_state = false;
     }
@@ -634,8 +648,8 @@ int rg_level_substep(rg_ctx* c, int ilevel, double dx, int pressure_cap, int use
     Plan* P;
     if (int rc = get_plan(c, ilevel, &P)) return rc;
     record_updates(c, ilevel, *P);
-    if (int rc = ensure_flux(c, *P)) return rc;
     const bool leaf = P->nactive == P->ncells;  // no refined cell: fused substep
+    if (int rc = leaf ? ensure_leaf(c, *P) : ensure_flux(c, *P)) return rc;
     const double cfl = c->params.courant_factor;
     const int cap_key = pressure_cap ? 1 : 0;
     if (leaf) {
@@ -662,6 +676,10 @@ int rg_level_substep(rg_ctx* c, int ilevel, double dx, int pressure_cap, int use
         // first substep of this plan: run it eagerly, then tune the face
         // kernel on its primitives before any graph captures the launch shape
         if (int rc = enqueue()) return rc;
+        // (the brick step's primitives are in lattice order, and after its
+        // first step in the second array: d_prim is free for the timing)
+        if (leaf && brick_step_on(c, *P))
+            if (int rc = launch_prim(c, *P)) return rc;
         if (int rc = autotune_face(c, *P, step_consts(c))) return rc;
     } else if (use_graph) {
         // a graph bakes dx, the courant factor and the pressure cap into its launches
@@ -761,6 +779,7 @@ int rg_level_run(rg_ctx* c, int ilevel, double dx, int pressure_cap, double t_st
                          "rg_level_run needs a level without refined cells whose stencils stay inside it (one box)");
     double t = t_start;
     long long n = 0;
+    if (int rc = ensure_leaf(c, *P)) return rc;
     if (P->face_variant < 0) {
         // the first substep of a plan runs eagerly and chooses the face shape
         double dt = 0.0;
@@ -775,7 +794,7 @@ int rg_level_run(rg_ctx* c, int ilevel, double dx, int pressure_cap, double t_st
         }
     }
     record_updates(c, ilevel, *P);
-    if (int rc = ensure_flux(c, *P)) return rc;
+    if (int rc = ensure_leaf(c, *P)) return rc;
     const double cfl = c->params.courant_factor;
     const int cap_key = pressure_cap ? 1 : 0;
     const bool ready = c->next_level == ilevel && c->next_cap == cap_key && c->next_dx == dx && c->next_cfl == cfl;
@@ -1049,7 +1068,13 @@ int rg_exact_stats(rg_ctx* c, int64_t* iters, int64_t* calls, int reset) {
 
 int rg_set_autotune(rg_ctx* c, int on) {
     CTX_GUARD(c);
+    c->next_level = -1;  // with and without the brick step the next primitives are in different arrays
     c->no_autotune = (on == 0);
+    for (auto& p : c->plans)
+        if (p.graph) {
+            cudaGraphExecDestroy(p.graph);
+            p.graph = nullptr;
+        }
     drop_amr_graphs(c);
     return RG_OK;
 }
@@ -1066,12 +1091,14 @@ int rg_face_config(rg_ctx* c, int ilevel, int* variant, int* batch, float* ms) {
 
 int rg_set_face_config(rg_ctx* c, int ilevel, int variant, int batch) {
     CTX_GUARD(c);
+    c->next_level = -1;  // the shapes keep the next substep's primitives in different arrays
     if (variant < 0 || variant >= kNumFaceVariants || batch < 1)
         return set_error(c, RG_ERR_ARG, "variant must be in [0, 11), batch >= 1");
     Plan* P;
     if (int rc = get_plan(c, ilevel, &P)) return rc;
     P->face_variant = variant;
     P->face_batch = batch;
+    P->pinned = true;
     remember_shape(c, *P);
     if (P->graph) {
         cudaGraphExecDestroy(P->graph);

@@ -59,6 +59,9 @@ int autotune_face(rg_ctx* c, Plan& P, const StepK& K) {
         for (int b : kBatches) {
             if (v >= kFirstPipeVariant && b != 1) continue;  // round-robin tiles / bricks: no batch
             if (v >= kFirstBrickVariant && !(P.nbox > 0 ? P.box_lattice : P.lattice)) continue;
+            // on a lattice a gathering shape never comes near the brick ones: one is timed, the default
+            if ((P.nbox > 0 ? P.box_lattice : P.lattice) && v < kFirstBrickVariant && (v != kDefaultFaceVariant || b != 1))
+                continue;
             if (v > kFirstBrickVariant && P.nbox > 0) continue;  // one boxed brick shape
             if (P.nbox > 0 && !boxed_variant_distinct(v)) continue;
             float tmin = 1e30f;

@@ -385,18 +385,32 @@ __device__ __noinline__ unsigned tile_dir_plain(const TreeView& T, const PlanVie
     return iters;
 }
 
+// Neighbours of a cell along one direction and their stencils.
+struct TileIds {
+    int l, r, ll, lr, rl, rr;
+    __device__ __forceinline__ TileIds(const PlanView& P, int idim, int p) {
+        const size_t nc = (size_t)P.ncells, s0 = 2 * (size_t)idim;
+        l = __ldg(P.icn + s0 * nc + p);
+        r = __ldg(P.icn + (s0 + 1) * nc + p);
+        ll = __ldg(P.stc + (s0 * 2 + 0) * nc + p);
+        lr = __ldg(P.stc + (s0 * 2 + 1) * nc + p);
+        rl = __ldg(P.stc + ((s0 + 1) * 2 + 0) * nc + p);
+        rr = __ldg(P.stc + ((s0 + 1) * 2 + 1) * nc + p);
+    }
+};
+
 // The same in the branch-free forms, for cells whose two interfaces are ghost
 // or zero ones; the fluxes in f.  False: not covered, take the plain forms.
 template <int NDIM, int RS, bool POW2>
 __device__ __forceinline__ bool tile_dir_fast(const TreeView& T, const PlanView& P, const double* __restrict__ prim,
-                                              int p, int c, int idim, bool z0, bool z1, double dt, const DxDiv& D,
-                                              const StepK& K, double (*f)[Dims<NDIM>::NV], unsigned& iters) {
+                                              const TileIds& I, int c, int idim, bool z0, bool z1, double dt,
+                                              const DxDiv& D, const StepK& K, double (*f)[Dims<NDIM>::NV],
+                                              unsigned& iters) {
     constexpr int NV = Dims<NDIM>::NV;
-    const size_t ncell = (size_t)T.ncell, nc = (size_t)P.ncells, s0 = 2 * (size_t)idim;
-    const int l = P.icn[s0 * nc + p], r = P.icn[(s0 + 1) * nc + p];
+    const size_t ncell = (size_t)T.ncell;
+    const int l = I.l, r = I.r;
     // stencils of the two neighbours (the cell itself stands in where no problem is solved)
-    const int ll = z0 ? c : P.stc[(s0 * 2 + 0) * nc + p], lr = z0 ? c : P.stc[(s0 * 2 + 1) * nc + p];
-    const int rl = z1 ? c : P.stc[((s0 + 1) * 2 + 0) * nc + p], rr = z1 ? c : P.stc[((s0 + 1) * 2 + 1) * nc + p];
+    const int ll = z0 ? c : I.ll, lr = z0 ? c : I.lr, rl = z1 ? c : I.rl, rr = z1 ? c : I.rr;
     if (min(min(min(l, r), min(ll, lr)), min(rl, rr)) <= 0) return false;
     double qc[NV], ql[NV], qr[NV], qf[NV], qn[NV], qmo[NV], qpo[NV], qm[NV], qp[NV];
     load_rot<NDIM>(prim, ncell, c, idim, qc);
@@ -461,10 +475,13 @@ __global__ void __launch_bounds__(TILE * NDIM * R, MINB)
             int kd0 = K_NONE;
             if (valid) {
                 const int s0 = 2 * idim;
-                kd0 = P.kind[(size_t)s0 * nc + p];
+                // every index the cell needs is asked for before any is looked at: one memory latency, then
+                // the primitives' (kinds first, then ids, then stencils were four in a row)
+                kd0 = __ldg(P.kind + (size_t)s0 * nc + p);
+                const int kd1 = __ldg(P.kind + (size_t)(s0 + 1) * nc + p);
+                const int c = cell_of(T, P, p);
+                const TileIds I(P, idim, p);
                 if (kd0 != K_NONE) {
-                    const int kd1 = P.kind[(size_t)(s0 + 1) * nc + p];
-                    const int c = cell_of(T, P, p);
                     double dt = dt0;
                     DxDiv D = D0;
                     if constexpr (BOXED) step_of_box(P, p, dt, D);
@@ -477,10 +494,10 @@ __global__ void __launch_bounds__(TILE * NDIM * R, MINB)
                         if (K.fast && (k0 == K_GHOST || k0 == K_ZERO) && (k1 == K_GHOST || k1 == K_ZERO) &&
                             D.dx > 0x1p-60 && D.dx < 0x1p60) {
                             if (D.pow2)
-                                ok = tile_dir_fast<NDIM, RS, true>(T, P, prim, p, c, idim, k0 == K_ZERO, k1 == K_ZERO, dt,
+                                ok = tile_dir_fast<NDIM, RS, true>(T, P, prim, I, c, idim, k0 == K_ZERO, k1 == K_ZERO, dt,
                                                                    D, K, f, it);
                             else
-                                ok = tile_dir_fast<NDIM, RS, false>(T, P, prim, p, c, idim, k0 == K_ZERO, k1 == K_ZERO,
+                                ok = tile_dir_fast<NDIM, RS, false>(T, P, prim, I, c, idim, k0 == K_ZERO, k1 == K_ZERO,
                                                                     dt, D, K, f, it);
                         }
                     }

@@ -18,104 +18,13 @@
 // flux sum in registers in slot order.
 #pragma once
 
-#include "rg_face.cuh"
+#include "rg_brick.cuh"
 
 namespace rg {
 
-constexpr int BRICK = 8, BHALO = 2, BSIDE = BRICK + 2 * BHALO, BSITES = BSIDE * BSIDE * BSIDE;
+constexpr int BSITES = BSIDE * BSIDE * BSIDE;
 constexpr int BRICK_THREADS = 256;
 constexpr size_t BRICK_SMEM = sizeof(double) * 5 * BSITES;  // 69,120 bytes (3D: nvar 5)
-
-// Rotated primitive state of shared-memory site `site`: the normal velocity
-// read from plane o1 into slot 1, the tangential ones from o2 and o3 (planes
-// of the direction, set once per direction by brick_planes), so the rotation
-// costs no data movement after the loads.
-__device__ __forceinline__ void brick_state(const double* __restrict__ sq, int site, int o1, int o2, int o3,
-                                            double* q) {
-    q[0] = sq[site];
-    q[1] = sq[o1 + site];
-    q[2] = sq[o2 + site];
-    q[3] = sq[o3 + site];
-    q[4] = sq[4 * BSITES + site];
-}
-
-// Planes of slots 1..3 for direction idim: rot_swap<3>'s exchange of slot 1
-// with slot 1 + idim, applied to where the values are read from.
-__device__ __forceinline__ void brick_planes(int idim, int& o1, int& o2, int& o3) {
-    o1 = (1 + idim) * BSITES;
-    o2 = (idim == 1 ? 1 : 2) * BSITES;
-    o3 = (idim == 2 ? 1 : 3) * BSITES;
-}
-
-// Lattice geometry of a level: one lattice (nbox == 0: extents ex, ey, ez) or
-// one lattice per ensemble box (extents ext[3b..3b+2], sites from off[b] in
-// the concatenated maps, bricks from brick_off[b]).
-struct BrickGeom {
-    int ex, ey, ez, nbox;
-    const int* ext;
-    const int* off;
-    const int* brick_off;
-};
-
-// Fluxes of one cell and direction in the plain forms, to the scratch.
-template <int RS>
-__device__ __noinline__ unsigned brick_dir_plain(const double* sq, int site, int idim, bool ghost, double dt,
-                                                 const DxDiv& D, const StepK& K, double* flux, int nc, int p) {
-    constexpr int NV = 5;
-    const int stride = idim == 0 ? 1 : (idim == 1 ? BSIDE : BSIDE * BSIDE);
-    int o1, o2, o3;
-    unsigned iters = 0;
-    brick_planes(idim, o1, o2, o3);
-    double qc[NV], ql[NV], qr[NV], qmo[NV], qpo[NV];
-    brick_state(sq, site, o1, o2, o3, qc);
-    brick_state(sq, site - stride, o1, o2, o3, ql);
-    brick_state(sq, site + stride, o1, o2, o3, qr);
-    own_trace<3>(qc, ql, qr, dt, D, K, qmo, qpo);
-#pragma unroll
-    for (int side = 0; side < 2; ++side) {
-        // neighbour n = c -/+ e, its stencil (n - e, n + e) = (c - 2e, c) / (c, c + 2e)
-        double qfar[NV], qm[NV], qp[NV], f[NV];
-        brick_state(sq, side ? site + 2 * stride : site - 2 * stride, o1, o2, o3, qfar);
-        const double* qn = side ? qr : ql;
-        const double* qnl = side ? qc : qfar;
-        const double* qnr = side ? qfar : qc;
-        if (ghost) ghost_trace<3>(qn, qnl, qnr, dt, D, K, qm, qp);
-        else own_trace<3>(qn, qnl, qnr, dt, D, K, qm, qp);
-        if (side == 0) iters += riemann<3, RS>(qm, qpo, f, K);
-        else iters += riemann<3, RS>(qmo, qp, f, K);
-        rot_swap<3>(f, idim);
-#pragma unroll
-        for (int iv = 0; iv < NV; ++iv) flux[((size_t)(2 * idim + side) * NV + iv) * nc + p] = f[iv];
-    }
-    return iters;
-}
-
-// The two fluxes of one cell and direction in the branch-free forms (a ghost
-// neighbour on both sides); false: not covered, take the plain forms.
-template <int RS, bool POW2>
-__device__ __forceinline__ bool brick_dir_fast(const double* __restrict__ sq, int site, int idim, const FastStep& S,
-                                               const FastStep& Sc, const StepK& K, double* f0, double* f1,
-                                               unsigned& iters) {
-    constexpr int NV = 5;
-    const int stride = idim == 0 ? 1 : (idim == 1 ? BSIDE : BSIDE * BSIDE);
-    int o1, o2, o3;
-    brick_planes(idim, o1, o2, o3);
-    double qc[NV], ql[NV], qr[NV], qfl[NV], qfr[NV], qmo[NV], qpo[NV], qm[NV], qp[NV];
-    brick_state(sq, site, o1, o2, o3, qc);
-    brick_state(sq, site - stride, o1, o2, o3, ql);
-    brick_state(sq, site + stride, o1, o2, o3, qr);
-    brick_state(sq, site - 2 * stride, o1, o2, o3, qfl);
-    brick_state(sq, site + 2 * stride, o1, o2, o3, qfr);
-    Check C;
-    trace_fast<3, POW2, false, true, true>(qc, ql, qr, K.own, S, K.gamma, qmo, qpo, C);
-    trace_fast<3, POW2, false, true, false>(ql, qfl, qc, K.ghost, Sc, K.gamma, qm, nullptr, C);
-    trace_fast<3, POW2, false, false, true>(qr, qc, qfr, K.ghost, Sc, K.gamma, nullptr, qp, C);
-    const bool ok = C.num_ok();
-    const bool a = riemann_fast<3, RS>(qm, qpo, f0, K, iters), b = riemann_fast<3, RS>(qmo, qp, f1, K, iters);
-    rot_swap<3>(f0, idim);
-    rot_swap<3>(f1, idim);
-    return ok && a && b;
-}
 
 // One cell of a brick: its fluxes in the three directions to the scratch, its
 // own flux sum in slot order.
@@ -133,15 +42,17 @@ __device__ __forceinline__ void brick_cell(const double* sq, int site, int p, in
         double* out = flux + (size_t)(2 * idim * NV) * nc + p;
         unsigned it = 0;
         bool ok = false;
-        if (FAST) ok = brick_dir_fast<RS, POW2>(sq, site, idim, S, Sc, K, f[0], f[1], it);
-        if (FAST && ok) {
+        const int stride = idim == 0 ? 1 : (idim == 1 ? BSIDE : BSIDE * BSIDE);
+        if (FAST) ok = brick_dir_fast<RS, POW2, BSITES>(sq, site, idim, stride, S, Sc, K, f[0], f[1], it);
+        if (!ok) {
+            double g[2 * NV];  // (the call's array lives in memory, the loop's in registers)
+            it = brick_face_plain<RS, BSITES>(sq, site, idim, stride, 0, ghost, dt, D, K, g) +
+                 brick_face_plain<RS, BSITES>(sq, site, idim, stride, 1, ghost, dt, D, K, g + NV);
 #pragma unroll
-            for (int k = 0; k < 2 * NV; ++k) out[(size_t)k * nc] = f[k / NV][k % NV];
-        } else {
-            it = brick_dir_plain<RS>(sq, site, idim, ghost, dt, D, K, flux, nc, p);
-#pragma unroll
-            for (int k = 0; k < 2 * NV; ++k) f[k / NV][k % NV] = out[(size_t)k * nc];
+            for (int k = 0; k < 2 * NV; ++k) f[k / NV][k % NV] = g[k];
         }
+#pragma unroll
+        for (int k = 0; k < 2 * NV; ++k) out[(size_t)k * nc] = f[k / NV][k % NV];
         iters += it;
 #pragma unroll
         for (int iv = 0; iv < NV; ++iv) fs[iv] = (fs[iv] + f[0][iv]) - f[1][iv];

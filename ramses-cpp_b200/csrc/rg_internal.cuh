@@ -58,7 +58,8 @@ struct DevStatus {
     double run_t;                                 // rg_level_run: the level's time and
     long long run_steps;                          // substeps, advanced on the device,
     long long run_limit;                          // and the step count this launch stops at
-    unsigned int cfl_done, cfl_pad;               // blocks of a CFL pass done (its clock update)
+    unsigned int cfl_done;                        // blocks of a CFL pass done (its clock update)
+    int prim_sel;  // the brick step's primitives are read from d_prim (0) or d_prim2 (1)
 };
 
 // The resident AMR step's clock update after a level's CFL pass
@@ -153,6 +154,7 @@ struct Plan {
     double graph_dx = 0.0, graph_cfl = 0.0;
     int face_variant = -1, face_batch = 4;  // autotuned face-kernel shape (-1: not tuned yet)
     float face_ms = 0.f;
+    bool pinned = false;  // by rg_set_face_config
     int substeps_run = 0;
     int line = -1;             // 1D: one periodic line in list order (-1: not looked at; rg_run1d.cu)
     int lattice = 0;           // the level is one complete periodic lattice (rg_lattice.cu)
@@ -160,6 +162,7 @@ struct Plan {
     int lat_kind = 0;          // the (single) interface kind of its faces
     int* lat_id = nullptr;     // [ex*ey*ez] cell id of each lattice site (x fastest)
     int* lat_p = nullptr;      // [ex*ey*ez] plan position of each site
+    int* lat_ord = nullptr;    // [sites] each cell's seven updates in loop order, 3 bits each (slot, 7 its own)
     // ensemble levels whose boxes are each one periodic lattice: per box its
     // extent, its first site in lat_id/lat_p and its first brick
     int box_lattice = 0;
@@ -195,6 +198,7 @@ struct Plan {
 struct TunedShape {
     int variant = -1, batch = 1, ncells = 0;
     float ms = 0.f;
+    bool pinned = false;
 };
 
 // A captured run of the resident AMR coarse step (rg_amr.cu: the level-step
@@ -241,6 +245,7 @@ struct rg_ctx {
     // state
     size_t cap_state = 0;
     double *d_uold = nullptr, *d_unew = nullptr, *d_prim = nullptr;
+    double* d_prim2 = nullptr;  // the brick step's second primitive array (made on first use)
     bool have_state = false;
 
     // scratch shared by all levels (levels run one after another on the stream)
@@ -407,6 +412,8 @@ Plan* existing_plan(rg_ctx* c, int ilevel);  // built plan or nullptr; never bui
 void drop_amr_graphs(rg_ctx* c);
 int compute_cell_levels(rg_ctx* c);
 // step launchers (enqueue only)
+// the primitives of the level's cells and stencil cells from uold, by cell id
+int launch_prim(rg_ctx* c, const Plan& p);
 int launch_set_unew(rg_ctx* c, const Plan& p);
 int launch_set_uold(rg_ctx* c, const Plan& p);
 // set_unew: also HydroSolver::set_unew of the level in the same pass;
@@ -441,6 +448,16 @@ int launch_leaf_core(rg_ctx* c, const Plan& p, double dx, int pressure_cap, doub
 // a leaf level whose stencils and updates stay inside it: its fold can prepare
 // the next substep
 inline bool leaf_fusable(const Plan& P) { return P.nextra_prim == 0 && P.ntarg == P.ncells && !P.level0; }
+// The substep of such a level in one kernel (rg_brick_step.cuh): a lattice (of
+// one grid or of every box) whose update order is known, unless a face shape
+// was pinned or the choice of shapes is off.  Up to kRunBlockCells cells the
+// run kernel's arrays are used.
+inline bool brick_step_on(const rg_ctx* c, const Plan& P) {
+    return P.lat_ord && leaf_fusable(P) && P.nactive == P.ncells && P.ncells > kRunBlockCells && !P.pinned &&
+           !c->no_autotune && (P.nbox > 0 ? P.box_lattice != 0 : P.lattice != 0);
+}
+int launch_brick_prefix(rg_ctx* c, const Plan& P, double dx, int pressure_cap, double courant_factor);
+int launch_brick_step(rg_ctx* c, const Plan& P, double dx, int pressure_cap, double courant_factor);
 int launch_godunov_ext(rg_ctx* c, const Plan& p, const double* uold, double* unew, double* prim, double* flux);
 TreeView tree_view(const rg_ctx* c);
 void remember_shape(rg_ctx* c, const Plan& P);

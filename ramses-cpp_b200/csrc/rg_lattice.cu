@@ -150,11 +150,77 @@ __global__ void k_box_lattice_check(TreeView T, PlanView P, int nbox, const int*
     }
 }
 
+// Each site's updates in loop order as a word of 3-bit slots (OWN_SLOT: the
+// cell's own), from its event list; the list must hold the cell's own update
+// and one reflux from each lattice neighbour through the face they share.
+// One lattice (nbox 0, extents ex, ey, ez) or one per box.
+__global__ void k_lattice_order(PlanView P, int nbox, int ex, int ey, int ez, const int* __restrict__ ext,
+                                const int* __restrict__ off, const int* __restrict__ lat_p, int* ord, int* bad) {
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < P.ncells; g += gridDim.x * blockDim.x) {
+        int base = 0;
+        if (nbox > 0) {
+            int lo = 0, hi = nbox - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (off[mid] <= g) lo = mid;
+                else hi = mid - 1;
+            }
+            base = off[lo];
+            ex = ext[3 * lo];
+            ey = ext[3 * lo + 1];
+            ez = ext[3 * lo + 2];
+        }
+        const int site = g - base, x = site % ex, y = (site / ex) % ey, z = site / (ex * ey);
+        const int p = lat_p[g], a = P.toff[p];
+        bool ok = P.toff[p + 1] - a == 7;
+        int word = 0, seen = 0;
+        for (int e = 0; ok && e < 7; ++e) {
+            const int key = P.tev[a + e], slot = key & 7, cp = key >> 3;
+            const int ps = (cp & 7) * P.noct + (cp >> 3);
+            int xx = x, yy = y, zz = z;
+            if (slot != OWN_SLOT) {  // the source whose face `slot` is shared with this cell
+                const int d = slot & 1 ? -1 : 1;
+                if (slot < 2) xx = wrap(x + d, ex);
+                else if (slot < 4) yy = wrap(y + d, ey);
+                else zz = wrap(z + d, ez);
+            }
+            ok = slot != 6 && ps == lat_p[base + xx + ex * (yy + ey * zz)];
+            seen |= 1 << slot;
+            word |= slot << (3 * e);
+        }
+        if (!ok || seen != 0xbf) atomicExch(bad, 1);
+        ord[g] = word;
+    }
+}
+
 int lblocks(rg_ctx* c, long long n) {
     long long b = (n + LTPB - 1) / LTPB, cap = (long long)c->sm_count * 16;
     return (int)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
+}  // namespace
+
+namespace {
+// the update order of an accepted lattice (left out, not an error, when the
+// event lists are not the lattice's)
+int build_order(rg_ctx* c, Plan& P) {
+    int* d_bad = nullptr;
+    int bad = 1;
+    if (P.ntarg != P.ncells) return RG_OK;
+    if (int rc = check_cuda(c, dev_alloc(c, &d_bad, sizeof(int)), "lattice order flag")) return rc;
+    if (int rc = check_cuda(c, dev_alloc(c, &P.lat_ord, sizeof(int) * (size_t)P.ncells), "lattice order")) return rc;
+    cudaMemsetAsync(d_bad, 0, sizeof(int), c->stream);
+    k_lattice_order<<<lblocks(c, P.ncells), LTPB, 0, c->stream>>>(P.view(), P.nbox, P.lat_e[0], P.lat_e[1], P.lat_e[2],
+                                                                  P.bl_ext, P.bl_off, P.lat_p, P.lat_ord, d_bad);
+    cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    const cudaError_t e = cudaStreamSynchronize(c->stream);
+    dev_free(c, d_bad);
+    if (bad || e != cudaSuccess) {
+        dev_free(c, P.lat_ord);
+        P.lat_ord = nullptr;
+    }
+    return check_cuda(c, e, "lattice order");
+}
 }  // namespace
 
 // Accepts the level as a lattice (P.lattice = 1, lat_id/lat_p filled) or
@@ -206,7 +272,7 @@ int build_lattice(rg_ctx* c, Plan& P) {
     P.lat_e[1] = (int)ey;
     P.lat_e[2] = (int)ez;
     P.lat_kind = kd;
-    return RG_OK;
+    return build_order(c, P);
 }
 
 int set_box_lattices(rg_ctx* c, Plan& P, const int* ext, const int* lat_id, const int* lat_p) {
@@ -235,7 +301,8 @@ int set_box_lattices(rg_ctx* c, Plan& P, const int* ext, const int* lat_id, cons
         dev_free(c, P.bl_ext);
         dev_free(c, P.bl_off);
         dev_free(c, P.bl_brick_off);
-        P.lat_id = P.lat_p = P.bl_ext = P.bl_off = P.bl_brick_off = nullptr;
+        dev_free(c, P.lat_ord);
+        P.lat_id = P.lat_p = P.lat_ord = P.bl_ext = P.bl_off = P.bl_brick_off = nullptr;
         P.box_lattice = 0;
         return rc;
     };
@@ -273,7 +340,7 @@ int set_box_lattices(rg_ctx* c, Plan& P, const int* ext, const int* lat_id, cons
     P.box_lattice = 1;
     P.bl_nbricks = (int)bricks;
     P.lat_kind = kind0;
-    return RG_OK;
+    return build_order(c, P);
 }
 
 }  // namespace rg

@@ -523,7 +523,10 @@ __global__ void k_courant_prim(TreeView T, PlanView P, const double* __restrict_
     block_atomic_min(best, &st->dtmin_bits);
 }
 
+// (the brick step's next substep reads d_prim, which the pass after this
+// writes: the step's finalize turns prim_sel over first)
 __global__ void k_courant_init(DevStatus* st, double dt_start) {
+    st->prim_sel = 1;
     st->dtmin_bits = (unsigned long long)__double_as_longlong(dt_start);
 }
 __device__ __forceinline__ void set_step_values(DevStatus* st, double dt, double dx) {
@@ -539,16 +542,19 @@ __device__ __forceinline__ void set_step_values(DevStatus* st, double dt, double
 __global__ void k_dt_finalize(DevStatus* st, double dx, double dt_start) {
     set_step_values(st, __longlong_as_double((long long)st->dtmin_bits), dx);
     st->dtmin_bits = (unsigned long long)__double_as_longlong(dt_start);
+    st->prim_sel ^= 1;
 }
 __global__ void k_dt_set(DevStatus* st, double dt, double dx) { set_step_values(st, dt, dx); }
 __global__ void k_dt_set_dev(DevStatus* st, const double* dt, double dx) { set_step_values(st, *dt, dx); }
 
 // ---- ensemble levels: one CFL step per box
-__global__ void k_box_courant_init(BoxStep* boxes, int nbox, double dt_start) {
+__global__ void k_box_courant_init(BoxStep* boxes, int nbox, double dt_start, DevStatus* st) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->prim_sel = 1;
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nbox; b += gridDim.x * blockDim.x)
         boxes[b].dtmin_bits = (unsigned long long)__double_as_longlong(dt_start);
 }
-__global__ void k_box_dt_finalize(BoxStep* boxes, int nbox, double dt_start) {
+__global__ void k_box_dt_finalize(BoxStep* boxes, int nbox, double dt_start, DevStatus* st) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->prim_sel ^= 1;
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nbox; b += gridDim.x * blockDim.x) {
         BoxStep& B = boxes[b];
         const double dt = __longlong_as_double((long long)B.dtmin_bits), dx = B.dx;
@@ -742,12 +748,20 @@ void launch_leaf_prefix_t(rg_ctx* c, const Plan& P, double dx, int pressure_cap,
     const double start = c->params.boxlen / 1e-10;
     if (P.nbox > 0) {
         const int bb = (P.nbox + 127) / 128;
-        k_box_courant_init<<<bb, 128, 0, c->stream>>>(P.boxes, P.nbox, start);
+        k_box_courant_init<<<bb, 128, 0, c->stream>>>(P.boxes, P.nbox, start, c->d_status);
+        if (NDIM == 3 && brick_step_on(c, P)) {
+            launch_brick_prefix(c, P, dx, pressure_cap, cfl);  // (the caller checks for launch errors)
+            return;
+        }
         k_courant_prim_boxes<NDIM><<<grid_for(c, nprim, 256), 256, 0, c->stream>>>(T, V, c->d_uold, c->d_prim,
                                                                                    K.gamma, K.smalle, cfl,
                                                                                    pressure_cap);
     } else {
         k_courant_init<<<1, 1, 0, c->stream>>>(c->d_status, start);
+        if (NDIM == 3 && brick_step_on(c, P)) {
+            launch_brick_prefix(c, P, dx, pressure_cap, cfl);
+            return;
+        }
         k_courant_prim<NDIM><<<grid_for(c, nprim, 256), 256, 0, c->stream>>>(T, V, c->d_uold, c->d_prim,
                                                                              c->d_status, dx, K.gamma, K.smalle,
                                                                              cfl, pressure_cap);
@@ -762,9 +776,16 @@ int launch_leaf_core_t(rg_ctx* c, const Plan& P, double dx, int pressure_cap, do
     TreeView T = tree_view(c);
     PlanView V = P.view();
     const double start = c->params.boxlen / 1e-10;
-    if (P.nbox > 0) k_box_dt_finalize<<<(P.nbox + 127) / 128, 128, 0, c->stream>>>(P.boxes, P.nbox, start);
+    if (P.nbox > 0) k_box_dt_finalize<<<(P.nbox + 127) / 128, 128, 0, c->stream>>>(P.boxes, P.nbox, start, c->d_status);
     else k_dt_finalize<<<1, 1, 0, c->stream>>>(c->d_status, dx, start);
     if (c->timing) cudaEventRecord(c->ev[1], c->stream);
+    if (NDIM == 3 && brick_step_on(c, P)) {
+        // face and fold in one kernel: its time counts as the face step's
+        if (int rc = launch_brick_step(c, P, dx, pressure_cap, cfl)) return rc;
+        if (c->timing) cudaEventRecord(c->ev[2], c->stream);
+        if (c->timing) cudaEventRecord(c->ev[3], c->stream);
+        return RG_OK;
+    }
     double* fsum = c->d_flux + (size_t)(2 * NDIM) * (NDIM + 2) * P.ncells;
     if (int rc = launch_face_tiles(c, P, K, c->d_uold, c->d_prim, c->d_flux, fsum)) return rc;
     if (c->timing) cudaEventRecord(c->ev[2], c->stream);
@@ -800,10 +821,24 @@ int launch_leaf_prefix(rg_ctx* c, const Plan& P, double dx, int pressure_cap, do
 
 int launch_leaf_core(rg_ctx* c, const Plan& P, double dx, int pressure_cap, double cfl) {
     if (P.ncells == 0) return RG_OK;
-    if (c->cap_flux < (size_t)(2 * c->params.ndim + 1) * (c->params.ndim + 2) * P.ncells)
+    if (brick_step_on(c, P)) {
+        if (!c->d_prim2) return set_error(c, RG_ERR_STATE, "second primitive array not there");
+    } else if (c->cap_flux < (size_t)(2 * c->params.ndim + 1) * (c->params.ndim + 2) * P.ncells) {
         return set_error(c, RG_ERR_STATE, "flux scratch not sized");
+    }
     if (c->params.ndim == 1) return launch_leaf_core_t<1>(c, P, dx, pressure_cap, cfl);
     return launch_leaf_core_t<3>(c, P, dx, pressure_cap, cfl);
+}
+
+int launch_prim(rg_ctx* c, const Plan& P) {
+    const StepK K = step_consts(c);
+    const int n = P.ncells + P.nextra_prim;
+    if (n == 0) return RG_OK;
+    if (c->params.ndim == 1)
+        k_prim<1><<<grid_for(c, n, 256), 256, 0, c->stream>>>(tree_view(c), P.view(), c->d_uold, c->d_prim, K.gamma, K.smalle);
+    else
+        k_prim<3><<<grid_for(c, n, 256), 256, 0, c->stream>>>(tree_view(c), P.view(), c->d_uold, c->d_prim, K.gamma, K.smalle);
+    return check_cuda(c, cudaGetLastError(), "primitives");
 }
 
 int launch_set_unew(rg_ctx* c, const Plan& P) {

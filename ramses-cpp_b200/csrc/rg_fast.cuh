@@ -31,11 +31,15 @@
 
 namespace rg {
 
+// RN(1/b).  The last step rounds correctly from any value within an ulp of
+// 1/b, but for a divisor whose significand is all ones only from above (from
+// below it meets a tie: b = 1 - 2^-53 would give 1, and 1/b with it); so the
+// cubic step adds 2^-55, more than its error and a quarter ulp at most.
 __device__ __forceinline__ double rcp_fast(double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
     const double e = fma(-b, y, 1.0);
-    y = fma(y, fma(e, e, e), y);
+    y = fma(y, fma(e, fma(-b, y, 2.0), 0x1p-55), y);
     return fma(y, fma(-b, y, 1.0), y);
 }
 // a / b with y = rcp_fast(b) (or the correctly rounded 1 / b)

@@ -36,7 +36,7 @@ __global__ void k(int mode, int n, unsigned long long* bad) {
     for (int i = 0; i < n; ++i) {
         uint64_t ra = rnd(s), rb = rnd(s);
         const int ea = (int)(rnd(s) % 1200) - 600, eb = (int)(rnd(s) % 700) - 130;
-        if (mode == 1) rb = ~(rb % 64);                       // divisors just below a power of two
+        if (mode == 1 || mode == 5) rb = ~(rb % 64);          // divisors just below a power of two
         if (mode == 2) { ra = ~(ra % 4096); rb = ~(rb % 4096); }
         if (mode == 3) { ra = ra & 1 ? ~(ra % 4096) : ra % 4096; rb = rb % 4096; }
         const double b = make(rb, eb);
@@ -45,7 +45,9 @@ __global__ void k(int mode, int n, unsigned long long* bad) {
             const double q = make(ra, 0);
             a = fma(b, q * 0x1p-53, b * q);
         }
+        if (mode == 5) a = make(0, ea);                           // powers of two over divisors of mode 1
         if (rb >> 63) a = -a;
+        if (rg::rcp_fast(b) != 1.0 / b) ++b0;
         if (rg::div_by(a, b, rg::rcp_fast(b)) != a / b) ++b0;
         const double x = make(ra, (ea & 1 ? 1 : 0) + 2 * (ea / 8));
         if (rg::sqrt_fast(x) != sqrt(x)) ++b1;
@@ -125,7 +127,7 @@ def forms(tmp_path_factory):
     return ctypes.CDLL(str(d / "t.so"))
 
 
-@pytest.mark.parametrize("mode", range(5))
+@pytest.mark.parametrize("mode", range(6))
 def test_quotients_and_roots_are_the_ieee_ones(forms, mode):
     bad = (ctypes.c_ulonglong * 2)()
     assert forms.check(mode, 2000, bad) == 0
@@ -234,5 +236,35 @@ def test_level_step_at_the_limits_matches_the_oracle(rgpu_lib, oracle, nx, level
             got = np.empty_like(unew)
             ctx.download_state(unew=got)
             assert same(got, unew), f"{np.count_nonzero(got != unew)} values differ"
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("nx,level,riem,slope,itype", [(1, 5, "hllc", 2, 1), (3, 4, "llf", 1, 2), (3, 4, "hll", 8, 3),
+                                                       (1, 5, "acoustic", 2, 1), (3, 4, "hllc", 4, 1)])
+def test_brick_step_at_the_limits_matches_the_oracle(rgpu_lib, oracle, nx, level, riem, slope, itype):
+    """Leaf substeps of lattice levels (one kernel a substep, graph and eager mixed, a pinned shape in between)."""
+    g = rg_tree.build_uniform(3, level, nx=nx, ny=nx, nz=nx)
+    ga = ga_of(g)
+    params = make_params(3, slope_type=slope, riemann=riem, interpol_type=itype)
+    ctx = rgpu.Context(params, 0)
+    try:
+        ctx.sync_topology(g)
+        dx = 1.0 / (nx * 2 ** level)
+        for seed in (3, 4):
+            u = odd_states(g, level, seed, False)
+            unew = u.copy()
+            ctx.upload_state(u, unew)
+            for k in range(5):
+                if k == 3:
+                    ctx.set_face_config(level, 10, 1)  # face and fold kernels from here on
+                dt = ctx.level_substep(level, dx, use_graph=k % 2 == 0, want_dt=True)
+                assert dt == oracle.courant(ga, 3, 5, level, dx, 1.4, 0.8, u, pressure_cap=False)
+                oracle.set_unew(ga, 3, 5, level, u, unew)
+                oracle.godunov_fine(ga, params, level, dt, dx, u, unew)
+                oracle.set_uold(ga, 3, 5, level, u, unew)
+                a, b = np.empty_like(u), np.empty_like(u)
+                ctx.download_state(a, b)
+                assert same(a, u) and same(b, unew), (seed, k)
     finally:
         ctx.close()

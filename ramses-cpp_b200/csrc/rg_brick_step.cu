@@ -11,10 +11,10 @@ int launch_brick_prefix(rg_ctx* c, const Plan& P, double dx, int pressure_cap, d
     const int blocks = std::min((P.ncells + 255) / 256, c->sm_count * 32);
     if (P.nbox > 0)
         k_brick_prefix<true><<<blocks, 256, 0, c->stream>>>(P.view(), G, P.lat_id, c->d_uold, c->d_prim, (size_t)c->ncell,
-                                                            c->d_status, dx, K.gamma, K.smalle, cfl, pressure_cap);
+                                                            c->d_status, dx, K.gas, K.smalle, cfl_consts(cfl, pressure_cap));
     else
         k_brick_prefix<false><<<blocks, 256, 0, c->stream>>>(P.view(), G, P.lat_id, c->d_uold, c->d_prim, (size_t)c->ncell,
-                                                             c->d_status, dx, K.gamma, K.smalle, cfl, pressure_cap);
+                                                             c->d_status, dx, K.gas, K.smalle, cfl_consts(cfl, pressure_cap));
     return check_cuda(c, cudaGetLastError(), "brick step primitives");
 }
 

@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(SCELLS, 2)
     k_brick_step(const __grid_constant__ PlanView P, BrickGeom G, const int* __restrict__ lat_id,
                  const int* __restrict__ lat_ord, int kind, double* __restrict__ prim0, double* __restrict__ prim1,
                  size_t ncell, double* __restrict__ uold, double* __restrict__ unew, DevStatus* st,
-                 const __grid_constant__ StepK K, double dx, double cfl, int pressure_cap) {
+                 const __grid_constant__ StepK K, double dx, CflK F) {
     constexpr int NV = 5;
     extern __shared__ __align__(16) double sq[];  // primitives [NV][SSITES], then incoming fluxes [6][NV][SCELLS]
     double* in = sq + NV * SSITES;
@@ -82,7 +82,10 @@ __global__ void __launch_bounds__(SCELLS, 2)
     Check C;
     // rows of the brick are six pairs of sites, whole pairs on either side of a wrap
     constexpr int PAIRS = SSITES / 2;
-    for (int t = threadIdx.x; t < PAIRS; t += SCELLS) {
+#pragma unroll
+    for (int k = 0; k < (PAIRS + SCELLS - 1) / SCELLS; ++k) {
+        const int t = (int)threadIdx.x + k * SCELLS;
+        if (t >= PAIRS) break;
         const int a = 2 * (t % (BSIDE / 2)), b = (t / (BSIDE / 2)) % BSIDE, cz = t / (SPLANE / 2);
         int x = x0 + a, y = y0 + b, z = z0 + cz;
         x = x < 0 ? x + ex : (x >= ex ? x - ex : x);
@@ -148,6 +151,9 @@ __global__ void __launch_bounds__(SCELLS, 2)
 #pragma unroll
         for (int iv = 0; iv < NV; ++iv) fs[iv] = (fs[iv] + f[0][iv]) - f[1][iv];
     }
+    double v[NV];  // asked for here, needed after the next problem
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) v[iv] = uold[iv * ncell + id];
     // the faces of the cells around the brick towards it: 32 on each x and y
     // side, 64 on each z side, one a thread; the outside cell's slot `side` is
     // the face it shares with the inside cell (cx, cy, cz)
@@ -177,9 +183,6 @@ __global__ void __launch_bounds__(SCELLS, 2)
 #pragma unroll
         for (int iv = 0; iv < NV; ++iv) to[iv * SCELLS] = f[iv];
     }
-    double v[NV];
-#pragma unroll
-    for (int iv = 0; iv < NV; ++iv) v[iv] = uold[iv * ncell + id];
     __syncthreads();
     // the seven updates in loop order (3 bits each: the slot, 7 the cell's own)
     auto reflux = [&](int slot) {
@@ -190,19 +193,18 @@ __global__ void __launch_bounds__(SCELLS, 2)
     };
     int left = 7;
     for (; (ord & 7) != OWN_SLOT; ord >>= 3, --left) reflux(ord & 7);
-    own_update<3>(fs, K.gamma, dtdx, v);
+    own_update<3>(fs, K.gas, dtdx, v);
     ord >>= 3;
     for (--left; left > 0; ord >>= 3, --left) reflux(ord & 7);
     double q[NV];
-    ctoprim<3>(v, q, K.gamma, K.smalle);
+    unsigned long long best = ~0ULL, bits;
+    if (prim_cfl<3, true, true>(v, q, dx, K.gas, K.smalle, F, &bits)) best = bits;
 #pragma unroll
     for (int iv = 0; iv < NV; ++iv) {
         unew[iv * ncell + id] = v[iv];
         uold[iv * ncell + id] = v[iv];
         prim_out[iv * pitch + first + lsite] = q[iv];
     }
-    unsigned long long best = ~0ULL, bits;
-    if (cfl_candidate<3>(v, dx, K.gamma, cfl, pressure_cap, &bits)) best = bits;
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
         best = other < best ? other : best;
@@ -225,8 +227,8 @@ __global__ void __launch_bounds__(SCELLS, 2)
 template <bool BOXED>
 __global__ void __launch_bounds__(256)
     k_brick_prefix(PlanView P, BrickGeom G, const int* __restrict__ lat_id, const double* __restrict__ uold,
-                   double* __restrict__ prim, size_t ncell, DevStatus* st, double dx, double gamma, double smalle,
-                   double cfl, int pressure_cap) {
+                   double* __restrict__ prim, size_t ncell, DevStatus* st, double dx,
+                   const __grid_constant__ FastGas gas, double smalle, CflK F) {
     constexpr int NV = 5;
     const int lane = threadIdx.x & 31;
     unsigned long long all = ~0ULL;
@@ -248,10 +250,9 @@ __global__ void __launch_bounds__(256)
             double u[NV], q[NV];
 #pragma unroll
             for (int iv = 0; iv < NV; ++iv) u[iv] = uold[iv * ncell + id];
-            ctoprim<3>(u, q, gamma, smalle);
+            if (prim_cfl<3, true, true>(u, q, BOXED ? P.boxes[box].dx : dx, gas, smalle, F, &bits)) best = bits;
 #pragma unroll
             for (int iv = 0; iv < NV; ++iv) prim[iv * (size_t)P.ncells + g] = q[iv];
-            if (cfl_candidate<3>(u, BOXED ? P.boxes[box].dx : dx, gamma, cfl, pressure_cap, &bits)) best = bits;
         }
         if constexpr (BOXED) {
             for (int o = 16; o > 0; o >>= 1) {
@@ -286,7 +287,7 @@ int launch_brick_step_t(rg_ctx* c, const Plan& P, double dx, int pressure_cap, d
     const BrickGeom G{P.lat_e[0], P.lat_e[1], P.lat_e[2], P.nbox, P.bl_ext, P.bl_off, P.bl_brick_off};
     kern<<<P.ncells / SCELLS, SCELLS, STEP_SMEM, c->stream>>>(P.view(), G, P.lat_id, P.lat_ord, P.lat_kind, c->d_prim,
                                                               c->d_prim2, (size_t)c->ncell, c->d_uold, c->d_unew,
-                                                              c->d_status, step_consts(c), dx, cfl, pressure_cap);
+                                                              c->d_status, step_consts(c), dx, cfl_consts(cfl, pressure_cap));
     return check_cuda(c, cudaGetLastError(), "brick step kernel");
 }
 

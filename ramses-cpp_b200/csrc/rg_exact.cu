@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(256, 4) k_exact_batch(int n, const double* __r
             // one reciprocal of gamma for the solver's three quotients by it
             const double y = rcp_fast(gamma), gm1 = gamma - 1.0;
             const FastGas G{gamma, gm1, rcp_fast(gm1), div_by(1e-10 * 1e-10, gamma, y),
-                            div_by(gamma + 1.0, 2.0 * gamma, 0.5 * y), div_by(1.0, gamma, y)};
+                            div_by(gamma + 1.0, 2.0 * gamma, 0.5 * y), div_by(1.0, gamma, y), 1};
             ok = exact_fast<NDIM>(a, b, f, G, niter, tol, guess, &ps, &it);
         }
         if (!ok) {

@@ -151,6 +151,7 @@ __device__ __forceinline__ void trace_fast(const double* q, const double* ql, co
 struct FastGas {
     double gamma, gm1, rgm1, smallp;
     double g6, rg;  // (gamma + 1) / (2 gamma) and 1 / gamma: the exact solver's
+    int fast;       // gamma - 1 in 2^-20 .. 2^20: quotients by it may use rgm1
 };
 
 // compute_flux and prim_to_cons of one state

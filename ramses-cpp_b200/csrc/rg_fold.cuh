@@ -7,6 +7,8 @@
 #include "rg_internal.cuh"
 #include "rg_physics.cuh"
 
+#include <cmath>
+
 namespace rg {
 namespace {
 
@@ -15,9 +17,11 @@ namespace {
 // the CPU loop order to u (the target's starting state).
 // FSUM: the face kernel stored each cell's own flux sum (fsum [nvar][ncells]),
 // so the own update reads it instead of re-adding the 2*ndim slots.
-// Own update with its clamps (HydroSolver.cpp:485-547).
+// Own update with its clamps (HydroSolver.cpp:485-547).  The three quotients
+// share the reciprocal of the clamped density, which lies in [1e-10, 1e6] (or
+// is NaN); a momentum too small for div_by's range squares to zero either way.
 template <int NDIM>
-__device__ __forceinline__ void own_update(const double* fs, double gamma, double dtdx, double* u) {
+__device__ __forceinline__ void own_update(const double* fs, const FastGas& G, double dtdx, double* u) {
     constexpr int NV = Dims<NDIM>::NV;
 #pragma unroll
     for (int iv = 0; iv < NV; ++iv) u[iv] = u[iv] + dtdx * fs[iv];
@@ -25,17 +29,19 @@ __device__ __forceinline__ void own_update(const double* fs, double gamma, doubl
     u[0] = d;
 #pragma unroll
     for (int i = 1; i <= NDIM; ++i) u[i] = sclamp(u[i], -d * 10.0, d * 10.0);
+    const double y = rcp_fast(d);
     double v2 = 0.0;
 #pragma unroll
     for (int i = 1; i <= NDIM; ++i) {
-        double v = u[i] / d;
+        double v = div_by(u[i], d, y);
         v2 = v2 + v * v;
     }
     constexpr int IE = NDIM + 1;
     double ei = u[IE] - 0.5 * d * v2;
-    if (ei < d * 1e-10 / (gamma - 1.0)) {
+    const double floor_e = G.fast ? div_by(d * 1e-10, G.gm1, G.rgm1) : d * 1e-10 / G.gm1;
+    if (ei < floor_e) {
         double e_non = 0;
-        u[IE] = d * 1e-10 / (gamma - 1.0) + 0.5 * d * v2 + e_non;
+        u[IE] = floor_e + 0.5 * d * v2 + e_non;
     }
     u[IE] = smin(u[IE], d * 1e8);
 }
@@ -45,7 +51,7 @@ __device__ __forceinline__ void own_update(const double* fs, double gamma, doubl
 // 12 GB flux scratch, 35 planes in flight per warp measured slower.
 template <int NDIM, bool FSUM, bool BATCH = true>
 __device__ __forceinline__ void fold_events(const PlanView& P, int a, int b, const double* __restrict__ flux,
-                                            const double* __restrict__ fsum, double gamma, double dtdx, double* u) {
+                                            const double* __restrict__ fsum, const FastGas& G, double dtdx, double* u) {
     constexpr int NV = Dims<NDIM>::NV, NS = Dims<NDIM>::NS, TTD = Dims<NDIM>::TTD;
     const int nc = P.ncells;
     const double factor = 1.0 / (1 << NDIM);
@@ -68,7 +74,7 @@ __device__ __forceinline__ void fold_events(const PlanView& P, int a, int b, con
 #pragma unroll
         for (int e = 0; e <= NS; ++e) {
             if (slots[e] == OWN_SLOT) {
-                own_update<NDIM>(v[e], gamma, dtdx, u);
+                own_update<NDIM>(v[e], G, dtdx, u);
             } else {
                 const double sign = (slots[e] & 1) ? -1.0 : 1.0;
 #pragma unroll
@@ -98,7 +104,7 @@ __device__ __forceinline__ void fold_events(const PlanView& P, int a, int b, con
 #pragma unroll
             for (int j = 0; j < C; ++j) {
                 if (slots[j] == OWN_SLOT) {
-                    own_update<NDIM>(v[j], gamma, dtdx, u);
+                    own_update<NDIM>(v[j], G, dtdx, u);
                 } else {
                     const double sign = (slots[j] & 1) ? -1.0 : 1.0;
 #pragma unroll
@@ -126,7 +132,7 @@ __device__ __forceinline__ void fold_events(const PlanView& P, int a, int b, con
                     for (int iv = 0; iv < NV; ++iv) fs[iv] = fs[iv] + sign * flux[((size_t)s * NV + iv) * nc + ps];
                 }
             }
-            own_update<NDIM>(fs, gamma, dtdx, u);
+            own_update<NDIM>(fs, G, dtdx, u);
         } else {
             double sign = (slot & 1) ? -1.0 : 1.0;
 #pragma unroll
@@ -173,6 +179,63 @@ __device__ __forceinline__ bool cfl_candidate(const double* u, double dx, double
         sq = sqrt(1.0 + 2.0 * cfl * alpha) - 1.0;
     }
     double dtc = (dx / u_wave) * sq / alpha;
+    *bits = (unsigned long long)__double_as_longlong(dtc);
+    return dtc >= 0.0;
+}
+
+// The constants of a CFL pass: the factor, sqrt(1 + 2 cfl 1e-4) - 1 (the same
+// expression cfl_candidate forms, by IEEE operations on either side) and the
+// cap switch.
+struct CflK {
+    double cfl, root;
+    int cap;
+};
+inline CflK cfl_consts(double cfl, int pressure_cap) {
+    return CflK{cfl, std::sqrt(1.0 + 2.0 * cfl * 0.0001) - 1.0, pressure_cap};
+}
+
+// ctoprim into q (if PRIM) and the CFL candidate (if CFL) of one cell with one
+// reciprocal of its density: eight IEEE divisions and two roots became three
+// reciprocals and one root.  Where a value is outside the checked range, the
+// plain functions.
+template <int NDIM, bool PRIM, bool CFL>
+__device__ __forceinline__ bool prim_cfl(const double* u, double* q, double dx, const FastGas& G, double smalle,
+                                         const CflK& F, unsigned long long* bits) {
+    constexpr int NV = Dims<NDIM>::NV, IP = Dims<NDIM>::IP;
+    Check C;
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) C.up(u[iv]);
+    if (!(C.top_ok() && G.fast && dx > 0x1p-60 && dx < 0x1p60)) {
+        if (PRIM) ctoprim<NDIM>(u, q, G.gamma, smalle);
+        return CFL ? cfl_candidate<NDIM>(u, dx, G.gamma, F.cfl, F.cap, bits) : false;
+    }
+    const double d = smax(u[0], 1e-10), y = rcp_fast(d);
+    if (PRIM) {
+        const double oor = div_by(1.0, d, y);
+        double eken = 0.0;
+        q[0] = d;
+#pragma unroll
+        for (int i = 1; i <= NDIM; ++i) {
+            q[i] = u[i] * oor;
+            eken = eken + 0.5 * q[i] * q[i];
+        }
+        q[IP] = G.gm1 * d * smax(u[IP] * oor - eken - 0.0, smalle);
+    }
+    if (!CFL) return false;
+    // (velocities too small for div_by's range vanish in both sums)
+    double v2 = 0.0, v[NDIM];
+#pragma unroll
+    for (int i = 0; i < NDIM; ++i) {
+        v[i] = div_by(u[1 + i], d, y);
+        v2 = v2 + v[i] * v[i];
+    }
+    double pr = smax((u[IP] - 0.5 * d * v2) * G.gm1, d * 1e-10);
+    if (F.cap) pr = smin(pr, d * 1e2);
+    const double cs2 = smax(div_by(G.gamma * pr, d, y), 1e-20);
+    double w = NDIM * sqrt_fast(smax(cs2, 1e-10));
+#pragma unroll
+    for (int i = 0; i < NDIM; ++i) w = w + fabs(v[i]);
+    const double dtc = div_by(div_by(dx, w, rcp_fast(w)) * F.root, 0.0001, 1.0 / 0.0001);
     *bits = (unsigned long long)__double_as_longlong(dtc);
     return dtc >= 0.0;
 }

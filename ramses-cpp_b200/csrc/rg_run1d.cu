@@ -81,8 +81,8 @@ size_t line_smem(int m) {
 template <int RS>
 __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLineThreads, 1)
     k_level_run_line(TreeView T, PlanView P, double* __restrict__ uold, double* __restrict__ unew,
-                     double* __restrict__ prim, DevStatus* st, const __grid_constant__ StepK K, double dx, double cfl,
-                     int pressure_cap, double dt_start, double t_end, long long max_steps) {
+                     double* __restrict__ prim, DevStatus* st, const __grid_constant__ StepK K, double dx, CflK F,
+                     double dt_start, double t_end, long long max_steps) {
     constexpr int NV = 3;
     extern __shared__ __align__(16) double smem[];
     cg::cluster_group cluster = cg::this_cluster();
@@ -163,12 +163,11 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLineThreads, 1)
             };
             if (i == n - 1) sub(fr);
             if (i > 0) sub(fl);
-            own_update<1>(fs, K.gamma, dtdx, v);
+            own_update<1>(fs, K.gas, dtdx, v);
             if (i < n - 1) sub(fr);
             if (i == 0) sub(fl);
-            ctoprim<1>(v, qq, K.gamma, K.smalle);
             unsigned long long bits;
-            if (cfl_candidate<1>(v, dx, K.gamma, cfl, pressure_cap, &bits) && bits < best) best = bits;
+            if (prim_cfl<1, true, true>(v, qq, dx, K.gas, K.smalle, F, &bits) && bits < best) best = bits;
             // into this piece and, at its edges, the neighbours' copies
             auto put = [&](double* ub, double* qb, int at) {
 #pragma unroll
@@ -244,7 +243,7 @@ int launch_line(rg_ctx* c, const Plan& P, double dx, int pressure_cap, double t_
                             "line run shared memory"))
         return rc;
     kern<<<kCta, kLineThreads, smem, c->stream>>>(tree_view(c), P.view(), c->d_uold, c->d_unew, c->d_prim, c->d_status,
-                                                  K, dx, c->params.courant_factor, pressure_cap,
+                                                  K, dx, cfl_consts(c->params.courant_factor, pressure_cap),
                                                   c->params.boxlen / 1e-10, t_end, max_steps);
     return check_cuda(c, cudaGetLastError(), "line run kernel");
 }

@@ -133,7 +133,7 @@ __device__ __forceinline__ double box_dtdx(const PlanView& P, int a) {
 template <int NDIM, bool LEAF, bool FSUM>
 __device__ __forceinline__ void fold_short(int bid, int nb, const TreeView& T, const PlanView& P,
                                            const double* __restrict__ flux, double* __restrict__ unew,
-                                           const DevStatus* __restrict__ st, double gamma, double* __restrict__ uold,
+                                           const DevStatus* __restrict__ st, const FastGas& G, double* __restrict__ uold,
                                            const double* __restrict__ fsum, double* __restrict__ uold_out) {
     constexpr int NV = Dims<NDIM>::NV;
     const size_t ncell = (size_t)T.ncell;
@@ -149,8 +149,8 @@ __device__ __forceinline__ void fold_short(int bid, int nb, const TreeView& T, c
         double u[NV];
 #pragma unroll
         for (int iv = 0; iv < NV; ++iv) u[iv] = src[(size_t)iv * ncell + cell - 1];
-        if (P.obox) fold_events<NDIM, FSUM, false>(P, a, b, flux, fsum, gamma, dtdx, u);
-        else fold_events<NDIM, FSUM>(P, a, b, flux, fsum, gamma, dtdx, u);
+        if (P.obox) fold_events<NDIM, FSUM, false>(P, a, b, flux, fsum, G, dtdx, u);
+        else fold_events<NDIM, FSUM>(P, a, b, flux, fsum, G, dtdx, u);
 #pragma unroll
         for (int iv = 0; iv < NV; ++iv) unew[(size_t)iv * ncell + cell - 1] = u[iv];
         if (from_old) {
@@ -183,8 +183,8 @@ constexpr int kLongThreads = 256, kLongChunk = 32, kLongPad = kLongChunk + 1;
 template <int NDIM, bool LEAF, bool FSUM>
 __device__ __forceinline__ void fold_long(int bid, int nb, const TreeView& T, const PlanView& P,
                                           const int* __restrict__ tlong, int nlong, const double* __restrict__ flux,
-                                          double* __restrict__ unew, const DevStatus* __restrict__ st, double gamma,
-                                          double* __restrict__ uold, const double* __restrict__ fsum,
+                                          double* __restrict__ unew, const DevStatus* __restrict__ st,
+                                          const FastGas& G, double* __restrict__ uold, const double* __restrict__ fsum,
                                           double* __restrict__ uold_out) {
     constexpr int NV = Dims<NDIM>::NV, NS = Dims<NDIM>::NS, TTD = Dims<NDIM>::TTD;
     // per warp: the terms of one chunk, variable-major, rows padded so the
@@ -268,7 +268,7 @@ __device__ __forceinline__ void fold_long(int bid, int nb, const TreeView& T, co
 #pragma unroll
                 for (int iv = 0; iv < NV; ++iv) vj[iv] = __shfl_sync(0xffffffffu, val[iv], j);
                 if (oj) {
-                    own_update<NDIM>(vj, gamma, dtdx, u);
+                    own_update<NDIM>(vj, G, dtdx, u);
                 } else {
 #pragma unroll
                     for (int iv = 0; iv < NV; ++iv) u[iv] = u[iv] - vj[iv];
@@ -303,25 +303,25 @@ inline int grid_for(rg_ctx* c, long long work, int block) {
 template <int NDIM, bool LEAF = false, bool FSUM = false>
 __global__ void __launch_bounds__(kLongThreads)
     k_fold(TreeView T, PlanView P, const int* __restrict__ tlong, int nlong, int long_blocks,
-           const double* __restrict__ flux, double* __restrict__ unew, const DevStatus* __restrict__ st, double gamma,
-           double* __restrict__ uold = nullptr, const double* __restrict__ fsum = nullptr,
+           const double* __restrict__ flux, double* __restrict__ unew, const DevStatus* __restrict__ st,
+           const __grid_constant__ FastGas G, double* __restrict__ uold = nullptr, const double* __restrict__ fsum = nullptr,
            double* __restrict__ uold_out = nullptr) {
     const int b = (int)blockIdx.x;
     if (b < long_blocks)
-        fold_long<NDIM, LEAF, FSUM>(b, long_blocks, T, P, tlong, nlong, flux, unew, st, gamma, uold, fsum, uold_out);
+        fold_long<NDIM, LEAF, FSUM>(b, long_blocks, T, P, tlong, nlong, flux, unew, st, G, uold, fsum, uold_out);
     else
-        fold_short<NDIM, LEAF, FSUM>(b - long_blocks, (int)gridDim.x - long_blocks, T, P, flux, unew, st, gamma, uold,
+        fold_short<NDIM, LEAF, FSUM>(b - long_blocks, (int)gridDim.x - long_blocks, T, P, flux, unew, st, G, uold,
                                      fsum, uold_out);
 }
 
 template <int NDIM, bool LEAF = false, bool FSUM = false>
 void launch_fold(rg_ctx* c, const Plan& P, const TreeView& T, const PlanView& V, const double* flux, double* unew,
-                 double gamma, double* uold = nullptr, const double* fsum = nullptr, double* uold_out = nullptr) {
+                 const FastGas& G, double* uold = nullptr, const double* fsum = nullptr, double* uold_out = nullptr) {
     const int long_blocks =
         P.nlong > 0 ? (int)std::min<long long>(((long long)P.nlong * 32 + kLongThreads - 1) / kLongThreads, 4096) : 0;
     const int grid = long_blocks + grid_for(c, P.ntarg, kLongThreads);
     k_fold<NDIM, LEAF, FSUM><<<grid, kLongThreads, 0, c->stream>>>(T, V, P.tlong, P.nlong, long_blocks, flux, unew,
-                                                                   c->d_status, gamma, uold, fsum, uold_out);
+                                                                   c->d_status, G, uold, fsum, uold_out);
 }
 
 // The block's minimum of `best` (every thread of the block calls this, none
@@ -351,9 +351,8 @@ __device__ __forceinline__ void block_atomic_min(unsigned long long best, unsign
 // targets so the per-box min can use a segmented shuffle.
 template <int NDIM, bool BOXED>
 __global__ void k_fold_next(TreeView T, PlanView P, const double* __restrict__ flux, double* __restrict__ unew,
-                            DevStatus* st, double gamma, double smalle, double* __restrict__ uold,
-                            const double* __restrict__ fsum, double* __restrict__ prim, double dx, double cfl,
-                            int pressure_cap) {
+                            DevStatus* st, const __grid_constant__ FastGas G, double smalle, double* __restrict__ uold,
+                            const double* __restrict__ fsum, double* __restrict__ prim, double dx, CflK F) {
     constexpr int NV = Dims<NDIM>::NV;
     const size_t ncell = (size_t)T.ncell;
     const int nt = P.ntarg;
@@ -374,21 +373,22 @@ __global__ void k_fold_next(TreeView T, PlanView P, const double* __restrict__ f
             for (int iv = 0; iv < NV; ++iv) u[iv] = uold[(size_t)iv * ncell + cell - 1];
             if (a < b) {
                 const double dtdx = BOXED ? box_dtdx<NDIM>(P, a) : dtdx0;
-                fold_events<NDIM, true, !BOXED>(P, a, b, flux, fsum, gamma, dtdx, u);
+                fold_events<NDIM, true, !BOXED>(P, a, b, flux, fsum, G, dtdx, u);
 #pragma unroll
                 for (int iv = 0; iv < NV; ++iv) {
                     unew[(size_t)iv * ncell + cell - 1] = u[iv];
                     uold[(size_t)iv * ncell + cell - 1] = u[iv];
                 }
             }
-            ctoprim<NDIM>(u, q, gamma, smalle);
+            if (BOXED) box = box_of(P, t);
+            unsigned long long bits;
+            const bool got = prim_cfl<NDIM, true, true>(u, q, BOXED ? P.boxes[box].dx : dx, G, smalle, F, &bits);
 #pragma unroll
             for (int iv = 0; iv < NV; ++iv) prim[(size_t)iv * ncell + cell - 1] = q[iv];
             if (T.son[cell - 1] == 0) {
-                if (BOXED) box = box_of(P, t);
-                unsigned long long bits;
-                if (cfl_candidate<NDIM>(u, BOXED ? P.boxes[box].dx : dx, gamma, cfl, pressure_cap, &bits))
-                    best = bits;
+                if (got) best = bits;
+            } else {
+                box = -1;
             }
         }
         if constexpr (BOXED) {
@@ -427,7 +427,7 @@ __global__ void k_copy_level(TreeView T, PlanView P, int nvar, const double* __r
 // HydroSolver::set_unew does).
 template <int NDIM>
 __global__ void k_courant(TreeView T, PlanView P, const double* __restrict__ uold, DevStatus* st, double dx,
-                          double gamma, double cfl, int pressure_cap, double* __restrict__ unew_copy,
+                          const __grid_constant__ FastGas G, CflK F, double* __restrict__ unew_copy,
                           ClockStep clock, double* __restrict__ prim, double smalle) {
     constexpr int NV = NDIM + 2;
     const size_t ncell = (size_t)T.ncell;
@@ -435,48 +435,27 @@ __global__ void k_courant(TreeView T, PlanView P, const double* __restrict__ uol
     // with prim: the extra (ghost-stencil) cells after the level's, primitives only
     const int total = prim ? P.ncells + P.nextra_prim : P.ncells;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < total; p += gridDim.x * blockDim.x) {
-        int id = (p < P.ncells) ? cell_of(T, P, p) : P.xprim[p - P.ncells];
+        const int id = (p < P.ncells) ? cell_of(T, P, p) : P.xprim[p - P.ncells];
+        const bool level = p < P.ncells, leaf = level && T.son[id - 1] <= 0;
+        double u[NV], q[NV];
+#pragma unroll
+        for (int iv = 0; iv < NV; ++iv) u[iv] = uold[(size_t)iv * ncell + id - 1];
+        unsigned long long b;
+        // positive doubles order like their bit patterns; NaN patterns sort
+        // above every finite value, matching std::min's NaN fall-through
         if (prim) {
             // k_prim's pass (ctoprim of uold), folded in
-            double u[NV], q[NV];
-#pragma unroll
-            for (int iv = 0; iv < NV; ++iv) u[iv] = uold[(size_t)iv * ncell + id - 1];
-            ctoprim<NDIM>(u, q, gamma, smalle);
+            const bool got = prim_cfl<NDIM, true, true>(u, q, dx, G, smalle, F, &b);
+            if (got && leaf && b < best) best = b;
 #pragma unroll
             for (int iv = 0; iv < NV; ++iv) prim[(size_t)iv * ncell + id - 1] = q[iv];
-            if (p >= P.ncells) continue;
+        } else if (leaf) {
+            if (prim_cfl<NDIM, false, true>(u, q, dx, G, smalle, F, &b) && b < best) best = b;
         }
-        if (unew_copy) {
+        if (unew_copy && level) {
 #pragma unroll
-            for (int iv = 0; iv < NDIM + 2; ++iv) unew_copy[(size_t)iv * ncell + id - 1] = uold[(size_t)iv * ncell + id - 1];
+            for (int iv = 0; iv < NV; ++iv) unew_copy[(size_t)iv * ncell + id - 1] = u[iv];
         }
-        if (T.son[id - 1] > 0) continue;
-        const double* u = uold + (id - 1);
-        double d = smax(u[0], 1e-10), v2 = 0.0;
-#pragma unroll
-        for (int i = 1; i <= NDIM; ++i) {
-            double v = u[i * ncell] / d;
-            v2 = v2 + v * v;
-        }
-        double e_non = 0.0, sum_gamma_p = 0.0;
-        double pr = smax((u[(NDIM + 1) * ncell] - 0.5 * d * v2 - e_non) * (gamma - 1.0), d * 1e-10);
-        if (pressure_cap) pr = smin(pr, d * 1e2);
-        double cs2 = cs2_of(d, pr, gamma);
-        cs2 = cs2 + sum_gamma_p / d;
-        double cs = sqrt(smax(cs2, 1e-10));
-        double u_wave = NDIM * cs;
-#pragma unroll
-        for (int i = 1; i <= NDIM; ++i) u_wave = u_wave + fabs(u[i * ncell] / d);
-        double a_grav = 0.0;
-#pragma unroll
-        for (int i = 1; i <= NDIM; ++i) a_grav = a_grav + fabs(0.0);
-        double alpha = a_grav * dx / (u_wave * u_wave);
-        alpha = smax(alpha, 0.0001);
-        double dtc = (dx / u_wave) * (sqrt(1.0 + 2.0 * cfl * alpha) - 1.0) / alpha;
-        // positive doubles order like their bit patterns; NaN patterns sort
-        // above every finite value, matching std::min's NaN fall-through.
-        unsigned long long b = (unsigned long long)__double_as_longlong(dtc);
-        if (dtc >= 0.0 && b < best) best = b;
     }
     block_atomic_min(best, &st->dtmin_bits);
     if (!clock.ck) return;
@@ -503,7 +482,7 @@ __global__ void k_clock_step(DevStatus* st, ClockStep clock) {
 // CFL candidate and primitives in one pass over uold (leaf-level substep).
 template <int NDIM>
 __global__ void k_courant_prim(TreeView T, PlanView P, const double* __restrict__ uold, double* __restrict__ prim,
-                               DevStatus* st, double dx, double gamma, double smalle, double cfl, int pressure_cap) {
+                               DevStatus* st, double dx, const __grid_constant__ FastGas G, double smalle, CflK F) {
     constexpr int NV = Dims<NDIM>::NV;
     const size_t ncell = (size_t)T.ncell;
     const int total = P.ncells + P.nextra_prim;
@@ -513,12 +492,12 @@ __global__ void k_courant_prim(TreeView T, PlanView P, const double* __restrict_
         double u[NV], q[NV];
 #pragma unroll
         for (int iv = 0; iv < NV; ++iv) u[iv] = uold[(size_t)iv * ncell + id - 1];
-        ctoprim<NDIM>(u, q, gamma, smalle);
+        unsigned long long b;
+        const bool got = prim_cfl<NDIM, true, true>(u, q, dx, G, smalle, F, &b);
 #pragma unroll
         for (int iv = 0; iv < NV; ++iv) prim[(size_t)iv * ncell + id - 1] = q[iv];
         if (t >= P.ncells || T.son[id - 1] > 0) continue;
-        unsigned long long b;
-        if (cfl_candidate<NDIM>(u, dx, gamma, cfl, pressure_cap, &b) && b < best) best = b;
+        if (got && b < best) best = b;
     }
     block_atomic_min(best, &st->dtmin_bits);
 }
@@ -630,8 +609,9 @@ StepK step_consts(const rg_ctx* c) {
     K.own = st == 2 || st == 3 ? Limiter{2.0, 0.5} : (st == 8 ? Limiter{1.5, 0.5} : Limiter{1.0, 1.0});
     K.ghost = it == 1 ? Limiter{0.5, 1.0} : (it == 2 ? Limiter{1.0, 0.25} : Limiter{HUGE_VAL, 0.25});
     K.gas = FastGas{p.gamma, p.gamma - 1.0, 1.0 / (p.gamma - 1.0), K.smallp, (p.gamma + 1.0) / (2.0 * p.gamma),
-                    1.0 / p.gamma};
-    K.fast = st != 0 && !(st >= 4 && st <= 7) && it >= 1 && it <= 3 && K.gas.gm1 > 0x1p-20 && K.gas.gm1 < 0x1p20;
+                    1.0 / p.gamma, 0};
+    K.gas.fast = K.gas.gm1 > 0x1p-20 && K.gas.gm1 < 0x1p20;
+    K.fast = st != 0 && !(st >= 4 && st <= 7) && it >= 1 && it <= 3 && K.gas.fast;
     return K;
 }
 
@@ -678,7 +658,7 @@ int launch_godunov_t(rg_ctx* c, const Plan& P, bool set_uold, const double* dt_d
     if (int rc = launch_face_tiles(c, P, K, c->d_uold, c->d_prim, c->d_flux, fsum)) return rc;
     if (E) cudaEventRecord(E[2], c->stream);
     double* uold_out = set_uold ? c->d_uold : nullptr;
-    launch_fold<NDIM, false, true>(c, P, T, V, c->d_flux, c->d_unew, K.gamma, nullptr, fsum, uold_out);
+    launch_fold<NDIM, false, true>(c, P, T, V, c->d_flux, c->d_unew, K.gas, nullptr, fsum, uold_out);
     if (E) cudaEventRecord(E[3], c->stream);
     return check_cuda(c, cudaGetLastError(), "godunov kernels");
 }
@@ -708,7 +688,7 @@ int launch_godunov_ext_t(rg_ctx* c, const Plan& P, const double* uold, double* u
         case RG_RIEMANN_ACOUSTIC: launch_face_ext_t<NDIM, RG_RIEMANN_ACOUSTIC>(c, P, K, uold, prim, flux); break;
         default: launch_face_ext_t<NDIM, RG_RIEMANN_LLF>(c, P, K, uold, prim, flux); break;
     }
-    launch_fold<NDIM>(c, P, T, V, flux, unew, K.gamma);
+    launch_fold<NDIM>(c, P, T, V, flux, unew, K.gas);
     return check_cuda(c, cudaGetLastError(), "godunov kernels (caller buffers)");
 }
 
@@ -763,8 +743,8 @@ void launch_leaf_prefix_t(rg_ctx* c, const Plan& P, double dx, int pressure_cap,
             return;
         }
         k_courant_prim<NDIM><<<grid_for(c, nprim, 256), 256, 0, c->stream>>>(T, V, c->d_uold, c->d_prim,
-                                                                             c->d_status, dx, K.gamma, K.smalle,
-                                                                             cfl, pressure_cap);
+                                                                             c->d_status, dx, K.gas, K.smalle,
+                                                                             cfl_consts(cfl, pressure_cap));
     }
 }
 
@@ -792,15 +772,15 @@ int launch_leaf_core_t(rg_ctx* c, const Plan& P, double dx, int pressure_cap, do
     const int g = grid_for(c, P.ntarg, 256);
     if (leaf_fusable(P)) {
         if (P.nbox > 0)
-            k_fold_next<NDIM, true><<<g, 256, 0, c->stream>>>(T, V, c->d_flux, c->d_unew, c->d_status, K.gamma,
-                                                              K.smalle, c->d_uold, fsum, c->d_prim, dx, cfl,
-                                                              pressure_cap);
+            k_fold_next<NDIM, true><<<g, 256, 0, c->stream>>>(T, V, c->d_flux, c->d_unew, c->d_status, K.gas,
+                                                              K.smalle, c->d_uold, fsum, c->d_prim, dx,
+                                                              cfl_consts(cfl, pressure_cap));
         else
-            k_fold_next<NDIM, false><<<g, 256, 0, c->stream>>>(T, V, c->d_flux, c->d_unew, c->d_status, K.gamma,
-                                                               K.smalle, c->d_uold, fsum, c->d_prim, dx, cfl,
-                                                               pressure_cap);
+            k_fold_next<NDIM, false><<<g, 256, 0, c->stream>>>(T, V, c->d_flux, c->d_unew, c->d_status, K.gas,
+                                                               K.smalle, c->d_uold, fsum, c->d_prim, dx,
+                                                               cfl_consts(cfl, pressure_cap));
     } else {
-        launch_fold<NDIM, true, true>(c, P, T, V, c->d_flux, c->d_unew, K.gamma, c->d_uold, fsum);
+        launch_fold<NDIM, true, true>(c, P, T, V, c->d_flux, c->d_unew, K.gas, c->d_uold, fsum);
     }
     if (c->timing) cudaEventRecord(c->ev[3], c->stream);
     return check_cuda(c, cudaGetLastError(), "leaf substep kernels");
@@ -867,12 +847,14 @@ int launch_courant(rg_ctx* c, const Plan& P, double dx, int pressure_cap, double
         const StepK K = step_consts(c);
         if (c->params.ndim == 1)
             k_courant<1><<<grid_for(c, work, 256), 256, 0, c->stream>>>(tree_view(c), P.view(), c->d_uold,
-                                                                        c->d_status, dx, c->params.gamma, cfl,
-                                                                        pressure_cap, copy, cs, prim, K.smalle);
+                                                                        c->d_status, dx, K.gas,
+                                                                        cfl_consts(cfl, pressure_cap), copy, cs, prim,
+                                                                        K.smalle);
         else
             k_courant<3><<<grid_for(c, work, 256), 256, 0, c->stream>>>(tree_view(c), P.view(), c->d_uold,
-                                                                        c->d_status, dx, c->params.gamma, cfl,
-                                                                        pressure_cap, copy, cs, prim, K.smalle);
+                                                                        c->d_status, dx, K.gas,
+                                                                        cfl_consts(cfl, pressure_cap), copy, cs, prim,
+                                                                        K.smalle);
     } else if (cs.ck) {
         k_clock_step<<<1, 1, 0, c->stream>>>(c->d_status, cs);
     }
@@ -990,7 +972,7 @@ __global__ void __launch_bounds__(kRunBlock) k_level_run_block(TreeView T, PlanV
 #pragma unroll
             for (int iv = 0; iv < NV; ++iv) u[iv] = uold[(size_t)iv * ncell + cell - 1];
             if (a < b) {
-                fold_events<NDIM, true, true>(P, a, b, flux, fsum, K.gamma, st->dtdx, u);
+                fold_events<NDIM, true, true>(P, a, b, flux, fsum, K.gas, st->dtdx, u);
 #pragma unroll
                 for (int iv = 0; iv < NV; ++iv) {
                     unew[(size_t)iv * ncell + cell - 1] = u[iv];

@@ -84,7 +84,7 @@ __global__ void ke(int n, int niter, double tol, unsigned long long* bad) {
         if (odd == 7) { for (int k = 0; k < 5; ++k) r[k] = l[k]; r[1] += 1e-9; }
         const double gamma = rnd(s) & 1 ? 1.4 : 5.0 / 3.0, smallp = 1e-10 * 1e-10 / gamma;
         const double guess = odd == 8 ? l[4] * 1.1 : -1.0;
-        const rg::FastGas G{gamma, gamma - 1.0, 1.0 / (gamma - 1.0), smallp, (gamma + 1.0) / (2.0 * gamma), 1.0 / gamma};
+        const rg::FastGas G{gamma, gamma - 1.0, 1.0 / (gamma - 1.0), smallp, (gamma + 1.0) / (2.0 * gamma), 1.0 / gamma, 1};
         int it;
         if (!rg::exact_fast<3>(l, r, f, G, niter, tol, guess, &ps, &it)) { ++plain; continue; }
         const int jt = rg::solve_exact_p<3>(l, r, g, gamma, smallp, niter, tol, guess, &pg);

@@ -1,5 +1,6 @@
 // rg_face_brick.cuh -- face kernel for levels that form one complete periodic
-// lattice (detected and verified by rg_lattice.cu).
+// lattice (detected and verified by rg_lattice.cu), refined cells among them or
+// not: the base level of an AMR run is one too (a few of its cells refined).
 //
 // Same arithmetic and outputs as k_face_tiles (rg_face.cuh): per (cell,
 // direction) the own MUSCL-Hancock trace, the two neighbours' face states by
@@ -27,11 +28,13 @@ constexpr int BRICK_THREADS = 256;
 constexpr size_t BRICK_SMEM = sizeof(double) * 5 * BSITES;  // 69,120 bytes (3D: nvar 5)
 
 // One cell of a brick: its fluxes in the three directions to the scratch, its
-// own flux sum in slot order.
+// own flux sum in slot order.  zero: bit s set where slot s faces a refined
+// cell and carries no flux.
 template <int RS, bool FAST, bool POW2>
 __device__ __forceinline__ void brick_cell(const double* sq, int site, int p, int nc, bool ghost, double dt,
                                            const DxDiv& D, const FastStep& S, const FastStep& Sc, const StepK& K,
-                                           double* __restrict__ flux, double* __restrict__ fsum, unsigned& iters) {
+                                           unsigned zero, double* __restrict__ flux, double* __restrict__ fsum,
+                                           unsigned& iters) {
     constexpr int NV = 5;
     double fs[NV];
 #pragma unroll
@@ -43,11 +46,14 @@ __device__ __forceinline__ void brick_cell(const double* sq, int site, int p, in
         unsigned it = 0;
         bool ok = false;
         const int stride = idim == 0 ? 1 : (idim == 1 ? BSIDE : BSIDE * BSIDE);
+        const unsigned none = (zero >> (2 * idim)) & 3u;
         if (FAST) ok = brick_dir_fast<RS, POW2, BSITES>(sq, site, idim, stride, S, Sc, K, f[0], f[1], it);
-        if (!ok) {
+        if (!ok || none) {
             double g[2 * NV];  // (the call's array lives in memory, the loop's in registers)
-            it = brick_face_plain<RS, BSITES>(sq, site, idim, stride, 0, ghost, dt, D, K, g) +
-                 brick_face_plain<RS, BSITES>(sq, site, idim, stride, 1, ghost, dt, D, K, g + NV);
+#pragma unroll
+            for (int k = 0; k < 2 * NV; ++k) g[k] = 0.0;
+            it = none & 1u ? 0u : brick_face_plain<RS, BSITES>(sq, site, idim, stride, 0, ghost, dt, D, K, g);
+            it += none & 2u ? 0u : brick_face_plain<RS, BSITES>(sq, site, idim, stride, 1, ghost, dt, D, K, g + NV);
 #pragma unroll
             for (int k = 0; k < 2 * NV; ++k) f[k / NV][k % NV] = g[k];
         }
@@ -74,9 +80,9 @@ __device__ __forceinline__ void brick_cell(const double* sq, int site, int p, in
 // apart, so the 16 lanes meet 16 different 8-byte banks.
 template <int RS, bool BOXED>
 __device__ __forceinline__ void brick_face(const PlanView& P, const BrickGeom& G, const int* __restrict__ lat_id,
-                                           const int* __restrict__ lat_p, int kind, const double* __restrict__ prim,
-                                           size_t ncell, double* __restrict__ flux, double* __restrict__ fsum,
-                                           const DevStatus* st, const StepK& K, int brick, double* sq,
+                                           const int* __restrict__ lat_p, const uint8_t* __restrict__ lat_mask,
+                                           int kind, const double* __restrict__ prim, size_t ncell,
+                                           double* __restrict__ flux, double* __restrict__ fsum, const DevStatus* st, const StepK& K, int brick, double* sq,
                                            unsigned long long& iters, unsigned long long& calls) {
     constexpr int NV = 5;
     int ex = G.ex, ey = G.ey, ez = G.ez, local = brick;
@@ -127,11 +133,14 @@ __device__ __forceinline__ void brick_face(const PlanView& P, const BrickGeom& G
         const int x = u % BRICK, z = u / (BRICK * BRICK);
         const int y = ((u >> 4) & 1) | ((u >> 2) & 2) | ((u >> 3) & 4);
         const int site = (x + BHALO) + BSIDE * ((y + BHALO) + BSIDE * (z + BHALO));
-        const int p = lat_p[(size_t)(bx * BRICK + x) + (size_t)ex * ((size_t)(by * BRICK + y) + (size_t)ey * (bz * BRICK + z))];
-        if (!fast) brick_cell<RS, false, false>(sq, site, p, nc, ghost, dt, D, S, Sc, K, flux, fsum, it);
-        else if (D.pow2) brick_cell<RS, true, true>(sq, site, p, nc, ghost, dt, D, S, Sc, K, flux, fsum, it);
-        else brick_cell<RS, true, false>(sq, site, p, nc, ghost, dt, D, S, Sc, K, flux, fsum, it);
-        done += 6;
+        const size_t g = (size_t)(bx * BRICK + x) + (size_t)ex * ((size_t)(by * BRICK + y) + (size_t)ey * (bz * BRICK + z));
+        const unsigned zero = lat_mask ? lat_mask[g] : 0u;
+        if (zero & LAT_REFINED) continue;
+        const int p = lat_p[g];
+        if (!fast) brick_cell<RS, false, false>(sq, site, p, nc, ghost, dt, D, S, Sc, K, zero, flux, fsum, it);
+        else if (D.pow2) brick_cell<RS, true, true>(sq, site, p, nc, ghost, dt, D, S, Sc, K, zero, flux, fsum, it);
+        else brick_cell<RS, true, false>(sq, site, p, nc, ghost, dt, D, S, Sc, K, zero, flux, fsum, it);
+        done += 6 - __popc(zero);
     }
     iters += it;
     calls += done;
@@ -139,12 +148,12 @@ __device__ __forceinline__ void brick_face(const PlanView& P, const BrickGeom& G
 
 template <int RS, int MINB, bool BOXED>
 __global__ void __launch_bounds__(BRICK_THREADS, MINB)
-    k_face_brick(PlanView P, BrickGeom G, const int* __restrict__ lat_id, const int* __restrict__ lat_p, int kind,
-                 const double* __restrict__ prim, size_t ncell, double* __restrict__ flux,
+    k_face_brick(PlanView P, BrickGeom G, const int* __restrict__ lat_id, const int* __restrict__ lat_p,
+                 const uint8_t* __restrict__ lat_mask, int kind, const double* __restrict__ prim, size_t ncell, double* __restrict__ flux,
                  double* __restrict__ fsum, DevStatus* st, const __grid_constant__ StepK K) {
     extern __shared__ __align__(16) double sq[];  // [NV][BSITES]
     unsigned long long iters = 0, calls = 0;
-    brick_face<RS, BOXED>(P, G, lat_id, lat_p, kind, prim, ncell, flux, fsum, st, K, (int)blockIdx.x, sq, iters,
+    brick_face<RS, BOXED>(P, G, lat_id, lat_p, lat_mask, kind, prim, ncell, flux, fsum, st, K, (int)blockIdx.x, sq, iters,
                           calls);
     if (RS == RG_RIEMANN_EXACT) {
         for (int o = 16; o > 0; o >>= 1) {
@@ -173,7 +182,7 @@ int launch_face_brick(rg_ctx* c, const Plan& P, const StepK& K, const double* pr
     const BrickGeom G{P.lat_e[0], P.lat_e[1], P.lat_e[2], P.nbox, P.bl_ext, P.bl_off, P.bl_brick_off};
     const int nbricks =
         BOXED ? P.bl_nbricks : (P.lat_e[0] / BRICK) * (P.lat_e[1] / BRICK) * (P.lat_e[2] / BRICK);
-    kern<<<nbricks, BRICK_THREADS, BRICK_SMEM, c->stream>>>(P.view(), G, P.lat_id, P.lat_p, P.lat_kind, prim,
+    kern<<<nbricks, BRICK_THREADS, BRICK_SMEM, c->stream>>>(P.view(), G, P.lat_id, P.lat_p, P.lat_mask, P.lat_kind, prim,
                                                             (size_t)c->ncell, flux, fsum, c->d_status, K);
     return check_cuda(c, cudaGetLastError(), "brick face kernel");
 }

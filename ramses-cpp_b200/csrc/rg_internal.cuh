@@ -39,6 +39,7 @@ enum Kind : int8_t { K_NONE = 0, K_ZERO = 1, K_GHOST = 2, K_SAME = 3, K_BOUND = 
 constexpr int KIND_MASK = 7;
 constexpr int KIND_REFLUX = 8;   // interface refluxes into its neighbour
 constexpr int KIND_REFLECT = 16; // boundary branch with btype == 1 (velocity flip)
+constexpr int LAT_REFINED = 64;  // lattice mask bit of a refined cell
 constexpr int OWN_SLOT = 7;      // event slot of a cell's own update
 
 // device error word: first error wins; info carries an index for the message
@@ -162,6 +163,7 @@ struct Plan {
     int lat_kind = 0;          // the (single) interface kind of its faces
     int* lat_id = nullptr;     // [ex*ey*ez] cell id of each lattice site (x fastest)
     int* lat_p = nullptr;      // [ex*ey*ez] plan position of each site
+    uint8_t* lat_mask = nullptr;  // levels with refined cells: per site the slots without flux, LAT_REFINED
     int* lat_ord = nullptr;    // [sites] each cell's seven updates in loop order, 3 bits each (slot, 7 its own)
     // ensemble levels whose boxes are each one periodic lattice: per box its
     // extent, its first site in lat_id/lat_p and its first brick

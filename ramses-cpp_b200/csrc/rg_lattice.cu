@@ -72,8 +72,10 @@ __global__ void k_lattice_fill(TreeView T, PlanView P, int scale0, int ex, int e
 
 __device__ __forceinline__ int wrap(int a, int n) { return a < 0 ? a + n : (a >= n ? a - n : a); }
 
+// mask != nullptr (a level with refined cells): a refined cell's faces and the
+// faces towards one are marked there instead of being of kind kind0.
 __global__ void k_lattice_check(TreeView T, PlanView P, int ex, int ey, int ez, const int* __restrict__ lat_id,
-                                const int* __restrict__ lat_p, int kind0, int* bad) {
+                                const int* __restrict__ lat_p, int kind0, uint8_t* mask, int* bad) {
     const size_t n = (size_t)ex * ey * ez;
     for (size_t site = (size_t)blockIdx.x * blockDim.x + threadIdx.x; site < n;
          site += (size_t)gridDim.x * blockDim.x) {
@@ -84,6 +86,13 @@ __global__ void k_lattice_check(TreeView T, PlanView P, int ex, int ey, int ez, 
             continue;
         }
         const int c = lat_id[site];
+        unsigned m = 0;
+        if (mask && T.son[c - 1] > 0) {
+            mask[site] = LAT_REFINED;
+            for (int s = 0; s < 6; ++s)
+                if (P.kind[s * (size_t)P.ncells + p] != K_NONE) atomicExch(bad, 1);
+            continue;
+        }
         for (int s = 0; s < 6; ++s) {
             const int idim = s >> 1, side = s & 1, d = side ? 1 : -1;
             auto at = [&](int off) {
@@ -96,10 +105,16 @@ __global__ void k_lattice_check(TreeView T, PlanView P, int ex, int ey, int ez, 
             const int nb = at(d), far = at(2 * d);
             const size_t nc = (size_t)P.ncells;
             const int want_nl = side ? c : far, want_nr = side ? far : c;
+            if (mask && P.kind[s * nc + p] == K_ZERO) {
+                m |= 1u << s;
+                if (P.icn[s * nc + p] != nb) atomicExch(bad, 1);
+                continue;
+            }
             if (P.icn[s * nc + p] != nb || P.stc[((size_t)s * 2 + 0) * nc + p] != want_nl ||
                 P.stc[((size_t)s * 2 + 1) * nc + p] != want_nr || P.kind[s * nc + p] != kind0)
                 atomicExch(bad, 1);
         }
+        if (mask) mask[site] = (uint8_t)m;
     }
 }
 
@@ -228,14 +243,20 @@ int build_order(rg_ctx* c, Plan& P) {
 // a level that is not a lattice is not an error.
 int build_lattice(rg_ctx* c, Plan& P) {
     P.lattice = 0;
-    if (c->params.ndim != 3 || P.level0 || P.ncells == 0 || P.nactive != P.ncells || P.ilevel < 2) return RG_OK;
+    if (c->params.ndim != 3 || P.level0 || P.ncells == 0 || P.nactive == 0 || P.ilevel < 2) return RG_OK;
+    // with refined cells: only levels large enough for the brick face kernel to be timed
+    const bool part = P.nactive != P.ncells;
+    if (part && P.ncells < (1 << 17)) return RG_OK;
     const long long side = 1LL << (P.ilevel - 1);
     const long long ex = (long long)c->nx * side, ey = (long long)c->ny * side, ez = (long long)c->nz * side;
     if (ex * ey * ez != P.ncells || ex % 8 || ey % 8 || ez % 8) return RG_OK;
-    // the interface kind of every face of a uniform leaf level: the first one's
+    // the interface kind of every face of a uniform leaf level: the first
+    // one's; with refined cells it must be the ghost kind
     int8_t kind0 = 0;
     if (int rc = check_cuda(c, cudaMemcpyAsync(&kind0, P.kind, 1, cudaMemcpyDeviceToHost, c->stream), "lattice kind"))
         return rc;
+    if (part)
+        if (int rc = check_cuda(c, dev_alloc(c, &P.lat_mask, (size_t)P.ncells), "lattice mask")) return rc;
     int* d_bad = nullptr;
     if (int rc = check_cuda(c, dev_alloc(c, &d_bad, sizeof(int)), "lattice flag")) return rc;
     if (int rc = check_cuda(c, dev_alloc(c, &P.lat_id, sizeof(int) * (size_t)P.ncells), "lattice ids")) return rc;
@@ -243,19 +264,21 @@ int build_lattice(rg_ctx* c, Plan& P) {
     cudaMemsetAsync(P.lat_p, 0xff, sizeof(int) * (size_t)P.ncells, c->stream);
     cudaMemsetAsync(d_bad, 0, sizeof(int), c->stream);
     if (int rc = check_cuda(c, cudaStreamSynchronize(c->stream), "lattice kind sync")) return rc;
-    const int kd = kind0;
+    const int kd = part ? (K_GHOST | KIND_REFLUX) : kind0;
     if ((kd & KIND_MASK) != K_GHOST && (kd & KIND_MASK) != K_SAME) {
         dev_free(c, d_bad);
         dev_free(c, P.lat_id);
         dev_free(c, P.lat_p);
+        dev_free(c, P.lat_mask);
         P.lat_id = P.lat_p = nullptr;
+        P.lat_mask = nullptr;
         return RG_OK;
     }
     const int scale0 = (int)side;  // cells per coarse cell and side
     k_lattice_fill<<<lblocks(c, P.ncells), LTPB, 0, c->stream>>>(tree_view(c), P.view(), scale0, (int)ex, (int)ey,
                                                                  (int)ez, P.lat_id, P.lat_p, d_bad);
     k_lattice_check<<<lblocks(c, P.ncells), LTPB, 0, c->stream>>>(tree_view(c), P.view(), (int)ex, (int)ey, (int)ez,
-                                                                  P.lat_id, P.lat_p, kd, d_bad);
+                                                                  P.lat_id, P.lat_p, kd, P.lat_mask, d_bad);
     int bad = 1;
     cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
     const cudaError_t e = cudaStreamSynchronize(c->stream);
@@ -264,7 +287,9 @@ int build_lattice(rg_ctx* c, Plan& P) {
     if (bad) {
         dev_free(c, P.lat_id);
         dev_free(c, P.lat_p);
+        dev_free(c, P.lat_mask);
         P.lat_id = P.lat_p = nullptr;
+        P.lat_mask = nullptr;
         return RG_OK;
     }
     P.lattice = 1;
@@ -272,7 +297,7 @@ int build_lattice(rg_ctx* c, Plan& P) {
     P.lat_e[1] = (int)ey;
     P.lat_e[2] = (int)ez;
     P.lat_kind = kd;
-    return build_order(c, P);
+    return part ? RG_OK : build_order(c, P);
 }
 
 int set_box_lattices(rg_ctx* c, Plan& P, const int* ext, const int* lat_id, const int* lat_p) {

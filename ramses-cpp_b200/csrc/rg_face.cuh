@@ -461,13 +461,21 @@ __global__ void __launch_bounds__(TILE * NDIM * R, MINB)
     const double dt0 = st->dt;
     const DxDiv D0{st->dx, st->inv_dx, st->dx_pow2 != 0};
     unsigned iters = 0, calls = 0;
+    // batch 0: the grid holds every tile, block b takes tiles b R .. b R + R - 1
+    // and the queue is left alone (its two round trips were 2 us of a small
+    // level's 16)
+    const bool queued = batch > 0;
+    const int grab = queued ? batch * R : R;
     for (;;) {
-        if (threadIdx.x == 0) s_base = (int)atomicAdd(&st->face_next, (unsigned)(batch * R));
-        __syncthreads();
-        const int base = s_base;
-        __syncthreads();
+        int base = (int)blockIdx.x * R;
+        if (queued) {
+            if (threadIdx.x == 0) s_base = (int)atomicAdd(&st->face_next, (unsigned)grab);
+            __syncthreads();
+            base = s_base;
+            __syncthreads();
+        }
         if (base >= ntiles) break;
-        const int end = min(base + batch * R, ntiles);
+        const int end = min(base + grab, ntiles);
         for (int t0 = base; t0 < end; t0 += R) {
             const int tile = t0 + r;
             const int p = tile * TILE + lane;
@@ -529,8 +537,9 @@ __global__ void __launch_bounds__(TILE * NDIM * R, MINB)
                     fsum[(size_t)iv * nc + p] = fs;
                 }
             }
-            __syncthreads();
+            if (queued) __syncthreads();
         }
+        if (!queued) break;
     }
     if (RS == RG_RIEMANN_EXACT) {
         unsigned long long wi = iters, wc = calls;
@@ -544,7 +553,7 @@ __global__ void __launch_bounds__(TILE * NDIM * R, MINB)
         }
     }
     // the last block out resets the work counter for the next launch
-    if (threadIdx.x == 0) {
+    if (queued && threadIdx.x == 0) {
         __threadfence();
         if (atomicAdd(&st->face_done, 1u) == gridDim.x - 1) {
             st->face_next = 0;
@@ -585,7 +594,13 @@ int launch_face_one(rg_ctx* c, const Plan& P, const StepK& K, int batch, const d
     const int ntiles = (P.ncells + TILE - 1) / TILE;
     const int grabs = (ntiles + batch * R - 1) / (batch * R);
     int grid = per_sm * c->sm_count;
-    if (grabs < grid) grid = grabs;
+    const int all = (ntiles + R - 1) / R;
+    if (all <= grid) {  // one wave: a block per group of R tiles, no queue
+        grid = all;
+        batch = 0;
+    } else if (grabs < grid) {
+        grid = grabs;
+    }
     if (grid < 1) grid = 1;
     kern<<<grid, block, 0, c->stream>>>(tree_view(c), P.view(), prim, uold, flux, fsum, c->d_status, K, batch);
     return check_cuda(c, cudaGetLastError(), "face kernel");

@@ -159,16 +159,6 @@ int ensure_flux(rg_ctx* c, const Plan& P) {
     return grow(c, &c->d_flux, &c->cap_flux, need, "flux scratch");
 }
 
-// What a leaf substep of the level needs: the brick step's second primitive
-// array, or the flux scratch (also the brick step's first call, which times
-// the face shapes for rg_godunov_level as every level's first step does).
-int ensure_leaf(rg_ctx* c, const Plan& P) {
-    if (!brick_step_on(c, P) || P.face_variant < 0)
-        if (int rc = ensure_flux(c, P)) return rc;
-    if (!brick_step_on(c, P) || c->d_prim2) return RG_OK;
-    return check_cuda(c, dev_alloc(c, &c->d_prim2, sizeof(double) * (size_t)c->nvar * c->ncell), "second primitives");
-}
-
 // rg_level_run's clock: start values, then after each substep t += dt, one
 // more step, and the WHILE node's condition for the next iteration
 __global__ void k_run_init(DevStatus* st, double t, long long steps) {
@@ -327,7 +317,6 @@ void rg_destroy(rg_ctx* c) {
     dev_free(c, c->d_uold);
     dev_free(c, c->d_unew);
     dev_free(c, c->d_prim);
-    dev_free(c, c->d_prim2);
     dev_free(c, c->d_flux);
     dev_free(c, c->d_mlp);
     dev_free(c, c->d_stage);
@@ -454,8 +443,6 @@ int rg_sync_topology(rg_ctx* c, const rg_grid_view* g) {
         if (int rc = grow(c, &c->d_unew, &cap, ns, "unew")) return rc;
         cap = c->cap_state;
         if (int rc = grow(c, &c->d_prim, &cap, ns, "prim")) return rc;
-        dev_free(c, c->d_prim2);
-        c->d_prim2 = nullptr;
         c->cap_state = std::max(c->cap_state, ns);
         c->have_state = false;
     }
@@ -649,9 +636,10 @@ int rg_level_substep(rg_ctx* c, int ilevel, double dx, int pressure_cap, int use
     if (int rc = get_plan(c, ilevel, &P)) return rc;
     record_updates(c, ilevel, *P);
     const bool leaf = P->nactive == P->ncells;  // no refined cell: fused substep
-    if (int rc = leaf ? ensure_leaf(c, *P) : ensure_flux(c, *P)) return rc;
+    if (int rc = ensure_flux(c, *P)) return rc;
     const double cfl = c->params.courant_factor;
     const int cap_key = pressure_cap ? 1 : 0;
+    bool prepared = leaf && leaf_fusable(*P) && P->ncells > 0;  // for the next substep
     if (leaf) {
         // the CFL word and primitives are current if the previous call was a
         // fused substep of this level with the same arguments
@@ -676,10 +664,12 @@ int rg_level_substep(rg_ctx* c, int ilevel, double dx, int pressure_cap, int use
         // first substep of this plan: run it eagerly, then tune the face
         // kernel on its primitives before any graph captures the launch shape
         if (int rc = enqueue()) return rc;
-        // (the brick step's primitives are in lattice order, and after its
-        // first step in the second array: d_prim is free for the timing)
-        if (leaf && brick_step_on(c, *P))
+        // (the brick step keeps its primitives in lattice order and uses the
+        // flux scratch, which the timing writes: the next substep starts anew)
+        if (leaf && brick_step_on(c, *P)) {
             if (int rc = launch_prim(c, *P)) return rc;
+            prepared = false;
+        }
         if (int rc = autotune_face(c, *P, step_consts(c))) return rc;
     } else if (use_graph) {
         // a graph bakes dx, the courant factor and the pressure cap into its launches
@@ -714,7 +704,7 @@ int rg_level_substep(rg_ctx* c, int ilevel, double dx, int pressure_cap, int use
     } else {
         if (int rc = enqueue()) return rc;
     }
-    if (leaf && leaf_fusable(*P) && P->ncells > 0) {
+    if (prepared) {
         c->next_level = ilevel;
         c->next_cap = cap_key;
         c->next_dx = dx;
@@ -779,7 +769,7 @@ int rg_level_run(rg_ctx* c, int ilevel, double dx, int pressure_cap, double t_st
                          "rg_level_run needs a level without refined cells whose stencils stay inside it (one box)");
     double t = t_start;
     long long n = 0;
-    if (int rc = ensure_leaf(c, *P)) return rc;
+    if (int rc = ensure_flux(c, *P)) return rc;
     if (P->face_variant < 0) {
         // the first substep of a plan runs eagerly and chooses the face shape
         double dt = 0.0;
@@ -794,7 +784,7 @@ int rg_level_run(rg_ctx* c, int ilevel, double dx, int pressure_cap, double t_st
         }
     }
     record_updates(c, ilevel, *P);
-    if (int rc = ensure_leaf(c, *P)) return rc;
+    if (int rc = ensure_flux(c, *P)) return rc;
     const double cfl = c->params.courant_factor;
     const int cap_key = pressure_cap ? 1 : 0;
     const bool ready = c->next_level == ilevel && c->next_cap == cap_key && c->next_dx == dx && c->next_cfl == cfl;

@@ -16,9 +16,10 @@
 //
 // 8x8x4 and 256 threads: 46 KB of primitives and 61 KB of fluxes, so that two
 // blocks share an SM and one stages or folds while the other solves.  The
-// primitives alternate between two arrays (DevStatus::prim_sel), since bricks
-// read their neighbours' old ones; these hold them in lattice order (x
-// fastest), so a brick's rows are read in 16-byte pieces without an index.
+// primitives alternate between two arrays (DevStatus::prim_sel: d_prim and the
+// flux scratch, which this step leaves unused), since bricks read their
+// neighbours' old ones; both hold them in lattice order (x fastest), so a
+// brick's rows are read in 16-byte pieces without an index.
 #pragma once
 
 #include "rg_brick.cuh"
@@ -151,9 +152,11 @@ __global__ void __launch_bounds__(SCELLS, 2)
 #pragma unroll
         for (int iv = 0; iv < NV; ++iv) fs[iv] = (fs[iv] + f[0][iv]) - f[1][iv];
     }
-    double v[NV];  // asked for here, needed after the next problem
+    double v[NV];
+    if constexpr (!BOXED) {  // asked for here, needed after the next problem (on boxes the registers are not there)
 #pragma unroll
-    for (int iv = 0; iv < NV; ++iv) v[iv] = uold[iv * ncell + id];
+        for (int iv = 0; iv < NV; ++iv) v[iv] = uold[iv * ncell + id];
+    }
     // the faces of the cells around the brick towards it: 32 on each x and y
     // side, 64 on each z side, one a thread; the outside cell's slot `side` is
     // the face it shares with the inside cell (cx, cy, cz)
@@ -182,6 +185,10 @@ __global__ void __launch_bounds__(SCELLS, 2)
         double* to = in + (2 * idim + side) * NV * SCELLS + step_thread(cx, cy, cz);
 #pragma unroll
         for (int iv = 0; iv < NV; ++iv) to[iv * SCELLS] = f[iv];
+    }
+    if constexpr (BOXED) {
+#pragma unroll
+        for (int iv = 0; iv < NV; ++iv) v[iv] = uold[iv * ncell + id];
     }
     __syncthreads();
     // the seven updates in loop order (3 bits each: the slot, 7 the cell's own)
@@ -286,7 +293,7 @@ int launch_brick_step_t(rg_ctx* c, const Plan& P, double dx, int pressure_cap, d
     }
     const BrickGeom G{P.lat_e[0], P.lat_e[1], P.lat_e[2], P.nbox, P.bl_ext, P.bl_off, P.bl_brick_off};
     kern<<<P.ncells / SCELLS, SCELLS, STEP_SMEM, c->stream>>>(P.view(), G, P.lat_id, P.lat_ord, P.lat_kind, c->d_prim,
-                                                              c->d_prim2, (size_t)c->ncell, c->d_uold, c->d_unew,
+                                                              c->d_flux, (size_t)c->ncell, c->d_uold, c->d_unew,
                                                               c->d_status, step_consts(c), dx, cfl_consts(cfl, pressure_cap));
     return check_cuda(c, cudaGetLastError(), "brick step kernel");
 }

@@ -60,7 +60,7 @@ struct DevStatus {
     long long run_steps;                          // substeps, advanced on the device,
     long long run_limit;                          // and the step count this launch stops at
     unsigned int cfl_done;                        // blocks of a CFL pass done (its clock update)
-    int prim_sel;  // the brick step's primitives are read from d_prim (0) or d_prim2 (1)
+    int prim_sel;  // the brick step's primitives are read from d_prim (0) or the flux scratch (1)
 };
 
 // The resident AMR step's clock update after a level's CFL pass
@@ -247,7 +247,6 @@ struct rg_ctx {
     // state
     size_t cap_state = 0;
     double *d_uold = nullptr, *d_unew = nullptr, *d_prim = nullptr;
-    double* d_prim2 = nullptr;  // the brick step's second primitive array (made on first use)
     bool have_state = false;
 
     // scratch shared by all levels (levels run one after another on the stream)

@@ -801,11 +801,8 @@ int launch_leaf_prefix(rg_ctx* c, const Plan& P, double dx, int pressure_cap, do
 
 int launch_leaf_core(rg_ctx* c, const Plan& P, double dx, int pressure_cap, double cfl) {
     if (P.ncells == 0) return RG_OK;
-    if (brick_step_on(c, P)) {
-        if (!c->d_prim2) return set_error(c, RG_ERR_STATE, "second primitive array not there");
-    } else if (c->cap_flux < (size_t)(2 * c->params.ndim + 1) * (c->params.ndim + 2) * P.ncells) {
+    if (c->cap_flux < (size_t)(2 * c->params.ndim + 1) * (c->params.ndim + 2) * P.ncells)
         return set_error(c, RG_ERR_STATE, "flux scratch not sized");
-    }
     if (c->params.ndim == 1) return launch_leaf_core_t<1>(c, P, dx, pressure_cap, cfl);
     return launch_leaf_core_t<3>(c, P, dx, pressure_cap, cfl);
 }

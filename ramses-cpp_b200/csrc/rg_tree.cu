@@ -867,8 +867,6 @@ int tree_grow_arrays(rg_ctx* c, int need) {
     for (int** p : oct_scr)
         if (int rc = renew(c, p, (size_t)g1, "oct scratch")) return rc;
     if (int rc = renew(c, &c->d_prim, (size_t)nv * n1, "primitives")) return rc;
-    dev_free(c, c->d_prim2);
-    c->d_prim2 = nullptr;
     c->cap_cell = cell1;
     c->cap_grid = (size_t)g1;
     c->cap_state = (size_t)nv * n1;

@@ -202,17 +202,26 @@ __device__ __forceinline__ void fold_long(int bid, int nb, const TreeView& T, co
         if (t >= nc) {
             const int cell = P.textra[t - nc];
             double u = lane < NV ? unew[(size_t)lane * ncell + cell - 1] : 0.0;
-            for (int e0 = a; e0 < b; e0 += kLongChunk) {
-                const int e = e0 + lane;
-                if (e < b) {
-                    const int key = P.tev[e];
-                    const int slot = key & 7, cp = key >> 3;
-                    const int ps = P.level0 ? cp : (cp % TTD) * P.noct + cp / TTD;
-                    const double sign = (slot & 1) ? -1.0 : 1.0;
+            // two chunks ahead an event's key is asked for, one ahead its
+            // flux: the walk of a chunk covers both latencies (one after the
+            // other they were most of a 192-update target's 6 us)
+            auto key_of = [&](int e) { return e < b ? P.tev[e] : -1; };
+            auto fetch = [&](int key, double* v) {
+                const int slot = key & 7, cp = key >> 3;
+                const int ps = P.level0 ? cp : (cp % TTD) * P.noct + cp / TTD;
 #pragma unroll
-                    for (int iv = 0; iv < NV; ++iv)
-                        my[iv * kLongPad + lane] = dtdx * sign * flux[((size_t)slot * NV + iv) * nc + ps] * factor;
-                }
+                for (int iv = 0; iv < NV; ++iv) v[iv] = key >= 0 ? flux[((size_t)slot * NV + iv) * nc + ps] : 0.0;
+            };
+            int key = key_of(a + lane), key1 = key_of(a + kLongChunk + lane);
+            double v[NV], v1[NV];
+            fetch(key, v);
+            for (int e0 = a; e0 < b; e0 += kLongChunk) {
+                const int key2 = key_of(e0 + 2 * kLongChunk + lane);
+                fetch(key1, v1);
+                const double w = dtdx * ((key & 1) ? -1.0 : 1.0);
+                if (key >= 0)
+#pragma unroll
+                    for (int iv = 0; iv < NV; ++iv) my[iv * kLongPad + lane] = w * v[iv] * factor;
                 __syncwarp();
                 const int m = (b - e0 < kLongChunk) ? b - e0 : kLongChunk;
                 if (lane < NV) {
@@ -221,6 +230,10 @@ __device__ __forceinline__ void fold_long(int bid, int nb, const TreeView& T, co
                     for (int j = 0; j < m; ++j) u = u - s[j];
                 }
                 __syncwarp();
+                key = key1;
+                key1 = key2;
+#pragma unroll
+                for (int iv = 0; iv < NV; ++iv) v[iv] = v1[iv];
             }
             if (lane < NV) unew[(size_t)lane * ncell + cell - 1] = u;
             continue;

@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "rg_face.cuh"
+#include "rg_fast.cuh"
 #include "rg_nav.cuh"
 
 namespace rg {
@@ -176,6 +177,44 @@ __device__ __forceinline__ double err_grad_u(double vl, double vc, double vr, do
                       fabs(vc - vl) / (cm + cg + fabs(vc) + fabs(vl) + floor_val));
 }
 
+// cell_state with one reciprocal of the density for its three velocities;
+// *ok false (values outside div_by's checked range, or a NaN): take cell_state.
+// A velocity too small for the range squares to zero either way.
+__device__ __forceinline__ CellState cell_state_fast(const TreeMut& M, int cell, double gm1, bool* ok) {
+    CellState s{};
+    const size_t nc = (size_t)M.ncell, i = (size_t)cell - 1;
+    double u[5];
+    Check C;
+#pragma unroll
+    for (int iv = 0; iv < 5; ++iv) {
+        u[iv] = M.uold[(size_t)iv * nc + i];
+        C.up(u[iv]);
+    }
+    *ok = *ok && C.top_ok();
+    s.d = smax(u[0], 1e-10);
+    const double y = rcp_fast(s.d);
+    double v2 = 0.0;
+#pragma unroll
+    for (int idim = 0; idim < 3; ++idim) {
+        s.v[idim] = div_by(u[1 + idim], s.d, y);
+        v2 = v2 + s.v[idim] * s.v[idim];
+    }
+    s.p = smax((u[4] - 0.5 * s.d * v2) * gm1, s.d * 1e-10);
+    return s;
+}
+
+// err_grad(l, c, r, 1e-10) > t on finite positive values: each quotient
+// against t / 2 by the product, the division only within 2^-50 of the limit
+__device__ __forceinline__ bool grad_above(double l, double c, double r, double t) {
+    const double h = 0.5 * t;
+    auto above = [&](double a, double b) {
+        const double m = h * b;
+        if (fabs(a - m) <= m * 0x1p-50) return 2.0 * (a / b) > t;
+        return a > m;
+    };
+    return above(fabs(r - c), r + c + 1e-10) || above(fabs(c - l), c + l + 1e-10);
+}
+
 // gradient criteria (TreeUpdater.cpp:491-535), 3D hydro: density, pressure,
 // velocity (no magnetic energy on the hydro path)
 __global__ void k_flag_grad(TreeMut M, const int* __restrict__ octs, int noct, double ed, double ep, double ev,
@@ -199,8 +238,24 @@ __global__ void k_flag_grad(TreeMut M, const int* __restrict__ octs, int noct, d
             if (nl[idim] == 0) nl[idim] = M.nbor[(size_t)(2 * idim) * M.ngridmax + ig - 1];
             if (nr[idim] == 0) nr[idim] = M.nbor[(size_t)(2 * idim + 1) * M.ngridmax + ig - 1];
         }
-        const CellState sc = cell_state(M, idc + 1, gamma);
         bool ok = false;
+        if (!(ev > 0.0)) {
+            // density and pressure only: without divisions
+            bool fine = ed < 0x1p100 && ep < 0x1p100 && (ed <= 0.0 || ed > 0x1p-100) && (ep <= 0.0 || ep > 0x1p-100);
+            const CellState sc = cell_state_fast(M, idc + 1, gamma - 1.0, &fine);
+            for (int idim = 0; idim < 3 && !ok && fine; ++idim) {
+                const int id_l = nl[idim], id_r = nr[idim];
+                const CellState sl = (id_l > 0 && id_l <= M.ncell) ? cell_state_fast(M, id_l, gamma - 1.0, &fine) : sc;
+                const CellState sr = (id_r > 0 && id_r <= M.ncell) ? cell_state_fast(M, id_r, gamma - 1.0, &fine) : sc;
+                ok = fine && ((ed > 0.0 && grad_above(sl.d, sc.d, sr.d, ed)) || (ep > 0.0 && grad_above(sl.p, sc.p, sr.p, ep)));
+            }
+            if (fine) {
+                if (ok) M.flag1[idc] = 1;
+                continue;
+            }
+            ok = false;
+        }
+        const CellState sc = cell_state(M, idc + 1, gamma);
         for (int idim = 0; idim < 3 && !ok; ++idim) {
             const int id_l = nl[idim], id_r = nr[idim];
             const CellState sl = (id_l > 0 && id_l <= M.ncell) ? cell_state(M, id_l, gamma) : sc;

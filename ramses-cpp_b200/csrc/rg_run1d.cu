@@ -78,6 +78,60 @@ size_t line_smem(int m) {
     return sizeof(double) * (2 * kCta * kLineWarps + 2 * 2 * 3 * (size_t)(m + 2 * kLineHalo) + 2 * 3 * (size_t)(m + 2));
 }
 
+// The flux of one (cell, side) pair in the branch-free forms (conservative
+// interpolation of the ghost states): ghost_1d_states, own_trace and the
+// solver on the same operands.  False: not covered, take the plain forms.
+template <int RS, bool POW2>
+__device__ __forceinline__ bool line_flux_fast(const double* uc, const double* ul, const double* ur, const double* qc,
+                                               const double* ql, const double* qr, int side, const FastStep& S,
+                                               const StepK& K, double* f, unsigned& it) {
+    constexpr int NV = 3;
+    Check C;
+    double qmo[NV], qpo[NV], far[NV], near[NV], qf[NV], qn[NV], qa[NV], qb[NV], qm[NV], qp[NV];
+    trace_fast<1, POW2, true, true, true>(qc, ql, qr, K.own, S, K.gamma, qmo, qpo, C);
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) {
+        const double h = 0.5 * limited<true>(ul[iv], uc[iv], ur[iv], K.ghost, C);
+        far[iv] = side ? uc[iv] + h : uc[iv] - h;
+        near[iv] = side ? uc[iv] - h : uc[iv] + h;
+        C.up(far[iv]);
+        C.up(near[iv]);
+    }
+    auto prim = [&](const double* u, double* q) {  // ctoprim with the branch-free reciprocal
+        const double d = smax(u[0], 1e-10), o = div_by(1.0, d, rcp_fast(d));
+        q[0] = d;
+        q[1] = u[1] * o;
+        q[2] = K.gas.gm1 * d * smax(u[2] * o - (0.0 + 0.5 * q[1] * q[1]) - 0.0, K.smalle);
+    };
+    prim(far, qf);
+    prim(near, qn);
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) {
+        const double l = side ? qn[iv] - qc[iv] : qn[iv] - qf[iv], r = side ? qf[iv] - qn[iv] : qc[iv] - qn[iv];
+        qa[iv] = qn[iv] - l;
+        qb[iv] = qn[iv] + r;
+    }
+    trace_fast<1, POW2, true, true, true>(qn, qa, qb, K.own, S, K.gamma, qm, qp, C);
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) {
+        qa[iv] = side ? qmo[iv] : qm[iv];
+        qb[iv] = side ? qp[iv] : qpo[iv];
+    }
+    const bool ok = riemann_fast<1, RS>(qa, qb, f, K, it);
+    return ok && C.top_ok() && C.num_ok();
+}
+
+template <int RS>
+__device__ __noinline__ int line_flux_plain(const double* uc, const double* ul, const double* ur, const double* qc,
+                                            const double* ql, const double* qr, int side, double dt, const DxDiv& D,
+                                            const StepK& K, double* f) {
+    constexpr int NV = 3;
+    double qmo[NV], qpo[NV], qm[NV], qp[NV];
+    own_trace<1>(qc, ql, qr, dt, D, K, qmo, qpo);
+    ghost_1d_states(uc, ul, ur, side, qc, dt, D, K, qm, qp);
+    return side == 0 ? riemann<1, RS>(qm, qpo, f, K) : riemann<1, RS>(qmo, qp, f, K);
+}
+
 template <int RS>
 __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLineThreads, 1)
     k_level_run_line(TreeView T, PlanView P, double* __restrict__ uold, double* __restrict__ unew,
@@ -104,6 +158,7 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLineThreads, 1)
     }
     const double inv = 1.0 / dx;
     const DxDiv D{dx, inv, is_pow2_with_normal_inverse(dx, inv)};
+    const bool fast = K.fast && K.interpol_var == 0 && dx > 0x1p-60 && dx < 0x1p60;
     const unsigned long long start_bits = (unsigned long long)__double_as_longlong(dt_start);
     unsigned long long word = st->dtmin_bits;
     double t = st->run_t, dt = 0.0;
@@ -114,12 +169,13 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLineThreads, 1)
     for (long long guard = 0; guard < max_steps; ++guard) {
         dt = __longlong_as_double((long long)word);
         const double dtdx = dt / dx;
+        const FastStep fs2 = fast_step(dt, dx, inv);
         const double* u = S.u + cur * NV * S.pitch;
         const double* q = S.q + cur * NV * S.pitch;
         // fluxes of cells -1 .. m of the piece, lower faces first
         for (int w = threadIdx.x; w < 2 * S.fp; w += blockDim.x) {
             const int side = w >= S.fp, jj = w - side * S.fp, c = jj - 1 + kLineHalo;
-            double qc[NV], ql[NV], qr[NV], qmo[NV], qpo[NV], ul[NV], uc[NV], ur[NV], qm[NV], qp[NV], f[NV];
+            double qc[NV], ql[NV], qr[NV], ul[NV], uc[NV], ur[NV], f[NV];
             const int nb = side ? c + 1 : c - 1;
 #pragma unroll
             for (int iv = 0; iv < NV; ++iv) {
@@ -130,9 +186,27 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLineThreads, 1)
                 uc[iv] = u[iv * S.pitch + nb];
                 ur[iv] = u[iv * S.pitch + nb + 1];
             }
-            own_trace<1>(qc, ql, qr, dt, D, K, qmo, qpo);
-            ghost_1d_states(uc, ul, ur, side, qc, dt, D, K, qm, qp);
-            const int it = side == 0 ? riemann<1, RS>(qm, qpo, f, K) : riemann<1, RS>(qmo, qp, f, K);
+            unsigned it = 0;
+            bool ok = false;
+            if (fast)
+                ok = D.pow2 ? line_flux_fast<RS, true>(uc, ul, ur, qc, ql, qr, side, fs2, K, f, it)
+                            : line_flux_fast<RS, false>(uc, ul, ur, qc, ql, qr, side, fs2, K, f, it);
+            if (!ok) {
+                // (copies: the call's arrays live in memory, the loop's in registers)
+                double a[7][NV];
+#pragma unroll
+                for (int iv = 0; iv < NV; ++iv) {
+                    a[0][iv] = uc[iv];
+                    a[1][iv] = ul[iv];
+                    a[2][iv] = ur[iv];
+                    a[3][iv] = qc[iv];
+                    a[4][iv] = ql[iv];
+                    a[5][iv] = qr[iv];
+                }
+                it = line_flux_plain<RS>(a[0], a[1], a[2], a[3], a[4], a[5], side, dt, D, K, a[6]);
+#pragma unroll
+                for (int iv = 0; iv < NV; ++iv) f[iv] = a[6][iv];
+            }
             if (RS == RG_RIEMANN_EXACT && jj >= 1 && jj <= m) {
                 iters += it;
                 ++calls;

@@ -61,7 +61,7 @@ __device__ __noinline__ unsigned brick_face_plain(const double* sq, int site, in
 }
 
 // The two fluxes of one cell and direction in the branch-free forms (a ghost
-// neighbour on both sides, every staged value finite and below 2^170); false:
+// neighbour on both sides, every staged state checked: top_ok, gas_ok); false:
 // not covered, take the plain forms.
 template <int RS, bool POW2, int SITES>
 __device__ __forceinline__ bool brick_dir_fast(const double* __restrict__ sq, int site, int idim, int stride,

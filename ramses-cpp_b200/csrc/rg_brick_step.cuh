@@ -81,9 +81,12 @@ __global__ void __launch_bounds__(SCELLS, 2)
     const int bx = local % nbx, by = (local / nbx) % nby, bz = local / (nbx * nby);
     const int x0 = bx * BRICK - BHALO, y0 = by * BRICK - BHALO, z0 = bz * SBZ - BHALO;
     Check C;
-    // rows of the brick are six pairs of sites, whole pairs on either side of a wrap
+    // rows of the brick are six pairs of sites, whole pairs on either side of a
+    // wrap; a round of the block at a time: the other block of the SM covers
+    // its latency, and with the three rounds' loads in flight together the
+    // kernel was 3 % slower (registers)
     constexpr int PAIRS = SSITES / 2;
-#pragma unroll
+#pragma unroll 1
     for (int k = 0; k < (PAIRS + SCELLS - 1) / SCELLS; ++k) {
         const int t = (int)threadIdx.x + k * SCELLS;
         if (t >= PAIRS) break;
@@ -102,11 +105,13 @@ __global__ void __launch_bounds__(SCELLS, 2)
             C.up(v[iv].y);
             reinterpret_cast<double2*>(sq + iv * SSITES)[t] = v[iv];
         }
+        C.gas(v[0].x, v[4].x);
+        C.gas(v[0].y, v[4].y);
     }
     if (threadIdx.x == 0) s_min = ~0ULL;
     const bool ghost = (kind & KIND_MASK) == K_GHOST;
     // cell sizes of 2^-60 .. 2^60 keep the slopes' quotients in range
-    const bool fast = __syncthreads_and(C.top_ok()) && ghost && K.fast && D.dx > 0x1p-60 && D.dx < 0x1p60;
+    const bool fast = __syncthreads_and(C.top_ok() && C.gas_ok()) && ghost && K.fast && D.dx > 0x1p-60 && D.dx < 0x1p60;
     const FastStep S = fast_step(dt, D.dx, D.inv), Sc = fast_step(dt, 2.0 * D.dx, 0.5 * D.inv);
     const int u = threadIdx.x, x = u & 7, y = ((u >> 4) & 1) | ((u >> 2) & 2) | ((u >> 3) & 4), z = u >> 6;
     const int site = (x + BHALO) + BSIDE * (y + BHALO) + SPLANE * (z + BHALO);
@@ -152,11 +157,6 @@ __global__ void __launch_bounds__(SCELLS, 2)
 #pragma unroll
         for (int iv = 0; iv < NV; ++iv) fs[iv] = (fs[iv] + f[0][iv]) - f[1][iv];
     }
-    double v[NV];
-    if constexpr (!BOXED) {  // asked for here, needed after the next problem (on boxes the registers are not there)
-#pragma unroll
-        for (int iv = 0; iv < NV; ++iv) v[iv] = uold[iv * ncell + id];
-    }
     // the faces of the cells around the brick towards it: 32 on each x and y
     // side, 64 on each z side, one a thread; the outside cell's slot `side` is
     // the face it shares with the inside cell (cx, cy, cz)
@@ -186,10 +186,9 @@ __global__ void __launch_bounds__(SCELLS, 2)
 #pragma unroll
         for (int iv = 0; iv < NV; ++iv) to[iv * SCELLS] = f[iv];
     }
-    if constexpr (BOXED) {
+    double v[NV];
 #pragma unroll
-        for (int iv = 0; iv < NV; ++iv) v[iv] = uold[iv * ncell + id];
-    }
+    for (int iv = 0; iv < NV; ++iv) v[iv] = uold[iv * ncell + id];
     __syncthreads();
     // the seven updates in loop order (3 bits each: the slot, 7 the cell's own)
     auto reflux = [&](int slot) {

@@ -429,7 +429,7 @@ __device__ __forceinline__ bool tile_dir_fast(const TreeView& T, const PlanView&
     if (rl != c) load_rot<NDIM>(prim, ncell, rl, idim, qn);
     trace_fast<NDIM, POW2, true, false, true>(qr, qn, qf, K.ghost, Sc, K.gamma, nullptr, qp, C);
     trace_fast<NDIM, POW2, true, true, true>(qc, ql, qr, K.own, S, K.gamma, qmo, qpo, C);
-    const bool ok = C.num_ok() && C.top_ok();
+    const bool ok = C.num_ok() && C.top_ok() && C.gas_ok();
     unsigned i0 = 0, i1 = 0;
     const bool a = riemann_fast<NDIM, RS>(qm, qpo, f[0], K, i0), b = riemann_fast<NDIM, RS>(qmo, qp, f[1], K, i1);
     iters = (z0 ? 0 : i0) + (z1 ? 0 : i1);

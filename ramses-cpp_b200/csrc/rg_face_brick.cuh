@@ -74,7 +74,7 @@ __device__ __forceinline__ void brick_cell(const double* sq, int site, int p, in
 //
 // The cells go through the branch-free forms where the solver's types, the
 // cell size and the brick's values allow (one vote of the block over the
-// staged states: finite, below 2^170); they keep every lane of a warp on one
+// staged states); they keep every lane of a warp on one
 // straight line, so the two Riemann problems of a direction overlap.  Lanes
 // of a half-warp take rows y and y + 2 of the brick: rows are 12 doubles
 // apart, so the 16 lanes meet 16 different 8-byte banks.
@@ -122,11 +122,12 @@ __device__ __forceinline__ void brick_face(const PlanView& P, const BrickGeom& G
             C.up(v);
             sq[iv * BSITES + t] = v;
         }
+        C.gas(sq[t], sq[4 * BSITES + t]);
     }
     const int nc = P.ncells;
     const bool ghost = (kind & KIND_MASK) == K_GHOST;
     // cell sizes of 2^-60 .. 2^60 keep the slopes' quotients in range
-    const bool fast = __syncthreads_and(C.top_ok()) && ghost && K.fast && D.dx > 0x1p-60 && D.dx < 0x1p60;
+    const bool fast = __syncthreads_and(C.top_ok() && C.gas_ok()) && ghost && K.fast && D.dx > 0x1p-60 && D.dx < 0x1p60;
     const FastStep S = fast_step(dt, D.dx, D.inv), Sc = fast_step(dt, 2.0 * D.dx, 0.5 * D.inv);
     unsigned it = 0, done = 0;
     for (int u = threadIdx.x; u < BRICK * BRICK * BRICK; u += blockDim.x) {

@@ -61,9 +61,22 @@ __device__ __forceinline__ double sqrt_fast(double x) {
 // largest high word, numerators zero or above 2^-800 by the smallest (0 wraps
 // to the top; a nonzero low word counts), so that with divisors in [2^-140,
 // 2^700] no step of a quotient over- or underflows.
+//
+// gas(): a density below 2^30 with a pressure of at least 2^-36.  Then neither
+// pressure floor (density times 1e-20 / gamma or 1e-20) nor the floor of the
+// squared sound speed (1e-20) can act, gamma being above 1, and the forms
+// leave the floors out; gas below that takes the plain forms.
 struct Check {
     static constexpr unsigned kTop = (1023u + 170u) << 20, kBottom = (1023u - 800u) << 20;
+    static constexpr int kDense = (1023 + 30) << 20, kThin = (1023 - 36) << 20;
     unsigned mx = 0, mn = 0xffffffffu;
+    int dense = 0, thin = 0x7fffffff;
+    __device__ __forceinline__ void gas(double r, double p) {
+        dense = max(dense, __double2hiint(r));
+        thin = min(thin, __double2hiint(p));
+        up(p);
+    }
+    __device__ __forceinline__ bool gas_ok() const { return dense < kDense && thin >= kThin; }
     __device__ __forceinline__ void up(double x) { mx = max(mx, (unsigned)__double2hiint(x) & 0x7fffffffu); }
     __device__ __forceinline__ void num(double a) {
         const unsigned h = ((unsigned)__double2hiint(a) & 0x7fffffffu) | min((unsigned)__double2loint(a), 1u);
@@ -74,7 +87,7 @@ struct Check {
 };
 
 // Limited slope parameters: the slope types 1, 2, 3 and 8 (and those the
-// reference treats as 1) are min(th |l|, th |r|, cf |l + r|) with the sign of
+// reference treats as 1) are min(th min(|l|, |r|), cf |l + r|) with the sign of
 // l where l r > 0, and so are the interpolation types 1..3 of the ghost
 // branch: |l + r| >= max(|l|, |r|) there, so cf = 1 leaves a minmod as it is,
 // and th = infinity the centred slope.
@@ -88,9 +101,8 @@ __device__ __forceinline__ double limited(double ql, double qc, double qr, const
     const double l = qc - ql, r = qr - qc;
     const double c = L.cf * fabs(l + r);
     if (CHK) C.up(c);
-    double m = L.th * fabs(l);
-    const double b = L.th * fabs(r);
-    m = b < m ? b : m;
+    const double al = fabs(l), ar = fabs(r);
+    double m = L.th * (ar < al ? ar : al);
     m = c < m ? c : m;
     m = copysign(m, l);
     return l * r > 0.0 ? m : 0.0;
@@ -108,7 +120,8 @@ __device__ __forceinline__ FastStep fast_step(double dt, double dx, double inv) 
 
 // compute_slopes / ghost slopes and trace of a rotated state: the upper face
 // state in qm, the lower in qp (either may be left out).  Primitive states:
-// their density is at least 1e-10 (ctoprim).
+// their density is at least 1e-10 (ctoprim).  Without CHK the caller has
+// checked the states (top_ok and gas_ok).
 template <int NDIM, bool POW2, bool CHK, bool QM, bool QP>
 __device__ __forceinline__ void trace_fast(const double* q, const double* ql, const double* qr, const Limiter& L,
                                            const FastStep& S, double gamma, double* qm, double* qp, Check& C) {
@@ -124,15 +137,14 @@ __device__ __forceinline__ void trace_fast(const double* q, const double* ql, co
             dq[iv] = div_by(s, S.dx, S.inv);
         }
     }
-    const double r = q[0], u = q[1], p = smax(q[IP], r * 1e-20);
+    const double r = q[0], u = q[1];
     const double y = rcp_fast(r);
     if (CHK) {
-        C.up(r);
-        C.up(p);
+        C.gas(r, q[IP]);
         C.up(dq[IP]);
     }
     C.num(dq[IP]);
-    const double cs2 = smax(div_by(gamma * p, r, y), 1e-20);
+    const double cs2 = div_by(gamma * q[IP], r, y);
     const double ru = dq[1] * r;
     const double b[3] = {S.hdt * (-u * dq[0] - ru), S.hdt * (-u * dq[1] - div_by(dq[IP], r, y)),
                          S.hdt * (-u * dq[IP] - ru * cs2)};
@@ -161,7 +173,6 @@ __device__ __forceinline__ void flux_cons(const double* q, const FastGas& G, dou
     double v2 = q[1] * q[1];
 #pragma unroll
     for (int i = 2; i <= NDIM; ++i) v2 = v2 + q[i] * q[i];
-    C.num(q[IP]);
     const double E = 0.5 * q[0] * v2 + div_by(q[IP], G.gm1, G.rgm1);
     C.up(E);
     const double m = q[0] * q[1];
@@ -181,10 +192,9 @@ __device__ __forceinline__ void flux_cons(const double* q, const FastGas& G, dou
 template <int NDIM>
 __device__ __forceinline__ double cs2_fast(const double* q, const FastGas& G, Check& C) {
     constexpr int IP = Dims<NDIM>::IP;
-    C.up(q[0]);
+    C.gas(q[0], q[IP]);
     C.up(q[1]);
-    C.up(q[IP]);
-    return smax(div_by(G.gamma * q[IP], q[0], rcp_fast(q[0])), 1e-20);
+    return div_by(G.gamma * q[IP], q[0], rcp_fast(q[0]));
 }
 
 // The Riemann solvers on traced states (their density is at least 1e-10 by
@@ -201,7 +211,7 @@ __device__ __forceinline__ bool hllc_fast(const double* ql, const double* qr, do
     const double rcl = rl * (ul - sl), rcr = rr * (sr - ur), div = rcr + rcl;
     const double nu = rcr * ur + rcl * ul + (pl - pr), np = rcr * pl + rcl * pr + rcl * rcr * (ul - ur);
     const double yd = rcp_fast(div);
-    const double ustar = smax(-1e6, smin(1e6, div_by(nu, div, yd)));
+    const double ustar = div_by(nu, div, yd);  // (its clamp to +-1e6 and that of den: checked below)
     const double pstar = smax(div_by(np, div, yd), 0.0);
     const bool supl = sl > 0.0, supr = sr < 0.0, star = !(supl || supr);
     const bool left = supl || (!supr && ustar > 0.0);
@@ -209,12 +219,14 @@ __device__ __forceinline__ bool hllc_fast(const double* ql, const double* qr, do
 #pragma unroll
     for (int iv = 0; iv < NV; ++iv) q[iv] = left ? ql[iv] : qr[iv];
     flux_cons<NDIM>(q, G, f, u0, C);
-    const bool base_ok = C.top_ok() && C.num_ok() && !(pl < rl * G.smallp) && !(pr < rr * G.smallp);
+    const bool base_ok = C.top_ok() && C.gas_ok();
     Check D;
     D.num(nu);
     D.num(np);
     const double so = left ? sl : sr;
-    const double den = left ? smin(so - ustar, -1e-10) : smax(so - ustar, 1e-10);
+    const double den = so - ustar;
+    const bool den_ok = (__double2hiint(den) ^ (left ? (int)0x80000000 : 0)) > __double2hiint(1e-10);
+    const bool ustar_ok = (__double2hiint(ustar) & 0x7fffffff) < __double2hiint(1e6);
     const double yn = rcp_fast(den);
     const double w = so - q[1];
     const double rstar = div_by(q[0] * w, den, yn);
@@ -231,7 +243,7 @@ __device__ __forceinline__ bool hllc_fast(const double* ql, const double* qr, do
         const double fs = f[iv] + so * (us[iv] - u0[iv]);
         f[iv] = star ? fs : f[iv];
     }
-    return base_ok && (!star || (D.num_ok() && !(div < 1e-5)));
+    return base_ok && (!star || (D.num_ok() && den_ok && ustar_ok && !(div < 1e-5)));
 }
 
 template <int NDIM>
@@ -245,7 +257,7 @@ __device__ __forceinline__ bool llf_fast(const double* ql, const double* qr, dou
     const double ha = 0.5 * smax(fabs(ql[1]) + al, fabs(qr[1]) + ar);
 #pragma unroll
     for (int i = 0; i < NV; ++i) f[i] = 0.5 * (fl[i] + fr[i]) - ha * (ur[i] - ul[i]);
-    return C.top_ok() && C.num_ok();
+    return C.top_ok() && C.gas_ok();
 }
 
 template <int NDIM>
@@ -260,7 +272,7 @@ __device__ __forceinline__ bool hll_fast(const double* ql, const double* qr, dou
     const double w = sr - sl, inv = div_by(1.0, w, rcp_fast(w));
 #pragma unroll
     for (int i = 0; i < NV; ++i) f[i] = (sr * fl[i] - sl * fr[i] + sr * sl * (ur[i] - ul[i])) * inv;
-    return C.top_ok() && C.num_ok() && !(w < 1e-20);
+    return C.top_ok() && C.gas_ok() && !(w < 1e-20);
 }
 
 // One Newton update of the two-shock solver (RiemannSolver.cpp:221-233).

@@ -118,7 +118,7 @@ __device__ __forceinline__ bool line_flux_fast(const double* uc, const double* u
         qb[iv] = side ? qp[iv] : qpo[iv];
     }
     const bool ok = riemann_fast<1, RS>(qa, qb, f, K, it);
-    return ok && C.top_ok() && C.num_ok();
+    return ok && C.top_ok() && C.num_ok() && C.gas_ok();
 }
 
 template <int RS>

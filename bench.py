@@ -68,7 +68,8 @@ WORKLOAD = ("3D Sedov blast with octree AMR, reference levelmin 7 / levelmax 10 
             "tree and state resident on the GPU")
 BYTES_PER_CELL_UPDATE = 80  # uold read once + unew written once, 5 FP64 variables each
 FACE_SOURCES = ("rg_face.cuh", "rg_face_brick.cuh", "rg_face_pipe.cuh", "rg_physics.cuh", "rg_face.cu",
-                "rg_face_1d.cu", "rg_face_3d.cu", "rg_internal.cuh", "rg_nav.cuh")
+                "rg_face_1d.cu", "rg_face_3d.cu", "rg_internal.cuh", "rg_nav.cuh", "rg_fast.cuh", "rg_brick.cuh",
+                "rg_brick_step.cuh", "rg_fold.cuh")
 
 
 def peaks():
@@ -217,6 +218,16 @@ def _amr_cpu_window(warmup, steps, parity_after, AmrRun, RefHarness, namelist, s
            "octs_per_level": [h.count_grids(il) for il in range(A["lmin"], A["lmax"] + 1)]}
     h.close()
     return out
+
+
+NO_REFERENCE = "the reference's sources are not on this machine and no harness built from them is in oracle/_ref"
+
+
+def reference_here():
+    """Can the reference arm, the CPU baseline and the drop-in reports run here?"""
+    sys.path.insert(0, str(ROOT / "tests"))
+    from refsupport import ensure_built
+    return ensure_built("ref")
 
 
 def run_cpu_window(warmup, steps, parity_after=None, timeout=1800):
@@ -413,7 +424,7 @@ def amr_headline(args, rank, world, local_rank):
         fl = rin["fp64_flops_per_cell_update"] * face_cells / face_s / 1e12
         ops = rin["fp64_ops_per_cell_update"] * face_cells / face_s / 1e12
         fp64 = {"bound": "fp64", "achieved": fl, "peak": fp64_peak, "unit": "TFLOP/s", "frac": fl / fp64_peak,
-                "op_frac": ops / (fp64_peak / 2), "kernel": "k_face_tiles",
+                "op_frac": ops / (fp64_peak / 2), "kernel": "k_face_brick, k_face_tiles",
                 "flops_per_cell_update": rin["fp64_flops_per_cell_update"],
                 "peak_source": "rg_measure_fp64_peak: independent DFMA chains on every SM (measured here)",
                 "flops_source": "profiles/roofline_inputs.json k_face_tiles_amr (ncu)", "stale": rin["stale"]}
@@ -426,7 +437,7 @@ def amr_headline(args, rank, world, local_rank):
                    "l2": "flushed between timed coarse steps (a 256 MB write outside the timed events)",
                    "parallelism": "replicas" if world > 1 else "single GPU"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": traffic, "kernel": "k_face_tiles (every level step of the coarse step)",
+                     "traffic": traffic, "kernel": "k_face_brick (base level) and k_face_tiles (every level step of the coarse step)",
                      "algorithmic_bytes_per_launch": BYTES_PER_CELL_UPDATE * per_launch_cells,
                      "launches": level_steps, "face_share_of_step": kms[1] / step2_ms,
                      "kernel_ms_per_coarse_step": {"prim": kms[0] / 2, "face": kms[1] / 2, "fold": kms[2] / 2,
@@ -450,8 +461,9 @@ def amr_headline(args, rank, world, local_rank):
 def uniform_report(local_rank, steps, warmup, face_variant=None):
     """Config 2: the uniform 128^3 Sedov level (reference levelmin = levelmax
     = 8), MonCen + HLLC, courant 0.8, one substep per step in a CUDA graph
-    (dt finalize, brick face kernel, fold that prepares the next substep);
-    inputs larger than L2 (state, primitives and flux scratch 0.8 GB)."""
+    (dt finalize, and one kernel for fluxes, fold, and the next substep's
+    primitives and CFL candidates); inputs larger than L2 (state and two
+    primitive arrays 0.4 GB)."""
     import numpy as np
     import torch
     import rg_tree
@@ -481,7 +493,9 @@ def uniform_report(local_rank, steps, warmup, face_variant=None):
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1)
     variant = ctx.face_config(L)[0]
-    face_kernel = "k_face_brick" if variant >= 9 else ("k_face_pipe" if variant >= 7 else "k_face_tiles")
+    # without a pinned shape the level's substep is one kernel, timed as its face step (the fold's time is zero)
+    face_kernel = "k_brick_step" if face_variant is None else (
+        "k_face_brick" if variant >= 9 else ("k_face_pipe" if variant >= 7 else "k_face_tiles"))
     ctx.set_timing(True)
     nk = min(steps, 40)
     acc = np.zeros(3)
@@ -652,7 +666,8 @@ def newton_report(local_rank, stream, steps):
     ctx.close()
     torch.cuda.empty_cache()
     try:
-        out["stress"]["reference_mode_vs_reference"] = run_sample("--stress-ref", str(tmp))
+        out["stress"]["reference_mode_vs_reference"] = (run_sample("--stress-ref", str(tmp)) if reference_here()
+                                                        else {"unavailable": NO_REFERENCE})
     finally:
         tmp.unlink(missing_ok=True)
 
@@ -1063,9 +1078,9 @@ def profile_case_amr():
 
 
 def profile_case_uniform():
-    """A small run for ncu captures of the brick face kernel: the uniform
-    128^3 Sedov level, two warm-up substeps, then one eager substep inside the
-    NVTX range "capture"."""
+    """A small run for ncu captures of the brick step kernel (k_brick_step):
+    the uniform 128^3 Sedov level, two warm-up substeps (the first times the
+    face shapes), then one eager substep inside the NVTX range "capture"."""
     import torch
     import rg_tree
     import rgpu
@@ -1076,7 +1091,6 @@ def profile_case_uniform():
                                         courant_factor=0.8), 0)
     ctx.sync_topology(g)
     ctx.upload_state(u0, u0)
-    ctx.set_face_config(L, 10, 1)
     for _ in range(2):
         ctx.level_substep(L, 1.0 / 2 ** L, pressure_cap=False, use_graph=False)
     ctx.synchronize()
@@ -1126,16 +1140,19 @@ def amr_exact_report(steps):
             "same_state_bits": plain["digest"] == learned["digest"]}
 
 
-def sod_report():
-    ref = run_sample("--sod-sample", "cpu")
+def sod_report(ref_here):
     gpu = run_sample("--sod-sample", "gpu")
-    return {"workload": "1D Sod, 1024 cells (reference levelmin=levelmax=11), MinMod + HLLC, courant 0.8, "
-                        "to t=0.245", "reference_cpu": ref, "gpu": gpu,
-            "bit_identical": ref["digest"] == gpu["digest"] and ref["steps"] == gpu["steps"],
-            "wall_speedup": ref["wall_s"] / gpu["wall_s"],
-            "note": "GPU run: rg_level_run, all 1729 substeps in one CUDA graph launch whose WHILE node stops "
-                    "at t >= 0.245 on the device (no dt read back between substeps); 1024 cells per substep, so "
-                    "it is launch-latency bound"}
+    out = {"workload": "1D Sod, 1024 cells (reference levelmin=levelmax=11), MinMod + HLLC, courant 0.8, "
+                       "to t=0.245", "gpu": gpu,
+           "note": "GPU run: rg_level_run, all 1729 substeps in one launch of a cluster of eight blocks (no dt read "
+                   "back between substeps); 1024 cells per substep, so it is bound by the latency of a substep"}
+    if not ref_here:
+        out["reference_cpu"] = {"unavailable": NO_REFERENCE}
+        return out
+    ref = run_sample("--sod-sample", "cpu")
+    out.update(reference_cpu=ref, bit_identical=ref["digest"] == gpu["digest"] and ref["steps"] == gpu["steps"],
+               wall_speedup=ref["wall_s"] / gpu["wall_s"])
+    return out
 
 
 def main():
@@ -1185,6 +1202,9 @@ def main():
     if args.impl == "reference":
         if world > 1 and rank != 0:
             return
+        if not reference_here():
+            print(json.dumps({"impl": "reference", "unavailable": NO_REFERENCE}))
+            return
         out = reference_arm(args, rank, world)
         print(json.dumps(out))
         return
@@ -1195,7 +1215,8 @@ def main():
         torch.cuda.set_device(local_rank)
         dist.init_process_group("nccl", timeout=datetime.timedelta(seconds=600))
     cpu = cpu_run = None
-    if rank == 0 and world == 1 and not args.no_cpu_baseline:
+    ref_here = rank == 0 and reference_here()
+    if ref_here and world == 1 and not args.no_cpu_baseline:
         # the reference on one core, before any CUDA work: its initialisation,
         # the W warm-up coarse steps and the first 2 coarse steps of the window
         cpu_run = run_cpu_window(args.warmup, 2, parity_after=args.warmup + 2)
@@ -1223,10 +1244,10 @@ def main():
             out["ensemble"] = ens_out
             if single:
                 out["ensemble"]["parity"] = ensemble_parity(local_rank)
-                out["amr_dropin"] = amr_report(3)
+                out["amr_dropin"] = amr_report(3) if ref_here else {"unavailable": NO_REFERENCE}
                 if "newton" in out:
-                    out["newton"]["amr_exact"] = amr_exact_report(3)
-                out["sod1d"] = sod_report()
+                    out["newton"]["amr_exact"] = amr_exact_report(3) if ref_here else {"unavailable": NO_REFERENCE}
+                out["sod1d"] = sod_report(ref_here)
     if world > 1:
         import torch.distributed as dist
         dist.barrier()

@@ -164,9 +164,10 @@ int rg_get_stream(rg_ctx* ctx, void** stream);
  * as ONE CUDA graph launch: a WHILE conditional node repeats the substep and
  * a clock kernel that adds dt on the device and sets the loop condition, so
  * no dt travels to the host between substeps.  Same state bits, t and step
- * count as the host loop.  Levels of at most 1024 cells run the whole loop
- * in one single-block kernel instead (block barriers between the phases of
- * a substep, no launch per substep).  Levels without refined cells whose
+ * count as the host loop.  A 1D level of 24 to 8192 cells that is one periodic
+ * line in list order runs the whole loop in one launch of a thread-block
+ * cluster instead, any other level of at most 1024 cells in one block (no
+ * launch per substep either way).  Levels without refined cells whose
  * stencils stay inside them (uniform periodic grids), one box; max_steps
  * bounds the loop, and each launch runs at most 65,536 substeps (the host
  * relaunches until t_end or max_steps), so no launch runs for long. */
@@ -365,7 +366,9 @@ int rg_face_config(rg_ctx* ctx, int ilevel, int* variant, int* batch, float* ms)
 /* Pin the face-kernel shape of a level (variant 0..10, batch >= 1; 7 and 8
  * select the software-pipelined kernel on levels above level 0 in 2D/3D,
  * 9 and 10 the brick kernel on levels that form one complete periodic
- * lattice; elsewhere those ids run the default shape). */
+ * lattice; elsewhere those ids run the default shape).  A pinned lattice
+ * level's substeps run the face and fold kernels; otherwise (and with the
+ * choice of shapes on) they are one kernel, with the same results. */
 int rg_set_face_config(rg_ctx* ctx, int ilevel, int variant, int batch);
 
 /* ---- device-resident tree maintenance (TreeUpdater on the GPU) -------------

@@ -372,7 +372,10 @@ int refresh_tree(rg_ctx* c);
 // in DevStatus run_t/run_steps.  Larger levels are faster spread over the GPU.
 constexpr int kRunBlockCells = 1024;
 // rg_level_run on a 1D level of at most kLineCells cells that is one periodic
-// line (line_check looks once per plan): one cluster launch (rg_run1d.cu)
+// line (line_check looks once per plan): one cluster launch (rg_run1d.cu).
+// us a substep, MinMod + HLLC, cluster against block or graph: 2.5 / 10.5 at 32
+// cells, 3.3 / 19.9 at 1024, 8.3 / 21.7 at 4096, 15.5 / 22.8 at 8192; twice
+// that would be past the graph's 23
 constexpr int kLineCells = 8192;
 int line_check(rg_ctx* c, Plan& P);
 int launch_run_line(rg_ctx* c, const Plan& P, double dx, int pressure_cap, double t_end, long long max_steps);

@@ -10,6 +10,7 @@ from pathlib import Path
 import numpy as np
 import pytest
 
+import rg_amr
 import rg_tree
 import rgpu
 from refsupport import make_params
@@ -266,5 +267,27 @@ def test_brick_step_at_the_limits_matches_the_oracle(rgpu_lib, oracle, nx, level
                 a, b = np.empty_like(u), np.empty_like(u)
                 ctx.download_state(a, b)
                 assert same(a, u) and same(b, unew), (seed, k)
+    finally:
+        ctx.close()
+
+
+def test_brick_face_kernel_on_a_base_level_with_refined_cells(rgpu_lib):
+    """The 64^3 base level of an AMR run (a lattice with refined cells): the brick shapes against the gathering one."""
+    ctx = rgpu.Context(make_params(3, slope_type=2, riemann="hllc", courant_factor=0.25), 0)
+    try:
+        rg_amr.initialize(ctx, 3, 7, 8, 40000, rg_amr.sedov_primitives(3, 7), 1.4, ed=0.1, ep=0.1)
+        run = rg_amr.DeviceAmrRun(ctx, nx=1, levelmin=7, nlevelmax=8, cfl=0.25, ed=0.1, ep=0.1)
+        for _ in range(3):
+            run.coarse_step()
+        assert 0 < ctx.cell_updates(7) < 64 ** 3
+        got = []
+        n = 5 * ctx.tree_sizes()[1]
+        for variant in (1, 9, 10):
+            ctx.set_face_config(7, variant, 1)
+            ctx.set_unew(7)
+            ctx.godunov_level(7, 1e-6, 1.0 / 2 ** 7)
+            got.append(np.empty(n))
+            ctx.download_state(unew=got[-1])
+        assert same(got[0], got[1]) and same(got[0], got[2])
     finally:
         ctx.close()

@@ -946,10 +946,15 @@ int rg_level_output(rg_ctx* c, int ilevel, double* out, int64_t cap) {
     if (P->level0) return set_error(c, RG_ERR_ARG, "the coarse level has no octs to write");
     if ((int64_t)n > cap) return set_error(c, RG_ERR_ARG, "out holds fewer than 2^ndim * nvar * noct doubles");
     if (n == 0) return RG_OK;
-    if (int rc = ensure_flux(c, *P)) return rc;  // the flux scratch is large enough to stage the records
+    // The records are staged at the end of the flux scratch: the next substep
+    // of a lattice level may have its primitives, nvar doubles a cell, at the
+    // start (brick_step_on), and the scratch holds (2 ndim + 1) nvar doubles
+    // for every cell of the largest level that used it.
+    if (int rc = ensure_flux(c, *P)) return rc;
     if (c->cap_flux < n) return set_error(c, RG_ERR_STATE, "staging too small");
-    if (int rc = launch_level_output(c, *P, c->d_flux)) return rc;
-    if (int rc = check_cuda(c, cudaMemcpyAsync(out, c->d_flux, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
+    double* stage = c->d_flux + (c->cap_flux - n);
+    if (int rc = launch_level_output(c, *P, stage)) return rc;
+    if (int rc = check_cuda(c, cudaMemcpyAsync(out, stage, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
                             "level output copy"))
         return rc;
     return check_cuda(c, cudaStreamSynchronize(c->stream), "level output sync");

@@ -1,0 +1,107 @@
+"""Calls between two substeps of a level.  A lattice level's substep leaves the
+next one's primitives and CFL candidates on the device; whatever else is called
+in between, the next substep's bits and dt are the oracle's (one lattice) or
+those of an uninterrupted sequence (ensembles)."""
+import numpy as np
+import pytest
+
+import rg_ensemble as ens
+import rg_tree
+import rgpu
+from refsupport import make_params
+from test_gpu_level import bits_equal, ga_of
+
+pytestmark = pytest.mark.gpu
+
+L5 = 5
+DX5 = 1.0 / 2 ** L5
+
+
+class OracleLevel:
+    """A level stepped by the oracle."""
+
+    def __init__(self, oracle, g, level, dx, u, **kw):
+        self.o, self.ga, self.level, self.dx = oracle, ga_of(g), level, dx
+        self.params = make_params(3, **kw)
+        self.uold, self.unew = u.copy(), u.copy()
+
+    def step(self):
+        dt = self.o.courant(self.ga, 3, 5, self.level, self.dx, 1.4, 0.8, self.uold, pressure_cap=False)
+        self.o.set_unew(self.ga, 3, 5, self.level, self.uold, self.unew)
+        self.o.godunov_fine(self.ga, self.params, self.level, dt, self.dx, self.uold, self.unew)
+        self.o.set_uold(self.ga, 3, 5, self.level, self.uold, self.unew)
+        return dt
+
+
+KW = dict(slope_type=2, riemann="hllc")
+
+
+def substeps(ctx, how, n):
+    """n substeps of the level; their last dt, or None where the call does not give it."""
+    if how == "run":
+        assert ctx.level_run(L5, DX5, 1e9, max_steps=n)[1] == n
+        return None
+    for _ in range(n):
+        dt = ctx.level_substep(L5, DX5, use_graph=how == "graph", want_dt=True)
+    return dt
+
+
+@pytest.mark.parametrize("how", ["graph", "eager", "run"])
+@pytest.mark.parametrize("between", ["output", "output of a coarser level"])
+def test_snapshot_between_substeps_of_a_lattice(rgpu_lib, oracle, how, between):
+    g = rg_tree.build_uniform(3, L5)
+    u = rg_tree.random_state(g, L5, seed=3)
+    ref = OracleLevel(oracle, g, L5, DX5, u, **KW)
+    ctx = rgpu.Context(make_params(3, **KW), 0)
+    try:
+        ctx.sync_topology(g)
+        ctx.upload_state(u, u)
+        got = np.empty_like(u)
+        for n in (2, 1, 1, 2, 3, 1):  # the snapshots meet either set of primitives
+            for _ in range(n):
+                dt = ref.step()
+            dt_gpu = substeps(ctx, how, n)
+            assert dt_gpu in (None, dt)
+            rec = ctx.level_output(L5 if between == "output" else L5 - 1, 3, 5)
+            if between == "output":
+                ids = np.concatenate([g.ncoarse + ic * g.ngridmax + g.level_octs[L5] for ic in range(8)]) - 1
+                assert bits_equal(rec[:, 0].reshape(-1), np.maximum(ref.uold.reshape(5, -1)[0, ids], 1e-10))
+            ctx.download_state(uold=got)
+            assert bits_equal(got, ref.uold), n
+    finally:
+        ctx.close()
+
+
+def forest_run(f, interrupt, steps=6):
+    params = rgpu.make_params(3, gamma=f.gamma, courant_factor=0.8, **KW)
+    ctx = rgpu.Context(params, 0)
+    try:
+        ctx.sync_topology(f.grid)
+        u = f.initial_state()
+        ctx.upload_state(u, u)
+        ctx.set_level_boxes(f.level, f.first_oct, f.dx)
+        ctx.set_level_lattices(f.level, *f.lattices())
+        dts = []
+        for k in range(steps):
+            ctx.level_substep(f.level, 0.0, use_graph=k % 2 == 0)
+            dts.append(ctx.level_box_dt(f.level, f.nbox))
+            interrupt(ctx)
+        ctx.download_state(uold=u)
+        return u, np.array(dts)
+    finally:
+        ctx.close()
+
+
+def specs_of(edges, seed=7):
+    pool = ens.box_specs(64, seed=seed)
+    out = []
+    for e in edges:
+        out.append(next(s for s in pool if s.edge == e and s not in out))
+    return out
+
+
+def test_snapshot_between_substeps_of_an_ensemble(rgpu_lib):
+    f = ens.Forest(specs_of([16, 24, 16]))
+    u, dts = forest_run(f, lambda ctx: None)
+    v, dts2 = forest_run(f, lambda ctx: ctx.level_output(f.level, 3, 5))
+    assert bits_equal(dts, dts2) and bits_equal(u, v)

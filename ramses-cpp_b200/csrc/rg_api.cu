@@ -145,11 +145,13 @@ int get_plan(rg_ctx* c, int ilevel, Plan** out) {
     return RG_OK;
 }
 
-// The flux scratch is shared by all levels and baked into captured graphs:
-// growing it invalidates every graph.
+// The flux scratch is shared by all levels, baked into captured graphs and may
+// hold the next substep's primitives: growing it invalidates every graph and
+// makes the next substep start anew.
 int ensure_flux(rg_ctx* c, const Plan& P) {
     size_t need = (size_t)(2 * c->params.ndim + 1) * (c->params.ndim + 2) * (size_t)P.ncells;
     if (c->cap_flux >= need && c->d_flux) return RG_OK;
+    c->next_level = -1;
     cudaStreamSynchronize(c->stream);
     for (auto& p : c->plans)
         if (p.graph) {

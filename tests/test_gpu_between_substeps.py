@@ -105,3 +105,45 @@ def test_snapshot_between_substeps_of_an_ensemble(rgpu_lib):
     u, dts = forest_run(f, lambda ctx: None)
     v, dts2 = forest_run(f, lambda ctx: ctx.level_output(f.level, 3, 5))
     assert bits_equal(dts, dts2) and bits_equal(u, v)
+
+
+def two_list_forest():
+    """Two boxes, 16^3 and 32^3, the second one's leaf octs in a list of their own after the first one's."""
+    f = ens.Forest(specs_of([16, 32]))
+    g = f.grid
+    octs = g.level_octs[f.level]
+    first = int(f.first_oct[1])
+    g.nlevelmax = f.level + 1
+    g.headl = np.append(g.headl, octs[first]).astype(np.int32)
+    g.next[octs[first - 1] - 1] = 0
+    g.level_octs[f.level], g.level_octs[f.level + 1] = octs[:first], octs[first:]
+    return f
+
+
+def test_output_that_needs_a_larger_scratch_between_substeps(rgpu_lib):
+    """The records of the longer list do not fit the scratch the shorter list's substep left its primitives in."""
+    f = two_list_forest()
+    ext, lat_id, _ = f.lattices()
+    ncell_a = int(ext[0].prod())
+    noct = int(f.first_oct[1])
+    pos = {int(c): ic * noct + k for ic in range(8) for k, c in
+           enumerate(f.grid.ncoarse + ic * f.grid.ngridmax + f.grid.level_octs[f.level])}
+    out = []
+    for interrupt in (False, True):
+        ctx = rgpu.Context(rgpu.make_params(3, gamma=f.gamma, courant_factor=0.8, **KW), 0)
+        try:
+            ctx.sync_topology(f.grid)
+            u = f.initial_state()
+            ctx.upload_state(u, u)
+            ctx.set_level_boxes(f.level, f.first_oct[:2], f.dx[:1])
+            ctx.set_level_lattices(f.level, ext[:1], lat_id[:ncell_a],
+                                   np.array([pos[int(c)] for c in lat_id[:ncell_a]], np.int32))
+            for k in range(4):
+                ctx.level_substep(f.level, 0.0, use_graph=k != 1)
+                if interrupt and k == 1:
+                    ctx.level_output(f.level + 1, 3, 5)
+            ctx.download_state(uold=u)
+            out.append((u, ctx.level_box_dt(f.level, 1)))
+        finally:
+            ctx.close()
+    assert bits_equal(out[0][0], out[1][0]) and bits_equal(out[0][1], out[1][1])

@@ -642,12 +642,12 @@ int rg_level_substep(rg_ctx* c, int ilevel, double dx, int pressure_cap, int use
     const double cfl = c->params.courant_factor;
     const int cap_key = pressure_cap ? 1 : 0;
     bool prepared = leaf && leaf_fusable(*P) && P->ncells > 0;  // for the next substep
+    // the CFL word and primitives are current if the previous call was a
+    // fused substep of this level with the same arguments
+    const bool ready = leaf && leaf_fusable(*P) && c->next_level == ilevel && c->next_cap == cap_key &&
+                       c->next_dx == dx && c->next_cfl == cfl;
+    c->next_level = -1;  // (an unfused substep forms its own: another level's are gone then)
     if (leaf) {
-        // the CFL word and primitives are current if the previous call was a
-        // fused substep of this level with the same arguments
-        const bool ready = leaf_fusable(*P) && c->next_level == ilevel && c->next_cap == cap_key &&
-                           c->next_dx == dx && c->next_cfl == cfl;
-        c->next_level = -1;
         if (!ready) {
             if (int rc = launch_leaf_prefix(c, *P, dx, pressure_cap, cfl)) return rc;
         } else if (c->timing) {

@@ -147,3 +147,25 @@ def test_output_that_needs_a_larger_scratch_between_substeps(rgpu_lib):
         finally:
             ctx.close()
     assert bits_equal(out[0][0], out[1][0]) and bits_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("how", ["graph", "eager", "run"])
+def test_substep_of_a_refined_level_between_substeps(rgpu_lib, oracle, how):
+    """Every cell of level 4 is refined: its substep moves nothing, but takes its own CFL step and primitives."""
+    g = rg_tree.build_uniform(3, L5)
+    u = rg_tree.random_state(g, L5, seed=5)
+    ref = OracleLevel(oracle, g, L5, DX5, u, **KW)
+    ctx = rgpu.Context(make_params(3, **KW), 0)
+    try:
+        ctx.sync_topology(g)
+        ctx.upload_state(u, u)
+        got = np.empty_like(u)
+        for n in (2, 1, 2):
+            for _ in range(n):
+                dt = ref.step()
+            assert substeps(ctx, how, n) in (None, dt)
+            assert ctx.level_substep(L5 - 1, 2 * DX5, use_graph=how == "graph", want_dt=True) == 1e10
+            ctx.download_state(uold=got)
+            assert bits_equal(got, ref.uold), n
+    finally:
+        ctx.close()

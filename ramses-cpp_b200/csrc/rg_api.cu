@@ -895,6 +895,15 @@ int rg_set_level_boxes(rg_ctx* c, int ilevel, int nbox, const int* first_oct, co
         boxes[(size_t)b] = BoxStep{0ULL, 0.0, dx[b], 0.0, 0.0, 0, 0};
     }
     if (int rc = check_cuda(c, cudaStreamSynchronize(c->stream), "boxes sync")) return rc;
+    // captured launches name the arrays freed here
+    if (P->graph) {
+        cudaGraphExecDestroy(P->graph);
+        P->graph = nullptr;
+    }
+    drop_amr_graphs(c);
+    // lattices belong to the partition they were set for, and so does a shape timed on them
+    if (!P->pinned && P->face_variant >= kFirstBrickVariant) P->face_variant = -1;
+    drop_lattice(c, *P);
     dev_free(c, P->obox);
     dev_free(c, P->boxes);
     P->obox = nullptr;
@@ -912,10 +921,6 @@ int rg_set_level_boxes(rg_ctx* c, int ilevel, int nbox, const int* first_oct, co
         return rc;
     if (int rc = check_cuda(c, cudaStreamSynchronize(c->stream), "boxes upload")) return rc;
     P->nbox = nbox;
-    if (P->graph) {
-        cudaGraphExecDestroy(P->graph);
-        P->graph = nullptr;
-    }
     return RG_OK;
 }
 

@@ -300,6 +300,19 @@ int build_lattice(rg_ctx* c, Plan& P) {
     return part ? RG_OK : build_order(c, P);
 }
 
+void drop_lattice(rg_ctx* c, Plan& P) {
+    dev_free(c, P.lat_id);
+    dev_free(c, P.lat_p);
+    dev_free(c, P.lat_ord);
+    dev_free(c, P.lat_mask);
+    dev_free(c, P.bl_ext);
+    dev_free(c, P.bl_off);
+    dev_free(c, P.bl_brick_off);
+    P.lat_id = P.lat_p = P.lat_ord = P.bl_ext = P.bl_off = P.bl_brick_off = nullptr;
+    P.lat_mask = nullptr;
+    P.lattice = P.box_lattice = P.bl_nbricks = 0;
+}
+
 int set_box_lattices(rg_ctx* c, Plan& P, const int* ext, const int* lat_id, const int* lat_p) {
     const int nbox = P.nbox;
     std::vector<int> hext(ext, ext + 3 * (size_t)nbox), hoff((size_t)nbox), hbrick((size_t)nbox + 1);

@@ -391,13 +391,7 @@ void free_plan(rg_ctx* c, Plan& p) {
     dev_free(c, p.obox);
     dev_free(c, p.boxes);
     dev_free(c, p.read_ids);
-    dev_free(c, p.lat_id);
-    dev_free(c, p.lat_p);
-    dev_free(c, p.lat_ord);
-    dev_free(c, p.lat_mask);
-    dev_free(c, p.bl_ext);
-    dev_free(c, p.bl_off);
-    dev_free(c, p.bl_brick_off);
+    drop_lattice(c, p);
     dev_free(c, p.tlong);
     p = Plan();
 }

@@ -169,3 +169,34 @@ def test_substep_of_a_refined_level_between_substeps(rgpu_lib, oracle, how):
             assert bits_equal(got, ref.uold), n
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("first", [[0, 2, 3], [0, 0.5, 2, 3], [0, 0.5, 1.25, 2, 3]])
+def test_boxes_partitioned_anew(rgpu_lib, first):
+    """A partition set after lattices were: the same boxes without them as if they had never been (fewer, as many and
+    more boxes; a context that sees only the second partition gives the bits)."""
+    f = ens.Forest(specs_of([16, 16, 16]))
+    n = int(f.first_oct[1])
+    first = np.array([int(x * n) for x in first], np.int32)
+    dx = np.full(len(first) - 1, f.dx[0])
+    out = []
+    for before in (True, False):
+        ctx = rgpu.Context(rgpu.make_params(3, gamma=f.gamma, courant_factor=0.8, **KW), 0)
+        try:
+            ctx.sync_topology(f.grid)
+            u = f.initial_state()
+            ctx.upload_state(u, u)
+            if before:
+                ctx.set_level_boxes(f.level, f.first_oct, f.dx)
+                ctx.set_level_lattices(f.level, *f.lattices())
+                for _ in range(3):
+                    ctx.level_substep(f.level, 0.0)
+                ctx.upload_state(u, u)
+            ctx.set_level_boxes(f.level, first, dx)
+            for _ in range(3):
+                ctx.level_substep(f.level, 0.0)
+            ctx.download_state(uold=u)
+            out.append((u, ctx.level_box_dt(f.level, len(dx))))
+        finally:
+            ctx.close()
+    assert bits_equal(out[0][0], out[1][0]) and bits_equal(out[0][1], out[1][1])

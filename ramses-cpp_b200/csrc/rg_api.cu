@@ -932,10 +932,6 @@ int rg_set_level_lattices(rg_ctx* c, int ilevel, int nbox, const int* extent, co
     if (!P || P->nbox != nbox) return set_error(c, RG_ERR_STATE, "set the level's boxes (rg_set_level_boxes) first");
     if (c->params.ndim != 3) return set_error(c, RG_ERR_UNSUPPORTED, "box lattices are a 3D form");
     if (int rc = set_box_lattices(c, *P, extent, lat_id, lat_p)) return rc;
-    if (P->graph) {
-        cudaGraphExecDestroy(P->graph);
-        P->graph = nullptr;
-    }
     // the tuned shape was timed without the brick kernel
     P->face_variant = -1;
     return RG_OK;

@@ -329,52 +329,54 @@ int set_box_lattices(rg_ctx* c, Plan& P, const int* ext, const int* lat_id, cons
     hbrick[(size_t)nbox] = (int)bricks;
     if (sites != P.ncells) return set_error(c, RG_ERR_ARG, "box lattices do not cover the level's cells once");
     int8_t kind0 = 0;
-    int* d_bad = nullptr;
-    int* d_seen = nullptr;
-    auto fail = [&](int rc) {
-        dev_free(c, d_bad);
-        dev_free(c, d_seen);
-        dev_free(c, P.lat_id);
-        dev_free(c, P.lat_p);
-        dev_free(c, P.bl_ext);
-        dev_free(c, P.bl_off);
-        dev_free(c, P.bl_brick_off);
-        dev_free(c, P.lat_ord);
-        P.lat_id = P.lat_p = P.lat_ord = P.bl_ext = P.bl_off = P.bl_brick_off = nullptr;
-        P.box_lattice = 0;
+    // made beside the level's present lattices, which stay as they are when the maps are refused
+    struct {
+        int *id = nullptr, *p = nullptr, *ext = nullptr, *off = nullptr, *brick = nullptr, *bad = nullptr, *seen = nullptr;
+    } N;
+    auto drop = [&](int rc) {
+        for (int* a : {N.id, N.p, N.ext, N.off, N.brick, N.bad, N.seen}) dev_free(c, a);
         return rc;
     };
-    fail(RG_OK);
     const size_t n = (size_t)P.ncells;
-    if (check_cuda(c, dev_alloc(c, &d_bad, sizeof(int)), "box lattice flag") ||
-        check_cuda(c, dev_alloc(c, &d_seen, sizeof(int) * n), "box lattice marks") ||
-        check_cuda(c, dev_alloc(c, &P.lat_id, sizeof(int) * n), "box lattice ids") ||
-        check_cuda(c, dev_alloc(c, &P.lat_p, sizeof(int) * n), "box lattice positions") ||
-        check_cuda(c, dev_alloc(c, &P.bl_ext, sizeof(int) * hext.size()), "box lattice extents") ||
-        check_cuda(c, dev_alloc(c, &P.bl_off, sizeof(int) * hoff.size()), "box lattice offsets") ||
-        check_cuda(c, dev_alloc(c, &P.bl_brick_off, sizeof(int) * hbrick.size()), "box lattice bricks"))
-        return fail(RG_ERR_NOMEM);
+    if (check_cuda(c, dev_alloc(c, &N.bad, sizeof(int)), "box lattice flag") ||
+        check_cuda(c, dev_alloc(c, &N.seen, sizeof(int) * n), "box lattice marks") ||
+        check_cuda(c, dev_alloc(c, &N.id, sizeof(int) * n), "box lattice ids") ||
+        check_cuda(c, dev_alloc(c, &N.p, sizeof(int) * n), "box lattice positions") ||
+        check_cuda(c, dev_alloc(c, &N.ext, sizeof(int) * hext.size()), "box lattice extents") ||
+        check_cuda(c, dev_alloc(c, &N.off, sizeof(int) * hoff.size()), "box lattice offsets") ||
+        check_cuda(c, dev_alloc(c, &N.brick, sizeof(int) * hbrick.size()), "box lattice bricks"))
+        return drop(RG_ERR_NOMEM);
     cudaStream_t s = c->stream;
     cudaMemcpyAsync(&kind0, P.kind, 1, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(P.lat_id, lat_id, sizeof(int) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(P.lat_p, lat_p, sizeof(int) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(P.bl_ext, hext.data(), sizeof(int) * hext.size(), cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(P.bl_off, hoff.data(), sizeof(int) * hoff.size(), cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(P.bl_brick_off, hbrick.data(), sizeof(int) * hbrick.size(), cudaMemcpyHostToDevice, s);
-    cudaMemsetAsync(d_seen, 0, sizeof(int) * n, s);
-    cudaMemsetAsync(d_bad, 0, sizeof(int), s);
-    if (int rc = check_cuda(c, cudaStreamSynchronize(s), "box lattice upload")) return fail(rc);
+    cudaMemcpyAsync(N.id, lat_id, sizeof(int) * n, cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(N.p, lat_p, sizeof(int) * n, cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(N.ext, hext.data(), sizeof(int) * hext.size(), cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(N.off, hoff.data(), sizeof(int) * hoff.size(), cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(N.brick, hbrick.data(), sizeof(int) * hbrick.size(), cudaMemcpyHostToDevice, s);
+    cudaMemsetAsync(N.seen, 0, sizeof(int) * n, s);
+    cudaMemsetAsync(N.bad, 0, sizeof(int), s);
+    if (int rc = check_cuda(c, cudaStreamSynchronize(s), "box lattice upload")) return drop(rc);
     if ((kind0 & KIND_MASK) != K_GHOST && (kind0 & KIND_MASK) != K_SAME)
-        return fail(set_error(c, RG_ERR_ARG, "box lattices need a level whose faces are all ghost faces"));
-    k_box_lattice_check<<<lblocks(c, P.ncells), LTPB, 0, s>>>(tree_view(c), P.view(), nbox, P.bl_ext, P.bl_off,
-                                                             P.lat_id, P.lat_p, kind0, d_seen, d_bad);
+        return drop(set_error(c, RG_ERR_ARG, "box lattices need a level whose faces are all ghost faces"));
+    k_box_lattice_check<<<lblocks(c, P.ncells), LTPB, 0, s>>>(tree_view(c), P.view(), nbox, N.ext, N.off, N.id, N.p,
+                                                             kind0, N.seen, N.bad);
     int bad = 1;
-    cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (int rc = check_cuda(c, cudaStreamSynchronize(s), "box lattice check")) return fail(rc);
-    dev_free(c, d_bad);
-    dev_free(c, d_seen);
-    d_bad = d_seen = nullptr;
-    if (bad) return fail(set_error(c, RG_ERR_ARG, "box lattices do not match the level's neighbours"));
+    cudaMemcpyAsync(&bad, N.bad, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (int rc = check_cuda(c, cudaStreamSynchronize(s), "box lattice check")) return drop(rc);
+    if (bad) return drop(set_error(c, RG_ERR_ARG, "box lattices do not match the level's neighbours"));
+    // the captured substep names the lattices that go
+    if (P.graph) {
+        cudaGraphExecDestroy(P.graph);
+        P.graph = nullptr;
+    }
+    drop_lattice(c, P);
+    dev_free(c, N.bad);
+    dev_free(c, N.seen);
+    P.lat_id = N.id;
+    P.lat_p = N.p;
+    P.bl_ext = N.ext;
+    P.bl_off = N.off;
+    P.bl_brick_off = N.brick;
     P.box_lattice = 1;
     P.bl_nbricks = (int)bricks;
     P.lat_kind = kind0;

@@ -200,3 +200,23 @@ def test_boxes_partitioned_anew(rgpu_lib, first):
         finally:
             ctx.close()
     assert bits_equal(out[0][0], out[1][0]) and bits_equal(out[0][1], out[1][1])
+
+
+def test_refused_lattices_change_nothing(rgpu_lib):
+    """Wrong maps between captured substeps are refused; the level goes on with the lattices it has."""
+    f = ens.Forest(specs_of([16, 24, 16]))
+    ext, lat_id, lat_p = f.lattices()
+    swapped, shifted = lat_p.copy(), lat_id.copy()
+    swapped[[5, 6]] = swapped[[6, 5]]
+    shifted[:16 ** 3] = np.roll(shifted[:16 ** 3].reshape(16, 16, 16), 1, axis=2).reshape(-1)
+
+    def wrong(ctx):
+        for e, i, p in ((ext, lat_id, swapped), (ext, shifted, lat_p), (ext[[1, 0, 2]], lat_id, lat_p),
+                        (ext + 1, lat_id, lat_p)):
+            with pytest.raises(rgpu.RGError):
+                ctx.set_level_lattices(f.level, e, i, p)
+        assert ctx.face_config(f.level)[0] == shape[0]
+    shape = []
+    u, dts = forest_run(f, lambda ctx: shape.append(ctx.face_config(f.level)[0]))
+    v, dts2 = forest_run(f, wrong)
+    assert bits_equal(dts, dts2) and bits_equal(u, v)

@@ -347,8 +347,10 @@ int rg_set_level_boxes(rg_ctx* ctx, int ilevel, int nbox, const int* first_oct, 
  * site of every box (box after box, x fastest), its cell id and its position
  * p = (ic-1)*noct + k in the level (k = position of its oct in the level
  * list).  The library checks every site against the level's neighbours,
- * ghost stencils and interface kinds before it uses the brick face kernel on
- * the boxes; a mismatch returns RG_ERR_ARG and changes nothing. */
+ * ghost stencils and interface kinds before it uses the brick kernels on
+ * the boxes; a mismatch returns RG_ERR_ARG and changes nothing.  Maps that
+ * match but give some box the cells of another (boxes alike in another order)
+ * are accepted and not used. */
 int rg_set_level_lattices(rg_ctx* ctx, int ilevel, int nbox, const int* extent, const int* lat_id,
                           const int* lat_p);
 /* dt of every box in the last substep (nbox must equal the level's count);

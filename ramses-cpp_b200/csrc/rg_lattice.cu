@@ -121,10 +121,12 @@ __global__ void k_lattice_check(TreeView T, PlanView P, int ex, int ey, int ez, 
 // Box lattices supplied by the host (one periodic lattice per ensemble box):
 // every site's plan position must hold that site's cell, every plan position
 // must appear once, and the plan's neighbours, ghost stencils and kinds must
-// be the box lattice's (periodic inside the box).
+// be the box lattice's (periodic inside the box).  *other: a site's cell is of
+// another box of the partition (boxes alike whose lattices come in another
+// order), whose dt and dx the brick kernels would not take.
 __global__ void k_box_lattice_check(TreeView T, PlanView P, int nbox, const int* __restrict__ ext,
                                     const int* __restrict__ off, const int* __restrict__ lat_id,
-                                    const int* __restrict__ lat_p, int kind0, int* seen, int* bad) {
+                                    const int* __restrict__ lat_p, int kind0, int* seen, int* bad, int* other) {
     const int n = P.ncells;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < n; g += gridDim.x * blockDim.x) {
         int lo = 0, hi = nbox - 1;
@@ -146,6 +148,7 @@ __global__ void k_box_lattice_check(TreeView T, PlanView P, int nbox, const int*
             atomicExch(bad, 1);
             continue;
         }
+        if (box_of(P, p) != b) atomicExch(other, 1);
         for (int s = 0; s < 6; ++s) {
             const int idim = s >> 1, side = s & 1, d = side ? 1 : -1;
             auto at = [&](int o) {
@@ -338,7 +341,7 @@ int set_box_lattices(rg_ctx* c, Plan& P, const int* ext, const int* lat_id, cons
         return rc;
     };
     const size_t n = (size_t)P.ncells;
-    if (check_cuda(c, dev_alloc(c, &N.bad, sizeof(int)), "box lattice flag") ||
+    if (check_cuda(c, dev_alloc(c, &N.bad, 2 * sizeof(int)), "box lattice flags") ||
         check_cuda(c, dev_alloc(c, &N.seen, sizeof(int) * n), "box lattice marks") ||
         check_cuda(c, dev_alloc(c, &N.id, sizeof(int) * n), "box lattice ids") ||
         check_cuda(c, dev_alloc(c, &N.p, sizeof(int) * n), "box lattice positions") ||
@@ -354,22 +357,23 @@ int set_box_lattices(rg_ctx* c, Plan& P, const int* ext, const int* lat_id, cons
     cudaMemcpyAsync(N.off, hoff.data(), sizeof(int) * hoff.size(), cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(N.brick, hbrick.data(), sizeof(int) * hbrick.size(), cudaMemcpyHostToDevice, s);
     cudaMemsetAsync(N.seen, 0, sizeof(int) * n, s);
-    cudaMemsetAsync(N.bad, 0, sizeof(int), s);
+    cudaMemsetAsync(N.bad, 0, 2 * sizeof(int), s);
     if (int rc = check_cuda(c, cudaStreamSynchronize(s), "box lattice upload")) return drop(rc);
     if ((kind0 & KIND_MASK) != K_GHOST && (kind0 & KIND_MASK) != K_SAME)
         return drop(set_error(c, RG_ERR_ARG, "box lattices need a level whose faces are all ghost faces"));
     k_box_lattice_check<<<lblocks(c, P.ncells), LTPB, 0, s>>>(tree_view(c), P.view(), nbox, N.ext, N.off, N.id, N.p,
-                                                             kind0, N.seen, N.bad);
-    int bad = 1;
-    cudaMemcpyAsync(&bad, N.bad, sizeof(int), cudaMemcpyDeviceToHost, s);
+                                                             kind0, N.seen, N.bad, N.bad + 1);
+    int bad[2] = {1, 1};
+    cudaMemcpyAsync(bad, N.bad, sizeof(bad), cudaMemcpyDeviceToHost, s);
     if (int rc = check_cuda(c, cudaStreamSynchronize(s), "box lattice check")) return drop(rc);
-    if (bad) return drop(set_error(c, RG_ERR_ARG, "box lattices do not match the level's neighbours"));
+    if (bad[0]) return drop(set_error(c, RG_ERR_ARG, "box lattices do not match the level's neighbours"));
     // the captured substep names the lattices that go
     if (P.graph) {
         cudaGraphExecDestroy(P.graph);
         P.graph = nullptr;
     }
     drop_lattice(c, P);
+    if (bad[1]) return drop(RG_OK);  // accepted, but of no use: the level stays a general one
     dev_free(c, N.bad);
     dev_free(c, N.seen);
     P.lat_id = N.id;

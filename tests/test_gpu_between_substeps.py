@@ -220,3 +220,33 @@ def test_refused_lattices_change_nothing(rgpu_lib):
     u, dts = forest_run(f, lambda ctx: shape.append(ctx.face_config(f.level)[0]))
     v, dts2 = forest_run(f, wrong)
     assert bits_equal(dts, dts2) and bits_equal(u, v)
+
+
+def test_lattices_of_boxes_in_another_order(rgpu_lib):
+    """The maps of two boxes of one size exchanged: every neighbour matches, but a box's dt and dx are not those of
+    the cells listed for it; the same bits as without lattices."""
+    f = ens.Forest(specs_of([16, 24, 16]))
+    ext, lat_id, lat_p = f.lattices()
+    n = 16 ** 3
+
+    def exchanged(a):
+        a = a.copy()
+        a[:n], a[-n:] = a[-n:].copy(), a[:n].copy()
+        return a
+    out = []
+    for lattices in ((ext, exchanged(lat_id), exchanged(lat_p)), None):
+        ctx = rgpu.Context(rgpu.make_params(3, gamma=f.gamma, courant_factor=0.8, **KW), 0)
+        try:
+            ctx.sync_topology(f.grid)
+            u = f.initial_state()
+            ctx.upload_state(u, u)
+            ctx.set_level_boxes(f.level, f.first_oct, f.dx)
+            if lattices:
+                ctx.set_level_lattices(f.level, *lattices)
+            for _ in range(3):
+                ctx.level_substep(f.level, 0.0)
+            ctx.download_state(uold=u)
+            out.append((u, ctx.level_box_dt(f.level, f.nbox)))
+        finally:
+            ctx.close()
+    assert bits_equal(out[0][0], out[1][0]) and bits_equal(out[0][1], out[1][1])

@@ -216,7 +216,7 @@ void dev_free(rg_ctx* c, void* p) {
 void remember_shape(rg_ctx* c, const Plan& P) {
     if (P.ilevel < 0) return;
     if ((int)c->tuned.size() <= P.ilevel) c->tuned.resize((size_t)P.ilevel + 1);
-    c->tuned[(size_t)P.ilevel] = TunedShape{P.face_variant, P.face_batch, P.ncells, P.face_ms};
+    c->tuned[(size_t)P.ilevel] = TunedShape{P.face_variant, P.face_batch, P.ncells, P.face_ms, P.pinned};
 }
 
 int refresh_tree(rg_ctx* c) {
@@ -932,8 +932,9 @@ int rg_set_level_lattices(rg_ctx* c, int ilevel, int nbox, const int* extent, co
     if (!P || P->nbox != nbox) return set_error(c, RG_ERR_STATE, "set the level's boxes (rg_set_level_boxes) first");
     if (c->params.ndim != 3) return set_error(c, RG_ERR_UNSUPPORTED, "box lattices are a 3D form");
     if (int rc = set_box_lattices(c, *P, extent, lat_id, lat_p)) return rc;
-    // the tuned shape was timed without the brick kernel
+    // the tuned shape was timed, or pinned, without the brick kernels
     P->face_variant = -1;
+    P->pinned = false;
     return RG_OK;
 }
 

@@ -250,3 +250,35 @@ def test_lattices_of_boxes_in_another_order(rgpu_lib):
         finally:
             ctx.close()
     assert bits_equal(out[0][0], out[1][0]) and bits_equal(out[0][1], out[1][1])
+
+
+def fold_ms(ctx, level, dx):
+    """Kernel time of a substep's fold: nothing (two events in a row, 3 us) where the substep is one kernel, whose time
+    is the face step's; 20 us and more for the fold of 64^3 cells."""
+    ctx.set_timing(True)
+    ctx.level_substep(level, dx, use_graph=False)
+    ctx.level_substep(level, dx, use_graph=False)
+    ctx.synchronize()
+    face, fold = ctx.kernel_ms()[1:3]
+    ctx.set_timing(False)
+    assert face > 0.004
+    return fold
+
+
+def test_pinned_shape_outlives_its_plan(rgpu_lib):
+    """A pinned lattice level runs the face and fold kernels, also after the plans are rebuilt."""
+    g = rg_tree.build_uniform(3, 7)
+    u = rg_tree.random_state(g, 7, seed=2)
+    ctx = rgpu.Context(make_params(3, **KW), 0)
+    try:
+        for k in range(3):
+            ctx.sync_topology(g)
+            ctx.upload_state(u, u)
+            ctx.level_substep(7, 1.0 / 128)
+            assert (fold_ms(ctx, 7, 1.0 / 128) > 0.008) == (k > 0), k
+            if k == 0:
+                ctx.set_face_config(7, 10, 1)
+                assert fold_ms(ctx, 7, 1.0 / 128) > 0.008
+            assert ctx.face_config(7)[0] == 10 or k == 0
+    finally:
+        ctx.close()

@@ -313,7 +313,9 @@ int launch_line(rg_ctx* c, const Plan& P, double dx, int pressure_cap, double t_
     const StepK K = step_consts(c);
     auto kern = k_level_run_line<RS>;
     const size_t smem = line_smem(P.ncells / kCta);
-    if (int rc = check_cuda(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    // the kernel's limit is the longest line's: threads with lines of several sizes share it
+    if (int rc = check_cuda(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    (int)line_smem(kLineCells / kCta)),
                             "line run shared memory"))
         return rc;
     kern<<<kCta, kLineThreads, smem, c->stream>>>(tree_view(c), P.view(), c->d_uold, c->d_unew, c->d_prim, c->d_status,

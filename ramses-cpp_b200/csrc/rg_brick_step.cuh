@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(SCELLS, 2)
     if (threadIdx.x == 0) s_min = ~0ULL;
     const bool ghost = (kind & KIND_MASK) == K_GHOST;
     // cell sizes of 2^-60 .. 2^60 keep the slopes' quotients in range
-    const bool fast = __syncthreads_and(C.top_ok() && C.gas_ok()) && ghost && K.fast && D.dx > 0x1p-60 && D.dx < 0x1p60;
+    const bool fast = __syncthreads_and(C.top_ok() && C.gas_ok()) && ghost && D.dx > 0x1p-60 && D.dx < 0x1p60;
     const FastStep S = fast_step(dt, D.dx, D.inv), Sc = fast_step(dt, 2.0 * D.dx, 0.5 * D.inv);
     const int u = threadIdx.x, x = u & 7, y = ((u >> 4) & 1) | ((u >> 2) & 2) | ((u >> 3) & 4), z = u >> 6;
     const int site = (x + BHALO) + BSIDE * (y + BHALO) + SPLANE * (z + BHALO);
@@ -135,8 +135,7 @@ __global__ void __launch_bounds__(SCELLS, 2)
         }
         if (!ok) {
             double g[2 * NV];  // (the call's array lives in memory, the loop's in registers)
-            it = brick_face_plain<RS, SSITES>(sq, site, idim, stride, 0, ghost, dt, D, K, g) +
-                 brick_face_plain<RS, SSITES>(sq, site, idim, stride, 1, ghost, dt, D, K, g + NV);
+            it = brick_dir_plain<RS, SSITES>(sq, site, idim, stride, 0u, ghost, dt, D, K, g);
 #pragma unroll
             for (int k = 0; k < 2 * NV; ++k) f[k / NV][k % NV] = g[k];
         }

@@ -28,10 +28,11 @@ constexpr int BRICK_THREADS = 256;
 constexpr size_t BRICK_SMEM = sizeof(double) * 5 * BSITES;  // 69,120 bytes (3D: nvar 5)
 
 // One cell of a brick: its fluxes in the three directions to the scratch, its
-// own flux sum in slot order.  zero: bit s set where slot s faces a refined
-// cell and carries no flux.
-template <int RS, bool FAST, bool POW2>
-__device__ __forceinline__ void brick_cell(const double* sq, int site, int p, int nc, bool ghost, double dt,
+// own flux sum in slot order.  FORMS: this instance has the branch-free forms
+// (fast: the brick's values allow them); without, the plain ones are in line.
+// zero: bit s set where slot s faces a refined cell and carries no flux.
+template <int RS, bool FORMS, bool POW2>
+__device__ __forceinline__ void brick_cell(const double* sq, int site, int p, int nc, bool ghost, bool fast, double dt,
                                            const DxDiv& D, const FastStep& S, const FastStep& Sc, const StepK& K,
                                            unsigned zero, double* __restrict__ flux, double* __restrict__ fsum,
                                            unsigned& iters) {
@@ -44,18 +45,19 @@ __device__ __forceinline__ void brick_cell(const double* sq, int site, int p, in
         double f[2][NV];
         double* out = flux + (size_t)(2 * idim * NV) * nc + p;
         unsigned it = 0;
-        bool ok = false;
         const int stride = idim == 0 ? 1 : (idim == 1 ? BSIDE : BSIDE * BSIDE);
         const unsigned none = (zero >> (2 * idim)) & 3u;
-        if (FAST) ok = brick_dir_fast<RS, POW2, BSITES>(sq, site, idim, stride, S, Sc, K, f[0], f[1], it);
-        if (!ok || none) {
-            double g[2 * NV];  // (the call's array lives in memory, the loop's in registers)
+        if constexpr (FORMS) {
+            bool ok = false;
+            if (fast) ok = brick_dir_fast<RS, POW2, BSITES>(sq, site, idim, stride, S, Sc, K, f[0], f[1], it);
+            if (!ok || none) {
+                double g[2 * NV];  // (the call's array lives in memory, the loop's in registers)
+                it = brick_dir_plain<RS, BSITES>(sq, site, idim, stride, none, ghost, dt, D, K, g);
 #pragma unroll
-            for (int k = 0; k < 2 * NV; ++k) g[k] = 0.0;
-            it = none & 1u ? 0u : brick_face_plain<RS, BSITES>(sq, site, idim, stride, 0, ghost, dt, D, K, g);
-            it += none & 2u ? 0u : brick_face_plain<RS, BSITES>(sq, site, idim, stride, 1, ghost, dt, D, K, g + NV);
-#pragma unroll
-            for (int k = 0; k < 2 * NV; ++k) f[k / NV][k % NV] = g[k];
+                for (int k = 0; k < 2 * NV; ++k) f[k / NV][k % NV] = g[k];
+            }
+        } else {
+            it = brick_dir<RS, BSITES>(sq, site, idim, stride, none, ghost, dt, D, K, f[0]);
         }
 #pragma unroll
         for (int k = 0; k < 2 * NV; ++k) out[(size_t)k * nc] = f[k / NV][k % NV];
@@ -72,13 +74,13 @@ __device__ __forceinline__ void brick_cell(const double* sq, int site, int p, in
 // then every cell's fluxes and own flux sum.  Newton statistics of the exact
 // solver are added to iters / calls.
 //
-// The cells go through the branch-free forms where the solver's types, the
-// cell size and the brick's values allow (one vote of the block over the
-// staged states); they keep every lane of a warp on one
+// The cells go through the branch-free forms where the solver's types (FORMS:
+// the launch looks), the cell size and the brick's values allow (one vote of
+// the block over the staged states); they keep every lane of a warp on one
 // straight line, so the two Riemann problems of a direction overlap.  Lanes
 // of a half-warp take rows y and y + 2 of the brick: rows are 12 doubles
 // apart, so the 16 lanes meet 16 different 8-byte banks.
-template <int RS, bool BOXED>
+template <int RS, bool BOXED, bool FORMS>
 __device__ __forceinline__ void brick_face(const PlanView& P, const BrickGeom& G, const int* __restrict__ lat_id,
                                            const int* __restrict__ lat_p, const uint8_t* __restrict__ lat_mask,
                                            int kind, const double* __restrict__ prim, size_t ncell,
@@ -119,15 +121,15 @@ __device__ __forceinline__ void brick_face(const PlanView& P, const BrickGeom& G
 #pragma unroll
         for (int iv = 0; iv < NV; ++iv) {
             const double v = __ldg(prim + iv * ncell + id);
-            C.up(v);
+            if (FORMS) C.up(v);
             sq[iv * BSITES + t] = v;
         }
-        C.gas(sq[t], sq[4 * BSITES + t]);
+        if (FORMS) C.gas(sq[t], sq[4 * BSITES + t]);
     }
     const int nc = P.ncells;
     const bool ghost = (kind & KIND_MASK) == K_GHOST;
     // cell sizes of 2^-60 .. 2^60 keep the slopes' quotients in range
-    const bool fast = __syncthreads_and(C.top_ok() && C.gas_ok()) && ghost && K.fast && D.dx > 0x1p-60 && D.dx < 0x1p60;
+    const bool fast = __syncthreads_and(!FORMS || (C.top_ok() && C.gas_ok())) && ghost && D.dx > 0x1p-60 && D.dx < 0x1p60;
     const FastStep S = fast_step(dt, D.dx, D.inv), Sc = fast_step(dt, 2.0 * D.dx, 0.5 * D.inv);
     unsigned it = 0, done = 0;
     for (int u = threadIdx.x; u < BRICK * BRICK * BRICK; u += blockDim.x) {
@@ -138,23 +140,23 @@ __device__ __forceinline__ void brick_face(const PlanView& P, const BrickGeom& G
         const unsigned zero = lat_mask ? lat_mask[g] : 0u;
         if (zero & LAT_REFINED) continue;
         const int p = lat_p[g];
-        if (!fast) brick_cell<RS, false, false>(sq, site, p, nc, ghost, dt, D, S, Sc, K, zero, flux, fsum, it);
-        else if (D.pow2) brick_cell<RS, true, true>(sq, site, p, nc, ghost, dt, D, S, Sc, K, zero, flux, fsum, it);
-        else brick_cell<RS, true, false>(sq, site, p, nc, ghost, dt, D, S, Sc, K, zero, flux, fsum, it);
+        if (!FORMS || D.pow2)
+            brick_cell<RS, FORMS, true>(sq, site, p, nc, ghost, fast, dt, D, S, Sc, K, zero, flux, fsum, it);
+        else brick_cell<RS, FORMS, false>(sq, site, p, nc, ghost, fast, dt, D, S, Sc, K, zero, flux, fsum, it);
         done += 6 - __popc(zero);
     }
     iters += it;
     calls += done;
 }
 
-template <int RS, int MINB, bool BOXED>
+template <int RS, int MINB, bool BOXED, bool FORMS>
 __global__ void __launch_bounds__(BRICK_THREADS, MINB)
     k_face_brick(PlanView P, BrickGeom G, const int* __restrict__ lat_id, const int* __restrict__ lat_p,
                  const uint8_t* __restrict__ lat_mask, int kind, const double* __restrict__ prim, size_t ncell, double* __restrict__ flux,
                  double* __restrict__ fsum, DevStatus* st, const __grid_constant__ StepK K) {
     extern __shared__ __align__(16) double sq[];  // [NV][BSITES]
     unsigned long long iters = 0, calls = 0;
-    brick_face<RS, BOXED>(P, G, lat_id, lat_p, lat_mask, kind, prim, ncell, flux, fsum, st, K, (int)blockIdx.x, sq, iters,
+    brick_face<RS, BOXED, FORMS>(P, G, lat_id, lat_p, lat_mask, kind, prim, ncell, flux, fsum, st, K, (int)blockIdx.x, sq, iters,
                           calls);
     if (RS == RG_RIEMANN_EXACT) {
         for (int o = 16; o > 0; o >>= 1) {
@@ -168,9 +170,9 @@ __global__ void __launch_bounds__(BRICK_THREADS, MINB)
     }
 }
 
-template <int RS, int MINB, bool BOXED = false>
-int launch_face_brick(rg_ctx* c, const Plan& P, const StepK& K, const double* prim, double* flux, double* fsum) {
-    auto kern = k_face_brick<RS, MINB, BOXED>;
+template <int RS, int MINB, bool BOXED, bool FORMS>
+int launch_face_brick_t(rg_ctx* c, const Plan& P, const StepK& K, const double* prim, double* flux, double* fsum) {
+    auto kern = k_face_brick<RS, MINB, BOXED, FORMS>;
     static bool attr_set[64] = {};  // per device: the shared-memory opt-in is a function attribute
     const int dev = c->device & 63;
     if (!attr_set[dev]) {
@@ -186,6 +188,12 @@ int launch_face_brick(rg_ctx* c, const Plan& P, const StepK& K, const double* pr
     kern<<<nbricks, BRICK_THREADS, BRICK_SMEM, c->stream>>>(P.view(), G, P.lat_id, P.lat_p, P.lat_mask, P.lat_kind, prim,
                                                             (size_t)c->ncell, flux, fsum, c->d_status, K);
     return check_cuda(c, cudaGetLastError(), "brick face kernel");
+}
+
+template <int RS, int MINB, bool BOXED = false>
+int launch_face_brick(rg_ctx* c, const Plan& P, const StepK& K, const double* prim, double* flux, double* fsum) {
+    return K.fast ? launch_face_brick_t<RS, MINB, BOXED, true>(c, P, K, prim, flux, fsum)
+                  : launch_face_brick_t<RS, MINB, BOXED, false>(c, P, K, prim, flux, fsum);
 }
 
 }  // namespace rg

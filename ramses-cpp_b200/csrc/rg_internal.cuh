@@ -452,13 +452,24 @@ int launch_leaf_core(rg_ctx* c, const Plan& p, double dx, int pressure_cap, doub
 // a leaf level whose stencils and updates stay inside it: its fold can prepare
 // the next substep
 inline bool leaf_fusable(const Plan& P) { return P.nextra_prim == 0 && P.ntarg == P.ncells && !P.level0; }
+// The branch-free forms (rg_fast.cuh) have slope types 1, 2, 3, 8 and those
+// compute_slope treats as 1, interpolation types 1..3, and a gamma - 1 whose
+// quotients may use its reciprocal.
+inline bool forms_apply(const rg_params& p) {
+    const int st = p.slope_type, it = p.interpol_type;
+    const double gm1 = p.gamma - 1.0;
+    return st != 0 && !(st >= 4 && st <= 7) && it >= 1 && it <= 3 && gm1 > 0x1p-20 && gm1 < 0x1p20;
+}
 // The substep of such a level in one kernel (rg_brick_step.cuh): a lattice (of
 // one grid or of every box) whose update order is known, unless a face shape
 // was pinned or the choice of shapes is off.  Up to kRunBlockCells cells the
-// run kernel's arrays are used.
+// run kernel's arrays are used.  Without the branch-free forms the face and
+// fold kernels are the better two: the forms' place is taken by a call for
+// each direction of a cell (us a substep of 128^3 cells, slope type 7: 1163
+// against 780).
 inline bool brick_step_on(const rg_ctx* c, const Plan& P) {
     return P.lat_ord && leaf_fusable(P) && P.nactive == P.ncells && P.ncells > kRunBlockCells && !P.pinned &&
-           !c->no_autotune && (P.nbox > 0 ? P.box_lattice != 0 : P.lattice != 0);
+           forms_apply(c->params) && !c->no_autotune && (P.nbox > 0 ? P.box_lattice != 0 : P.lattice != 0);
 }
 int launch_brick_prefix(rg_ctx* c, const Plan& P, double dx, int pressure_cap, double courant_factor);
 int launch_brick_step(rg_ctx* c, const Plan& P, double dx, int pressure_cap, double courant_factor);

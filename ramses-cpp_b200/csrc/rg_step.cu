@@ -617,14 +617,14 @@ StepK step_consts(const rg_ctx* c) {
     K.exact_niter = p.exact_niter > 0 ? p.exact_niter : 10;
     K.exact_tol = p.exact_tol > 0 ? p.exact_tol : 1e-6;
     K.mlp = (p.riemann == RG_RIEMANN_EXACT && p.exact_guess == RG_GUESS_LEARNED && c->mlp_valid) ? c->d_mlp : nullptr;
-    // slope types 1, 2, 3, 8 and those compute_slope treats as 1; 0 and 4..7 take the plain forms
+    // (the limiters of the types forms_apply names)
     const int st = p.slope_type, it = p.interpol_type;
     K.own = st == 2 || st == 3 ? Limiter{2.0, 0.5} : (st == 8 ? Limiter{1.5, 0.5} : Limiter{1.0, 1.0});
     K.ghost = it == 1 ? Limiter{0.5, 1.0} : (it == 2 ? Limiter{1.0, 0.25} : Limiter{HUGE_VAL, 0.25});
     K.gas = FastGas{p.gamma, p.gamma - 1.0, 1.0 / (p.gamma - 1.0), K.smallp, (p.gamma + 1.0) / (2.0 * p.gamma),
                     1.0 / p.gamma, 0};
     K.gas.fast = K.gas.gm1 > 0x1p-20 && K.gas.gm1 < 0x1p20;
-    K.fast = st != 0 && !(st >= 4 && st <= 7) && it >= 1 && it <= 3 && K.gas.fast;
+    K.fast = forms_apply(p);
     return K;
 }
 

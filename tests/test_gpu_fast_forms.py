@@ -291,3 +291,24 @@ def test_brick_face_kernel_on_a_base_level_with_refined_cells(rgpu_lib):
         assert same(got[0], got[1]) and same(got[0], got[2])
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("kw,one", [(dict(slope_type=2), True), (dict(slope_type=0), False), (dict(slope_type=7), False),
+                                    (dict(interpol_type=0), False), (dict(interpol_type=4), False),
+                                    (dict(riemann="acoustic"), True), (dict(riemann="exact", slope_type=5), False)])
+def test_lattice_substeps_take_one_kernel_where_the_forms_apply(rgpu_lib, kw, one):
+    """A 64^3 substep's fold time: none in the one-kernel step; slope and interpolation types without branch-free forms
+    take the face and fold kernels (there the one kernel was up to 2.7 times slower)."""
+    g = rg_tree.build_uniform(3, 7)
+    u = rg_tree.random_state(g, 7, seed=1)
+    ctx = rgpu.Context(make_params(3, **{**dict(slope_type=1, riemann="hllc"), **kw}), 0)
+    try:
+        ctx.sync_topology(g)
+        ctx.upload_state(u, u)
+        ctx.set_timing(True)
+        for _ in range(3):
+            ctx.level_substep(7, 1.0 / 128, use_graph=False)
+        ctx.synchronize()
+        assert (ctx.kernel_ms()[2] < 0.008) == one
+    finally:
+        ctx.close()

@@ -39,10 +39,12 @@ struct BrickGeom {
 
 // The two fluxes of one cell and direction in the plain forms, one trace of the
 // cell for both; sides in `none` (bit per side) carry no flux.  Returns the
-// Newton updates.  In line in the kernels without branch-free forms; a call
-// where those do not cover a cell (one per direction: a call per face formed
+// Newton updates.  In line in the kernels without branch-free forms, a call
+// where those do not cover a cell: one per direction (a call per face formed
 // the cell's trace twice and took 1.3 times the two-kernel step's time where
-// every cell went that way).
+// every cell went that way), and without the forms with floors in it (what the
+// call may overwrite costs the loop around it also where it is not made: with
+// them k_brick_step took 474 instead of 434 us at 128^3).
 template <int RS, int SITES>
 __device__ __forceinline__ unsigned brick_dir(const double* sq, int site, int idim, int stride, unsigned none, bool ghost,
                                               double dt, const DxDiv& D, const StepK& K, double* f) {
@@ -106,9 +108,10 @@ __device__ __noinline__ unsigned brick_face_plain(const double* sq, int site, in
 }
 
 // The two fluxes of one cell and direction in the branch-free forms (a ghost
-// neighbour on both sides, every staged state checked: top_ok, gas_ok); false:
-// not covered, take the plain forms.
-template <int RS, bool POW2, int SITES>
+// neighbour on both sides, every staged state checked: top_ok, gas_ok; FLOOR:
+// with the floors, the states checked here); false: not covered, take the
+// plain forms.
+template <int RS, bool POW2, bool FLOOR, int SITES, bool CHK = false>
 __device__ __forceinline__ bool brick_dir_fast(const double* __restrict__ sq, int site, int idim, int stride,
                                                const FastStep& S, const FastStep& Sc, const StepK& K, double* f0,
                                                double* f1, unsigned& iters) {
@@ -121,11 +124,11 @@ __device__ __forceinline__ bool brick_dir_fast(const double* __restrict__ sq, in
     B.load(sq, site - 2 * stride, qfl);
     B.load(sq, site + 2 * stride, qfr);
     Check C;
-    trace_fast<3, POW2, false, true, true>(qc, ql, qr, K.own, S, K.gamma, qmo, qpo, C);
-    trace_fast<3, POW2, false, true, false>(ql, qfl, qc, K.ghost, Sc, K.gamma, qm, nullptr, C);
-    trace_fast<3, POW2, false, false, true>(qr, qc, qfr, K.ghost, Sc, K.gamma, nullptr, qp, C);
-    const bool ok = C.num_ok();
-    const bool a = riemann_fast<3, RS>(qm, qpo, f0, K, iters), b = riemann_fast<3, RS>(qmo, qp, f1, K, iters);
+    trace_fast<3, POW2, CHK, true, true, FLOOR>(qc, ql, qr, K.own, S, K.gamma, qmo, qpo, C);
+    trace_fast<3, POW2, CHK, true, false, FLOOR>(ql, qfl, qc, K.ghost, Sc, K.gamma, qm, nullptr, C);
+    trace_fast<3, POW2, CHK, false, true, FLOOR>(qr, qc, qfr, K.ghost, Sc, K.gamma, nullptr, qp, C);
+    const bool ok = C.num_ok() && (!CHK || C.top_ok());
+    const bool a = riemann_fast<3, RS, FLOOR>(qm, qpo, f0, K, iters), b = riemann_fast<3, RS, FLOOR>(qmo, qp, f1, K, iters);
     rot_swap<3>(f0, idim);
     rot_swap<3>(f1, idim);
     return ok && a && b;
@@ -133,7 +136,7 @@ __device__ __forceinline__ bool brick_dir_fast(const double* __restrict__ sq, in
 
 // One of them: both face states of both cells are formed and the side's
 // chosen, so the two sides share one piece of code.
-template <int RS, bool POW2, int SITES>
+template <int RS, bool POW2, bool FLOOR, int SITES, bool CHK = false>
 __device__ __forceinline__ bool brick_face_fast(const double* __restrict__ sq, int site, int idim, int stride, int side,
                                                 const FastStep& S, const FastStep& Sc, const StepK& K, double* f) {
     constexpr int NV = 5;
@@ -144,20 +147,20 @@ __device__ __forceinline__ bool brick_face_fast(const double* __restrict__ sq, i
     B.load(sq, site, qc);
     B.load(sq, site - stride, ql);
     B.load(sq, site + stride, qr);
-    trace_fast<3, POW2, false, true, true>(qc, ql, qr, K.own, S, K.gamma, qmo, qpo, C);
+    trace_fast<3, POW2, CHK, true, true, FLOOR>(qc, ql, qr, K.own, S, K.gamma, qmo, qpo, C);
     B.load(sq, n, qc);
     B.load(sq, n - stride, ql);
     B.load(sq, n + stride, qr);
-    trace_fast<3, POW2, false, true, true>(qc, ql, qr, K.ghost, Sc, K.gamma, qm, qp, C);
+    trace_fast<3, POW2, CHK, true, true, FLOOR>(qc, ql, qr, K.ghost, Sc, K.gamma, qm, qp, C);
 #pragma unroll
     for (int iv = 0; iv < NV; ++iv) {
         ql[iv] = side ? qmo[iv] : qm[iv];
         qr[iv] = side ? qp[iv] : qpo[iv];
     }
     unsigned it = 0;
-    const bool a = riemann_fast<3, RS>(ql, qr, f, K, it);
+    const bool a = riemann_fast<3, RS, FLOOR>(ql, qr, f, K, it);
     rot_swap<3>(f, idim);
-    return C.num_ok() && a;
+    return C.num_ok() && (!CHK || C.top_ok()) && a;
 }
 
 }  // namespace rg

@@ -38,12 +38,15 @@ __device__ __forceinline__ int step_thread(int x, int y, int z) {
     return x | ((y & 2) << 2) | ((y & 1) << 4) | ((y & 4) << 3) | (z << 6);
 }
 
-template <int RS, bool BOXED>
-__global__ void __launch_bounds__(SCELLS, 2)
-    k_brick_step(const __grid_constant__ PlanView P, BrickGeom G, const int* __restrict__ lat_id,
-                 const int* __restrict__ lat_ord, int kind, double* __restrict__ prim0, double* __restrict__ prim1,
-                 size_t ncell, double* __restrict__ uold, double* __restrict__ unew, DevStatus* st,
-                 const __grid_constant__ StepK K, double dx, CflK F) {
+// FLOOR: in the forms with floors; without, false (and nothing done) if the
+// brick's values need those.  VOTE: the block looks at the staged states, not
+// each cell.
+template <int RS, bool BOXED, bool FLOOR, bool VOTE>
+__device__ __forceinline__ bool step_brick(const PlanView& P, const BrickGeom& G, const int* __restrict__ lat_id,
+                                           const int* __restrict__ lat_ord, int kind, double* __restrict__ prim0,
+                                           double* __restrict__ prim1, size_t ncell, double* __restrict__ uold,
+                                           double* __restrict__ unew, DevStatus* st, const StepK& K, double dx,
+                                           const CflK& F) {
     constexpr int NV = 5;
     extern __shared__ __align__(16) double sq[];  // primitives [NV][SSITES], then incoming fluxes [6][NV][SCELLS]
     double* in = sq + NV * SSITES;
@@ -105,13 +108,15 @@ __global__ void __launch_bounds__(SCELLS, 2)
             C.up(v[iv].y);
             reinterpret_cast<double2*>(sq + iv * SSITES)[t] = v[iv];
         }
-        C.gas(v[0].x, v[4].x);
-        C.gas(v[0].y, v[4].y);
+        if (!FLOOR) {
+            C.gas(v[0].x, v[4].x);
+            C.gas(v[0].y, v[4].y);
+        }
     }
     if (threadIdx.x == 0) s_min = ~0ULL;
     const bool ghost = (kind & KIND_MASK) == K_GHOST;
-    // cell sizes of 2^-60 .. 2^60 keep the slopes' quotients in range
-    const bool fast = __syncthreads_and(C.top_ok() && C.gas_ok()) && ghost && D.dx > 0x1p-60 && D.dx < 0x1p60;
+    const bool fast = __syncthreads_and(!VOTE || (C.top_ok() && (FLOOR || C.gas_ok()))) && ghost && forms_take(D.dx);
+    if (!FLOOR && !fast) return false;
     const FastStep S = fast_step(dt, D.dx, D.inv), Sc = fast_step(dt, 2.0 * D.dx, 0.5 * D.inv);
     const int u = threadIdx.x, x = u & 7, y = ((u >> 4) & 1) | ((u >> 2) & 2) | ((u >> 3) & 4), z = u >> 6;
     const int site = (x + BHALO) + BSIDE * (y + BHALO) + SPLANE * (z + BHALO);
@@ -130,8 +135,8 @@ __global__ void __launch_bounds__(SCELLS, 2)
         unsigned it = 0;
         bool ok = false;
         if (fast) {
-            ok = D.pow2 ? brick_dir_fast<RS, true, SSITES>(sq, site, idim, stride, S, Sc, K, f[0], f[1], it)
-                        : brick_dir_fast<RS, false, SSITES>(sq, site, idim, stride, S, Sc, K, f[0], f[1], it);
+            ok = D.pow2 ? brick_dir_fast<RS, true, FLOOR, SSITES, !VOTE>(sq, site, idim, stride, S, Sc, K, f[0], f[1], it)
+                        : brick_dir_fast<RS, false, FLOOR, SSITES, !VOTE>(sq, site, idim, stride, S, Sc, K, f[0], f[1], it);
         }
         if (!ok) {
             double g[2 * NV];  // (the call's array lives in memory, the loop's in registers)
@@ -172,8 +177,8 @@ __global__ void __launch_bounds__(SCELLS, 2)
         double f[NV];
         bool ok = false;
         if (fast) {
-            ok = D.pow2 ? brick_face_fast<RS, true, SSITES>(sq, outside, idim, stride, side, S, Sc, K, f)
-                        : brick_face_fast<RS, false, SSITES>(sq, outside, idim, stride, side, S, Sc, K, f);
+            ok = D.pow2 ? brick_face_fast<RS, true, FLOOR, SSITES, !VOTE>(sq, outside, idim, stride, side, S, Sc, K, f)
+                        : brick_face_fast<RS, false, FLOOR, SSITES, !VOTE>(sq, outside, idim, stride, side, S, Sc, K, f);
         }
         if (!ok) {
             double g[NV];
@@ -224,6 +229,35 @@ __global__ void __launch_bounds__(SCELLS, 2)
             atomicAdd(&st->exact_iters, wi);
             atomicAdd(&st->exact_calls, 6ull * 32ull);
         }
+    }
+    return true;
+}
+
+// A brick with gas the forms without floors do not cover, from its staging on.
+// Only the HLLC solver has both (us a substep at 128^3, without floors / with
+// them everywhere: 454 / 518; a hypersonic flow a third of whose cells are at
+// the pressure floor: 686 with both, 1065 with the plain forms behind those
+// without floors).  In the others the floors are a few comparisons, and what a
+// second copy does to the first one's registers costs more (LLF 456 with both,
+// 430 with floors everywhere).
+template <int RS, bool BOXED>
+__device__ __noinline__ void step_brick_floor(const PlanView& P, BrickGeom G, const int* lat_id, const int* lat_ord,
+                                              int kind, double* prim0, double* prim1, size_t ncell, double* uold,
+                                              double* unew, DevStatus* st, const StepK& K, double dx, CflK F) {
+    step_brick<RS, BOXED, true, false>(P, G, lat_id, lat_ord, kind, prim0, prim1, ncell, uold, unew, st, K, dx, F);
+}
+
+template <int RS, bool BOXED>
+__global__ void __launch_bounds__(SCELLS, 2)
+    k_brick_step(const __grid_constant__ PlanView P, const __grid_constant__ BrickGeom G,
+                 const int* __restrict__ lat_id, const int* __restrict__ lat_ord, int kind, double* __restrict__ prim0,
+                 double* __restrict__ prim1, size_t ncell, double* __restrict__ uold, double* __restrict__ unew,
+                 DevStatus* st, const __grid_constant__ StepK K, double dx, const __grid_constant__ CflK F) {
+    if constexpr (RS != RG_RIEMANN_HLLC) {
+        step_brick<RS, BOXED, true, true>(P, G, lat_id, lat_ord, kind, prim0, prim1, ncell, uold, unew, st, K, dx, F);
+    } else {
+        if (!step_brick<RS, BOXED, false, true>(P, G, lat_id, lat_ord, kind, prim0, prim1, ncell, uold, unew, st, K, dx, F))
+            step_brick_floor<RS, BOXED>(P, G, lat_id, lat_ord, kind, prim0, prim1, ncell, uold, unew, st, K, dx, F);
     }
 }
 

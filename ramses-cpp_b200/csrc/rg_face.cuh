@@ -221,12 +221,12 @@ __device__ __forceinline__ int riemann(const double* ql, const double* qr, doubl
 
 // The branch-free solvers (the exact one loops, its updates are branch-free;
 // the acoustic one has its plain form only).
-template <int NDIM, int RS>
+template <int NDIM, int RS, bool FLOOR = false>
 __device__ __forceinline__ bool riemann_fast(const double* ql, const double* qr, double* f, const StepK& K,
                                              unsigned& iters) {
-    if constexpr (RS == RG_RIEMANN_HLLC) return hllc_fast<NDIM>(ql, qr, f, K.gas);
-    else if constexpr (RS == RG_RIEMANN_HLL) return hll_fast<NDIM>(ql, qr, f, K.gas);
-    else if constexpr (RS == RG_RIEMANN_LLF) return llf_fast<NDIM>(ql, qr, f, K.gas);
+    if constexpr (RS == RG_RIEMANN_HLLC) return hllc_fast<NDIM, FLOOR>(ql, qr, f, K.gas);
+    else if constexpr (RS == RG_RIEMANN_HLL) return hll_fast<NDIM, FLOOR>(ql, qr, f, K.gas);
+    else if constexpr (RS == RG_RIEMANN_LLF) return llf_fast<NDIM, FLOOR>(ql, qr, f, K.gas);
     else if constexpr (RS == RG_RIEMANN_EXACT) {
         int it;
         const bool ok = exact_fast<NDIM>(ql, qr, f, K.gas, K.exact_niter, K.exact_tol,
@@ -332,14 +332,14 @@ __device__ __forceinline__ void neighbour_face(const TreeView& T, const PlanView
 // the next launch (nothing ever waits on another block).
 constexpr int TILE = 32;
 
-// The two fluxes of level cell p (cell id c) along idim in the plain forms, to
-// the scratch.  LEVEL0 as in k_face_tiles.  Returns the Newton updates and
-// adds the Riemann problems solved to *calls.
+// The two fluxes of level cell p (cell id c) along idim in the plain forms.
+// LEVEL0 as in k_face_tiles.  Returns the Newton updates and adds the Riemann
+// problems solved to calls.
 template <int NDIM, int RS, bool LEVEL0>
-__device__ __noinline__ unsigned tile_dir_plain(const TreeView& T, const PlanView& P, const double* __restrict__ prim,
-                                                const double* __restrict__ uold, int p, int c, int idim, int kd0,
-                                                int kd1, double dt, const DxDiv& D, const StepK& K, double* flux,
-                                                unsigned* calls) {
+__device__ __forceinline__ unsigned tile_dir(const TreeView& T, const PlanView& P, const double* __restrict__ prim,
+                                             const double* __restrict__ uold, int p, int c, int idim, int kd0, int kd1,
+                                             double dt, const DxDiv& D, const StepK& K, double (*fl)[Dims<NDIM>::NV],
+                                             unsigned& calls) {
     constexpr int NV = Dims<NDIM>::NV;
     const size_t ncell = (size_t)T.ncell;
     const int nc = P.ncells, s0 = 2 * idim;
@@ -376,12 +376,28 @@ __device__ __noinline__ unsigned tile_dir_plain(const TreeView& T, const PlanVie
                                                  qf);
             if (side == 0) iters += riemann<NDIM, RS>(qf, qpo, f, K);
             else iters += riemann<NDIM, RS>(qmo, qf, f, K);
-            ++*calls;
+            ++calls;
             rot_swap<NDIM>(f, idim);
         }
 #pragma unroll
-        for (int iv = 0; iv < NV; ++iv) flux[((size_t)s * NV + iv) * nc + p] = f[iv];
+        for (int iv = 0; iv < NV; ++iv) fl[side][iv] = f[iv];
     }
+    return iters;
+}
+// The same as a call that leaves them in the scratch, for cells the
+// branch-free forms do not cover.
+template <int NDIM, int RS>
+__device__ __noinline__ unsigned tile_dir_plain(const TreeView& T, const PlanView& P, const double* __restrict__ prim,
+                                                const double* __restrict__ uold, int p, int c, int idim, int kd0,
+                                                int kd1, double dt, const DxDiv& D, const StepK& K, double* out,
+                                                unsigned* calls) {
+    constexpr int NV = Dims<NDIM>::NV;
+    double f[2][NV];
+    unsigned n = 0;
+    const unsigned iters = tile_dir<NDIM, RS, false>(T, P, prim, uold, p, c, idim, kd0, kd1, dt, D, K, f, n);
+    *calls += n;
+#pragma unroll
+    for (int k = 0; k < 2 * NV; ++k) out[(size_t)k * P.ncells] = f[k / NV][k % NV];
     return iters;
 }
 
@@ -418,6 +434,11 @@ __device__ __forceinline__ bool tile_dir_fast(const TreeView& T, const PlanView&
     load_rot<NDIM>(prim, ncell, r, idim, qr);
     const FastStep S = fast_step(dt, D.dx, D.inv), Sc = fast_step(dt, 2.0 * D.dx, 0.5 * D.inv);
     Check C;
+    // one cold cell sends its warp to the plain forms anyway: none of it comes here first
+    C.gas(qc[0], qc[NV - 1]);
+    C.gas(ql[0], ql[NV - 1]);
+    C.gas(qr[0], qr[NV - 1]);
+    if (__any_sync(__activemask(), !C.gas_ok())) return false;
     load_rot<NDIM>(prim, ncell, ll, idim, qf);
 #pragma unroll
     for (int iv = 0; iv < NV; ++iv) qn[iv] = qc[iv];
@@ -429,7 +450,7 @@ __device__ __forceinline__ bool tile_dir_fast(const TreeView& T, const PlanView&
     if (rl != c) load_rot<NDIM>(prim, ncell, rl, idim, qn);
     trace_fast<NDIM, POW2, true, false, true>(qr, qn, qf, K.ghost, Sc, K.gamma, nullptr, qp, C);
     trace_fast<NDIM, POW2, true, true, true>(qc, ql, qr, K.own, S, K.gamma, qmo, qpo, C);
-    const bool ok = C.num_ok() && C.top_ok() && C.gas_ok();
+    const bool ok = C.num_ok() && C.top_ok();
     unsigned i0 = 0, i1 = 0;
     const bool a = riemann_fast<NDIM, RS>(qm, qpo, f[0], K, i0), b = riemann_fast<NDIM, RS>(qmo, qp, f[1], K, i1);
     iters = (z0 ? 0 : i0) + (z1 ? 0 : i1);
@@ -444,8 +465,10 @@ __device__ __forceinline__ bool tile_dir_fast(const TreeView& T, const PlanView&
 }
 
 // LEVEL0: instantiated for level 0 (the coarse cells, first-order traces) or
-// for the other levels, so neither instance carries the other's code
-template <int NDIM, int RS, int R, int MINB, bool BOXED, bool LEVEL0 = false>
+// for the other levels, so neither instance carries the other's code.  FORMS:
+// with the branch-free forms (3D) and a call for the cells they do not cover,
+// or with the plain ones in line
+template <int NDIM, int RS, int R, int MINB, bool BOXED, bool LEVEL0, bool FORMS>
 __global__ void __launch_bounds__(TILE * NDIM * R, MINB)
     k_face_tiles(const __grid_constant__ TreeView T, const __grid_constant__ PlanView P, const double* __restrict__ prim, const double* __restrict__ uold,
                  double* __restrict__ flux, double* __restrict__ fsum, DevStatus* st,
@@ -498,9 +521,12 @@ __global__ void __launch_bounds__(TILE * NDIM * R, MINB)
                     double* out = flux + (size_t)s0 * NV * nc + p;
                     unsigned it = 0;
                     bool ok = false;
-                    if constexpr (NDIM == 3 && !LEVEL0) {
+                    if constexpr (!FORMS) {
+                        it = tile_dir<NDIM, RS, LEVEL0>(T, P, prim, uold, p, c, idim, kd0, kd1, dt, D, K, f, calls);
+                        ok = true;
+                    } else {
                         if (K.fast && (k0 == K_GHOST || k0 == K_ZERO) && (k1 == K_GHOST || k1 == K_ZERO) &&
-                            D.dx > 0x1p-60 && D.dx < 0x1p60) {
+                            forms_take(D.dx)) {
                             if (D.pow2)
                                 ok = tile_dir_fast<NDIM, RS, true>(T, P, prim, I, c, idim, k0 == K_ZERO, k1 == K_ZERO, dt,
                                                                    D, K, f, it);
@@ -512,10 +538,9 @@ __global__ void __launch_bounds__(TILE * NDIM * R, MINB)
                     if (ok) {
 #pragma unroll
                         for (int k = 0; k < 2 * NV; ++k) out[(size_t)k * nc] = f[k / NV][k % NV];
-                        calls += (k0 != K_ZERO) + (k1 != K_ZERO);
-                    } else {
-                        it = tile_dir_plain<NDIM, RS, LEVEL0>(T, P, prim, uold, p, c, idim, kd0, kd1, dt, D, K, flux,
-                                                              &calls);
+                        if (FORMS) calls += (k0 != K_ZERO) + (k1 != K_ZERO);
+                    } else if constexpr (FORMS) {
+                        it = tile_dir_plain<NDIM, RS>(T, P, prim, uold, p, c, idim, kd0, kd1, dt, D, K, out, &calls);
 #pragma unroll
                         for (int k = 0; k < 2 * NV; ++k) f[k / NV][k % NV] = out[(size_t)k * nc];
                     }
@@ -573,6 +598,10 @@ __global__ void __launch_bounds__(TILE * NDIM * R, MINB)
 #define RG_FACE_VARIANTS(X) X(0, 1, 6) X(1, 1, 8) X(2, 1, 10) X(3, 1, 9) X(4, 2, 4) X(5, 2, 5) X(6, 2, 6)
 constexpr int kFirstPipeVariant = 7;
 constexpr int kFirstBrickVariant = 9;  // 9, 10: brick kernel (rg_face_brick.cuh), lattice levels only
+// does the level take the brick face kernel (with refined cells: in the branch-free forms only)?
+inline bool brick_shapes(const Plan& P, const StepK& K) {
+    return P.nbox > 0 ? P.box_lattice != 0 : P.lattice != 0 && (K.fast || !P.lat_mask);
+}
 constexpr int kNumFaceVariants = 11;
 constexpr int kDefaultFaceVariant = 1;
 // Ensemble levels (per-box dt and dx read per cell) instantiate only the
@@ -583,10 +612,10 @@ inline bool boxed_variant_distinct(int v) {
     return v == kDefaultFaceVariant || v == kBoxedAltVariant || v == kFirstPipeVariant || v == kFirstBrickVariant;
 }
 
-template <int NDIM, int RS, int R, int MINB, bool BOXED = false, bool LEVEL0 = false>
-int launch_face_one(rg_ctx* c, const Plan& P, const StepK& K, int batch, const double* uold, const double* prim,
+template <int NDIM, int RS, int R, int MINB, bool BOXED = false, bool LEVEL0, bool FORMS>
+int launch_face_kernel(rg_ctx* c, const Plan& P, const StepK& K, int batch, const double* uold, const double* prim,
                     double* flux, double* fsum) {
-    auto kern = k_face_tiles<NDIM, RS, R, MINB, BOXED, LEVEL0>;
+    auto kern = k_face_tiles<NDIM, RS, R, MINB, BOXED, LEVEL0, FORMS>;
     const int block = TILE * NDIM * R;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0);
@@ -604,6 +633,20 @@ int launch_face_one(rg_ctx* c, const Plan& P, const StepK& K, int batch, const d
     if (grid < 1) grid = 1;
     kern<<<grid, block, 0, c->stream>>>(tree_view(c), P.view(), prim, uold, flux, fsum, c->d_status, K, batch);
     return check_cuda(c, cudaGetLastError(), "face kernel");
+}
+
+// Where the slope and interpolation types have no branch-free forms the exact
+// solver takes an instance of its own (its plain form as a call for every cell:
+// 128^3 cells with slope type 7, default shape, 2005 us a substep instead of
+// 1612); the other solvers' calls cost nothing measurable.
+template <int NDIM, int RS, int R, int MINB, bool BOXED = false, bool LEVEL0 = false>
+int launch_face_one(rg_ctx* c, const Plan& P, const StepK& K, int batch, const double* uold, const double* prim,
+                    double* flux, double* fsum) {
+    constexpr bool FORMS = NDIM == 3 && !LEVEL0;
+    if constexpr (FORMS && RS == RG_RIEMANN_EXACT)
+        if (!K.fast)
+            return launch_face_kernel<NDIM, RS, R, MINB, BOXED, LEVEL0, false>(c, P, K, batch, uold, prim, flux, fsum);
+    return launch_face_kernel<NDIM, RS, R, MINB, BOXED, LEVEL0, FORMS>(c, P, K, batch, uold, prim, flux, fsum);
 }
 
 template <int NDIM, int RS>

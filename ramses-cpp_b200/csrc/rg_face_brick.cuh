@@ -31,7 +31,7 @@ constexpr size_t BRICK_SMEM = sizeof(double) * 5 * BSITES;  // 69,120 bytes (3D:
 // own flux sum in slot order.  FORMS: this instance has the branch-free forms
 // (fast: the brick's values allow them); without, the plain ones are in line.
 // zero: bit s set where slot s faces a refined cell and carries no flux.
-template <int RS, bool FORMS, bool POW2>
+template <int RS, bool FORMS, bool POW2, bool FLOOR, bool CHK>
 __device__ __forceinline__ void brick_cell(const double* sq, int site, int p, int nc, bool ghost, bool fast, double dt,
                                            const DxDiv& D, const FastStep& S, const FastStep& Sc, const StepK& K,
                                            unsigned zero, double* __restrict__ flux, double* __restrict__ fsum,
@@ -49,7 +49,7 @@ __device__ __forceinline__ void brick_cell(const double* sq, int site, int p, in
         const unsigned none = (zero >> (2 * idim)) & 3u;
         if constexpr (FORMS) {
             bool ok = false;
-            if (fast) ok = brick_dir_fast<RS, POW2, BSITES>(sq, site, idim, stride, S, Sc, K, f[0], f[1], it);
+            if (fast) ok = brick_dir_fast<RS, POW2, FLOOR, BSITES, CHK>(sq, site, idim, stride, S, Sc, K, f[0], f[1], it);
             if (!ok || none) {
                 double g[2 * NV];  // (the call's array lives in memory, the loop's in registers)
                 it = brick_dir_plain<RS, BSITES>(sq, site, idim, stride, none, ghost, dt, D, K, g);
@@ -57,7 +57,7 @@ __device__ __forceinline__ void brick_cell(const double* sq, int site, int p, in
                 for (int k = 0; k < 2 * NV; ++k) f[k / NV][k % NV] = g[k];
             }
         } else {
-            it = brick_dir<RS, BSITES>(sq, site, idim, stride, none, ghost, dt, D, K, f[0]);
+            it = brick_dir<RS, BSITES>(sq, site, idim, stride, 0u, ghost, dt, D, K, f[0]);
         }
 #pragma unroll
         for (int k = 0; k < 2 * NV; ++k) out[(size_t)k * nc] = f[k / NV][k % NV];
@@ -80,8 +80,12 @@ __device__ __forceinline__ void brick_cell(const double* sq, int site, int p, in
 // straight line, so the two Riemann problems of a direction overlap.  Lanes
 // of a half-warp take rows y and y + 2 of the brick: rows are 12 doubles
 // apart, so the 16 lanes meet 16 different 8-byte banks.
-template <int RS, bool BOXED, bool FORMS>
-__device__ __forceinline__ void brick_face(const PlanView& P, const BrickGeom& G, const int* __restrict__ lat_id,
+//
+// FLOOR: in the forms with floors; without, false (and nothing done) if the
+// level or the brick's values need those or the plain ones.  VOTE: the block
+// looks at the staged states, not each cell.
+template <int RS, bool BOXED, bool FORMS, bool FLOOR, bool VOTE>
+__device__ __forceinline__ bool brick_face(const PlanView& P, const BrickGeom& G, const int* __restrict__ lat_id,
                                            const int* __restrict__ lat_p, const uint8_t* __restrict__ lat_mask,
                                            int kind, const double* __restrict__ prim, size_t ncell,
                                            double* __restrict__ flux, double* __restrict__ fsum, const DevStatus* st, const StepK& K, int brick, double* sq,
@@ -121,15 +125,15 @@ __device__ __forceinline__ void brick_face(const PlanView& P, const BrickGeom& G
 #pragma unroll
         for (int iv = 0; iv < NV; ++iv) {
             const double v = __ldg(prim + iv * ncell + id);
-            if (FORMS) C.up(v);
+            if (FORMS && VOTE) C.up(v);
             sq[iv * BSITES + t] = v;
         }
-        if (FORMS) C.gas(sq[t], sq[4 * BSITES + t]);
+        if (FORMS && VOTE && !FLOOR) C.gas(sq[t], sq[4 * BSITES + t]);
     }
     const int nc = P.ncells;
     const bool ghost = (kind & KIND_MASK) == K_GHOST;
-    // cell sizes of 2^-60 .. 2^60 keep the slopes' quotients in range
-    const bool fast = __syncthreads_and(!FORMS || (C.top_ok() && C.gas_ok())) && ghost && D.dx > 0x1p-60 && D.dx < 0x1p60;
+    const bool fast = __syncthreads_and(!FORMS || !VOTE || (C.top_ok() && (FLOOR || C.gas_ok()))) && ghost && forms_take(D.dx);
+    if (FORMS && !FLOOR && !fast) return false;
     const FastStep S = fast_step(dt, D.dx, D.inv), Sc = fast_step(dt, 2.0 * D.dx, 0.5 * D.inv);
     unsigned it = 0, done = 0;
     for (int u = threadIdx.x; u < BRICK * BRICK * BRICK; u += blockDim.x) {
@@ -137,27 +141,52 @@ __device__ __forceinline__ void brick_face(const PlanView& P, const BrickGeom& G
         const int y = ((u >> 4) & 1) | ((u >> 2) & 2) | ((u >> 3) & 4);
         const int site = (x + BHALO) + BSIDE * ((y + BHALO) + BSIDE * (z + BHALO));
         const size_t g = (size_t)(bx * BRICK + x) + (size_t)ex * ((size_t)(by * BRICK + y) + (size_t)ey * (bz * BRICK + z));
-        const unsigned zero = lat_mask ? lat_mask[g] : 0u;
+        const unsigned zero = FORMS && lat_mask ? lat_mask[g] : 0u;
         if (zero & LAT_REFINED) continue;
         const int p = lat_p[g];
         if (!FORMS || D.pow2)
-            brick_cell<RS, FORMS, true>(sq, site, p, nc, ghost, fast, dt, D, S, Sc, K, zero, flux, fsum, it);
-        else brick_cell<RS, FORMS, false>(sq, site, p, nc, ghost, fast, dt, D, S, Sc, K, zero, flux, fsum, it);
+            brick_cell<RS, FORMS, true, FLOOR, !VOTE>(sq, site, p, nc, ghost, fast, dt, D, S, Sc, K, zero, flux, fsum, it);
+        else brick_cell<RS, FORMS, false, FLOOR, !VOTE>(sq, site, p, nc, ghost, fast, dt, D, S, Sc, K, zero, flux, fsum, it);
         done += 6 - __popc(zero);
     }
     iters += it;
     calls += done;
+    return true;
+}
+
+// A brick the forms without floors do not cover, from its staging on.
+template <int RS, bool BOXED>
+__device__ __noinline__ void brick_face_floor(const PlanView& P, const BrickGeom& G, const int* lat_id, const int* lat_p,
+                                              const uint8_t* lat_mask, int kind, const double* prim, size_t ncell,
+                                              double* flux, double* fsum, const DevStatus* st, const StepK& K, int brick,
+                                              double* sq, unsigned long long* count) {
+    unsigned long long iters = 0, calls = 0;
+    brick_face<RS, BOXED, true, true, false>(P, G, lat_id, lat_p, lat_mask, kind, prim, ncell, flux, fsum, st, K, brick, sq, iters,
+                                      calls);
+    count[0] = iters;
+    count[1] = calls;
 }
 
 template <int RS, int MINB, bool BOXED, bool FORMS>
 __global__ void __launch_bounds__(BRICK_THREADS, MINB)
-    k_face_brick(PlanView P, BrickGeom G, const int* __restrict__ lat_id, const int* __restrict__ lat_p,
+    k_face_brick(const __grid_constant__ PlanView P, const __grid_constant__ BrickGeom G, const int* __restrict__ lat_id, const int* __restrict__ lat_p,
                  const uint8_t* __restrict__ lat_mask, int kind, const double* __restrict__ prim, size_t ncell, double* __restrict__ flux,
                  double* __restrict__ fsum, DevStatus* st, const __grid_constant__ StepK K) {
     extern __shared__ __align__(16) double sq[];  // [NV][BSITES]
     unsigned long long iters = 0, calls = 0;
-    brick_face<RS, BOXED, FORMS>(P, G, lat_id, lat_p, lat_mask, kind, prim, ncell, flux, fsum, st, K, (int)blockIdx.x, sq, iters,
-                          calls);
+    if constexpr (FORMS && RS == RG_RIEMANN_HLLC) {
+        if (!brick_face<RS, BOXED, true, false, true>(P, G, lat_id, lat_p, lat_mask, kind, prim, ncell, flux, fsum, st, K,
+                                                      (int)blockIdx.x, sq, iters, calls)) {
+            unsigned long long count[2];
+            brick_face_floor<RS, BOXED>(P, G, lat_id, lat_p, lat_mask, kind, prim, ncell, flux, fsum, st, K,
+                                        (int)blockIdx.x, sq, count);
+            iters = count[0];
+            calls = count[1];
+        }
+    } else {
+        brick_face<RS, BOXED, FORMS, true, true>(P, G, lat_id, lat_p, lat_mask, kind, prim, ncell, flux, fsum, st, K,
+                                                 (int)blockIdx.x, sq, iters, calls);
+    }
     if (RS == RG_RIEMANN_EXACT) {
         for (int o = 16; o > 0; o >>= 1) {
             iters += __shfl_xor_sync(0xffffffffu, iters, o);

@@ -58,25 +58,31 @@ __device__ __forceinline__ double sqrt_fast(double x) {
 }
 
 // Operand checks, gathered: magnitudes below 2^170 (finite with them) by the
-// largest high word, numerators zero or above 2^-800 by the smallest (0 wraps
-// to the top; a nonzero low word counts), so that with divisors in [2^-140,
-// 2^700] no step of a quotient over- or underflows.
+// largest high word, numerators zero or above 2^-560 by the smallest (0 wraps
+// to the top; a nonzero low word counts).  The divisors lie between 2^-67 (a
+// pressure + 1e-20) and 2^410 (the HLLC's sum of density times wave speed, the
+// density below 2^235 by gas()), or 2^600 in the exact solver, whose
+// numerators there are above 2^-240; so no step of a quotient over- or
+// underflows, and the remainder of the correction is exact.
 //
-// gas(): a density below 2^30 with a pressure of at least 2^-36.  Then neither
-// pressure floor (density times 1e-20 / gamma or 1e-20) nor the floor of the
-// squared sound speed (1e-20) can act, gamma being above 1, and the forms
-// leave the floors out; gas below that takes the plain forms.
+// gas(): a pressure of at least 2^-64 times the density, from the difference
+// of the high words (an exponent and the mantissa's leading bits: the ratio's
+// logarithm within 0.1).  Then neither pressure floor (density times 1e-20 /
+// gamma or 1e-20) nor the floor of the squared sound speed (1e-20) can act,
+// gamma being above 1, and the forms leave the floors out; gas below that (a
+// flow so fast that its thermal energy is lost in the rounding of the total,
+// say) takes the forms with floors in the brick kernels, the plain ones
+// elsewhere.  The bias keeps the difference positive for pressures below 2^170 over
+// densities from 1e-10 on; a negative pressure's is far above the limit.
 struct Check {
-    static constexpr unsigned kTop = (1023u + 170u) << 20, kBottom = (1023u - 800u) << 20;
-    static constexpr int kDense = (1023 + 30) << 20, kThin = (1023 - 36) << 20;
-    unsigned mx = 0, mn = 0xffffffffu;
-    int dense = 0, thin = 0x7fffffff;
+    static constexpr unsigned kTop = (1023u + 170u) << 20, kBottom = (1023u - 560u) << 20;
+    static constexpr unsigned kBias = 204u << 20, kCold = kBias + (64u << 20);
+    unsigned mx = 0, mn = 0xffffffffu, cold = 0;
     __device__ __forceinline__ void gas(double r, double p) {
-        dense = max(dense, __double2hiint(r));
-        thin = min(thin, __double2hiint(p));
+        cold = max(cold, (unsigned)__double2hiint(r) - (unsigned)__double2hiint(p) + kBias);
         up(p);
     }
-    __device__ __forceinline__ bool gas_ok() const { return dense < kDense && thin >= kThin; }
+    __device__ __forceinline__ bool gas_ok() const { return cold < kCold; }
     __device__ __forceinline__ void up(double x) { mx = max(mx, (unsigned)__double2hiint(x) & 0x7fffffffu); }
     __device__ __forceinline__ void num(double a) {
         const unsigned h = ((unsigned)__double2hiint(a) & 0x7fffffffu) | min((unsigned)__double2loint(a), 1u);
@@ -108,6 +114,9 @@ __device__ __forceinline__ double limited(double ql, double qc, double qr, const
     return l * r > 0.0 ? m : 0.0;
 }
 
+// Cell sizes that keep the slopes' quotients in range.
+__device__ __forceinline__ bool forms_take(double dx) { return dx > 0x1p-60 && dx < 0x1p60; }
+
 // Values of a step the branch-free forms share (per cell size).
 struct FastStep {
     double hdt, hdt0;       // dt / 2, and times zero: the tangential source term
@@ -120,9 +129,10 @@ __device__ __forceinline__ FastStep fast_step(double dt, double dx, double inv) 
 
 // compute_slopes / ghost slopes and trace of a rotated state: the upper face
 // state in qm, the lower in qp (either may be left out).  Primitive states:
-// their density is at least 1e-10 (ctoprim).  Without CHK the caller has
-// checked the states (top_ok and gas_ok).
-template <int NDIM, bool POW2, bool CHK, bool QM, bool QP>
+// their density is at least 1e-10 (ctoprim).  The caller has checked the gas
+// (gas_ok) and, without CHK, the states (top_ok); FLOOR: with the pressure
+// floors, for gas that gas_ok refuses.
+template <int NDIM, bool POW2, bool CHK, bool QM, bool QP, bool FLOOR = false>
 __device__ __forceinline__ void trace_fast(const double* q, const double* ql, const double* qr, const Limiter& L,
                                            const FastStep& S, double gamma, double* qm, double* qp, Check& C) {
     constexpr int NV = Dims<NDIM>::NV, IP = Dims<NDIM>::IP;
@@ -137,14 +147,18 @@ __device__ __forceinline__ void trace_fast(const double* q, const double* ql, co
             dq[iv] = div_by(s, S.dx, S.inv);
         }
     }
-    const double r = q[0], u = q[1];
+    const double r = q[0], u = q[1], p = FLOOR ? smax(q[IP], r * 1e-20) : q[IP];
     const double y = rcp_fast(r);
     if (CHK) {
-        C.gas(r, q[IP]);
+        if (FLOOR) {
+            C.up(r);
+            C.up(p);
+        }
         C.up(dq[IP]);
     }
     C.num(dq[IP]);
-    const double cs2 = div_by(gamma * q[IP], r, y);
+    double cs2 = div_by(gamma * p, r, y);
+    if (FLOOR) cs2 = smax(cs2, 1e-20);
     const double ru = dq[1] * r;
     const double b[3] = {S.hdt * (-u * dq[0] - ru), S.hdt * (-u * dq[1] - div_by(dq[IP], r, y)),
                          S.hdt * (-u * dq[IP] - ru * cs2)};
@@ -189,29 +203,41 @@ __device__ __forceinline__ void flux_cons(const double* q, const FastGas& G, dou
     u[IP] = E;
 }
 
-template <int NDIM>
+template <int NDIM, bool FLOOR = false>
 __device__ __forceinline__ double cs2_fast(const double* q, const FastGas& G, Check& C) {
     constexpr int IP = Dims<NDIM>::IP;
-    C.gas(q[0], q[IP]);
-    C.up(q[1]);
-    return div_by(G.gamma * q[IP], q[0], rcp_fast(q[0]));
+    if (!FLOOR) {
+        C.up(q[1]);
+        C.gas(q[0], q[IP]);
+    }
+    const double c2 = div_by(G.gamma * q[IP], q[0], rcp_fast(q[0]));
+    return FLOOR ? smax(c2, 1e-20) : c2;
+}
+// Do the checks of a solver's states hold?  With floors the energies of both
+// sides, which flux_cons checks, bound velocity and pressure; and a traced
+// pressure is zero or above 2^-220, the state's being at least its floor.
+template <bool FLOOR>
+__device__ __forceinline__ bool states_ok(const Check& C) {
+    return C.top_ok() && (FLOOR || C.gas_ok());
 }
 
 // The Riemann solvers on traced states (their density is at least 1e-10 by
 // the trace's floor).  False: take the plain form.
-template <int NDIM>
+template <int NDIM, bool FLOOR = false>
 __device__ __forceinline__ bool hllc_fast(const double* ql, const double* qr, double* f, const FastGas& G) {
     constexpr int NV = Dims<NDIM>::NV, IP = Dims<NDIM>::IP;
     Check C;
-    const double rl = ql[0], ul = ql[1], pl = ql[IP], rr = qr[0], ur = qr[1], pr = qr[IP];
+    const double rl = ql[0], ul = ql[1], pl = FLOOR ? smax(ql[IP], rl * G.smallp) : ql[IP];
+    const double rr = qr[0], ur = qr[1], pr = FLOOR ? smax(qr[IP], rr * G.smallp) : qr[IP];
     // the larger of two roots is the root of the larger: one root, same bits
-    const double c2l = cs2_fast<NDIM>(ql, G, C), c2r = cs2_fast<NDIM>(qr, G, C);
+    const double c2l = cs2_fast<NDIM, FLOOR>(ql, G, C), c2r = cs2_fast<NDIM, FLOOR>(qr, G, C);
     const double cmax = sqrt_fast(smax(c2l, c2r));
     const double sl = smin(ul, ur) - cmax, sr = smax(ul, ur) + cmax;
     const double rcl = rl * (ul - sl), rcr = rr * (sr - ur), div = rcr + rcl;
     const double nu = rcr * ur + rcl * ul + (pl - pr), np = rcr * pl + rcl * pr + rcl * rcr * (ul - ur);
     const double yd = rcp_fast(div);
-    const double ustar = div_by(nu, div, yd);  // (its clamp to +-1e6 and that of den: checked below)
+    double ustar = div_by(nu, div, yd);  // (without floors its clamp to +-1e6 and that of den are checked below)
+    if (FLOOR) ustar = smax(-1e6, smin(1e6, ustar));
     const double pstar = smax(div_by(np, div, yd), 0.0);
     const bool supl = sl > 0.0, supr = sr < 0.0, star = !(supl || supr);
     const bool left = supl || (!supr && ustar > 0.0);
@@ -219,18 +245,34 @@ __device__ __forceinline__ bool hllc_fast(const double* ql, const double* qr, do
 #pragma unroll
     for (int iv = 0; iv < NV; ++iv) q[iv] = left ? ql[iv] : qr[iv];
     flux_cons<NDIM>(q, G, f, u0, C);
-    const bool base_ok = C.top_ok() && C.gas_ok();
+    if (FLOOR) {
+        C.up(rl);
+        C.up(rr);
+    }
+    // nearly equal slow states (their density times wave speed below 1e-5): the mean of the two fluxes
+    const bool mean = FLOOR && star && div < 1e-5;
+    double fm[NV];
+    if (FLOOR) {
+        double qo[NV], uo[NV];
+#pragma unroll
+        for (int iv = 0; iv < NV; ++iv) qo[iv] = left ? qr[iv] : ql[iv];
+        flux_cons<NDIM>(qo, G, fm, uo, C);
+#pragma unroll
+        for (int iv = 0; iv < NV; ++iv) fm[iv] = 0.5 * (f[iv] + fm[iv]);
+    }
+    const bool base_ok = states_ok<FLOOR>(C);
     Check D;
     D.num(nu);
     D.num(np);
     const double so = left ? sl : sr;
-    const double den = so - ustar;
-    const bool den_ok = (__double2hiint(den) ^ (left ? (int)0x80000000 : 0)) > __double2hiint(1e-10);
-    const bool ustar_ok = (__double2hiint(ustar) & 0x7fffffff) < __double2hiint(1e6);
+    double den = so - ustar;
+    if (FLOOR) den = left ? smin(den, -1e-10) : smax(den, 1e-10);
+    const bool den_ok = FLOOR || (__double2hiint(den) ^ (left ? (int)0x80000000 : 0)) > __double2hiint(1e-10);
+    const bool ustar_ok = FLOOR || (__double2hiint(ustar) & 0x7fffffff) < __double2hiint(1e6);
     const double yn = rcp_fast(den);
     const double w = so - q[1];
     const double rstar = div_by(q[0] * w, den, yn);
-    const double ne = w * u0[IP] - q[IP] * q[1] + pstar * ustar;
+    const double ne = w * u0[IP] - (FLOOR ? (left ? pl : pr) : q[IP]) * q[1] + pstar * ustar;
     D.num(ne);
     double us[NV];
     us[0] = rstar;
@@ -242,37 +284,38 @@ __device__ __forceinline__ bool hllc_fast(const double* ql, const double* qr, do
     for (int iv = 0; iv < NV; ++iv) {
         const double fs = f[iv] + so * (us[iv] - u0[iv]);
         f[iv] = star ? fs : f[iv];
+        if (FLOOR && mean) f[iv] = fm[iv];
     }
-    return base_ok && (!star || (D.num_ok() && den_ok && ustar_ok && !(div < 1e-5)));
+    return base_ok && (!star || mean || (D.num_ok() && den_ok && ustar_ok && !(div < 1e-5)));
 }
 
-template <int NDIM>
+template <int NDIM, bool FLOOR = false>
 __device__ __forceinline__ bool llf_fast(const double* ql, const double* qr, double* f, const FastGas& G) {
     constexpr int NV = Dims<NDIM>::NV;
     Check C;
     double fl[NV], fr[NV], ul[NV], ur[NV];
     flux_cons<NDIM>(ql, G, fl, ul, C);
     flux_cons<NDIM>(qr, G, fr, ur, C);
-    const double al = sqrt_fast(cs2_fast<NDIM>(ql, G, C)), ar = sqrt_fast(cs2_fast<NDIM>(qr, G, C));
+    const double al = sqrt_fast(cs2_fast<NDIM, FLOOR>(ql, G, C)), ar = sqrt_fast(cs2_fast<NDIM, FLOOR>(qr, G, C));
     const double ha = 0.5 * smax(fabs(ql[1]) + al, fabs(qr[1]) + ar);
 #pragma unroll
     for (int i = 0; i < NV; ++i) f[i] = 0.5 * (fl[i] + fr[i]) - ha * (ur[i] - ul[i]);
-    return C.top_ok() && C.gas_ok();
+    return states_ok<FLOOR>(C);
 }
 
-template <int NDIM>
+template <int NDIM, bool FLOOR = false>
 __device__ __forceinline__ bool hll_fast(const double* ql, const double* qr, double* f, const FastGas& G) {
     constexpr int NV = Dims<NDIM>::NV;
     Check C;
     double fl[NV], fr[NV], ul[NV], ur[NV];
     flux_cons<NDIM>(ql, G, fl, ul, C);
     flux_cons<NDIM>(qr, G, fr, ur, C);
-    const double al = sqrt_fast(cs2_fast<NDIM>(ql, G, C)), ar = sqrt_fast(cs2_fast<NDIM>(qr, G, C));
+    const double al = sqrt_fast(cs2_fast<NDIM, FLOOR>(ql, G, C)), ar = sqrt_fast(cs2_fast<NDIM, FLOOR>(qr, G, C));
     const double sl = smin(0.0, smin(ql[1] - al, qr[1] - ar)), sr = smax(0.0, smax(ql[1] + al, qr[1] + ar));
     const double w = sr - sl, inv = div_by(1.0, w, rcp_fast(w));
 #pragma unroll
     for (int i = 0; i < NV; ++i) f[i] = (sr * fl[i] - sl * fr[i] + sr * sl * (ur[i] - ul[i])) * inv;
-    return C.top_ok() && C.gas_ok() && !(w < 1e-20);
+    return states_ok<FLOOR>(C) && !(w < 1e-20);
 }
 
 // One Newton update of the two-shock solver (RiemannSolver.cpp:221-233).

@@ -205,7 +205,7 @@ __device__ __forceinline__ bool prim_cfl(const double* u, double* q, double dx, 
     Check C;
 #pragma unroll
     for (int iv = 0; iv < NV; ++iv) C.up(u[iv]);
-    if (!(C.top_ok() && G.fast && dx > 0x1p-60 && dx < 0x1p60)) {
+    if (!(C.top_ok() && G.fast && forms_take(dx))) {
         if (PRIM) ctoprim<NDIM>(u, q, G.gamma, smalle);
         return CFL ? cfl_candidate<NDIM>(u, dx, G.gamma, F.cfl, F.cap, bits) : false;
     }

@@ -87,6 +87,7 @@ __device__ __forceinline__ bool line_flux_fast(const double* uc, const double* u
                                                const StepK& K, double* f, unsigned& it) {
     constexpr int NV = 3;
     Check C;
+    C.gas(qc[0], qc[2]);
     double qmo[NV], qpo[NV], far[NV], near[NV], qf[NV], qn[NV], qa[NV], qb[NV], qm[NV], qp[NV];
     trace_fast<1, POW2, true, true, true>(qc, ql, qr, K.own, S, K.gamma, qmo, qpo, C);
 #pragma unroll
@@ -105,6 +106,7 @@ __device__ __forceinline__ bool line_flux_fast(const double* uc, const double* u
     };
     prim(far, qf);
     prim(near, qn);
+    C.gas(qn[0], qn[2]);
 #pragma unroll
     for (int iv = 0; iv < NV; ++iv) {
         const double l = side ? qn[iv] - qc[iv] : qn[iv] - qf[iv], r = side ? qf[iv] - qn[iv] : qc[iv] - qn[iv];
@@ -158,7 +160,7 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLineThreads, 1)
     }
     const double inv = 1.0 / dx;
     const DxDiv D{dx, inv, is_pow2_with_normal_inverse(dx, inv)};
-    const bool fast = K.fast && K.interpol_var == 0 && dx > 0x1p-60 && dx < 0x1p60;
+    const bool fast = K.fast && K.interpol_var == 0 && forms_take(dx);
     const unsigned long long start_bits = (unsigned long long)__double_as_longlong(dt_start);
     unsigned long long word = st->dtmin_bits;
     double t = st->run_t, dt = 0.0;

@@ -1,9 +1,9 @@
 // rg_fast.cuh -- branch-free forms of the face step's arithmetic with the same bits.
 //
-// What bounds the face kernels is the latency of the FP64 chains and the
-// instructions around them, not the FP64 pipe (36 % busy in the brick kernel
-// at 16 warps per SM): every IEEE division and square root of the compiler
-// carries a branch to its slow path, and every early return of a Riemann
+// What bounds the face kernels in the plain forms is the latency of the FP64
+// chains and the instructions around them, not the FP64 pipe (36 % busy in the
+// brick face kernel at 16 warps per SM, 601 us at 128^3): every IEEE division
+// and square root of the compiler carries a branch to its slow path, and every early return of a Riemann
 // solver another, so nothing of a cell's two problems overlaps.  The forms
 // here have no branch: quotients and roots come from a Newton iteration and a
 // final correction that is correctly rounded for operands away from the ends
@@ -21,10 +21,11 @@
 // of correction (Markstein; Cornea, Harrison, Tang, "Scientific Computing on
 // Itanium-based Systems", ch. 7-8).  The seeds are the PTX approximations
 // (2^-19.9 and 2^-19.0 relative, measured), so one cubic step reaches 2^-57.
-// Against the IEEE operations: no difference on 3e10 pairs and roots,
-// divisors and quotients next to the hard cases among them, nor on the 844
-// roots within 2^-43 ulp of a rounding boundary.  The results do not carry the sign
-// of a negative zero numerator over a positive divisor; no numerator here can be one.
+// tests/test_gpu_fast_forms.py holds them to the IEEE operations on 2e9 random
+// pairs and roots, numerators of 2^-600 .. 2^600 over divisors of 2^-130 ..
+// 2^570, quotients, divisors and roots next to their hard cases among them.
+// The results do not carry the sign of a negative zero numerator over a positive
+// divisor; no numerator here can be one.
 #pragma once
 
 #include "rg_physics.cuh"

@@ -249,7 +249,10 @@ struct rg_ctx {
     double *d_uold = nullptr, *d_unew = nullptr, *d_prim = nullptr;
     bool have_state = false;
 
-    // scratch shared by all levels (levels run one after another on the stream)
+    // scratch shared by all levels (levels run one after another on the
+    // stream).  Between two substeps of a lattice level its start may hold the
+    // next one's primitives (DevStatus::prim_sel); a call that writes there
+    // sets next_level to -1.
     size_t cap_flux = 0;
     double* d_flux = nullptr;
     size_t cap_scan = 0;

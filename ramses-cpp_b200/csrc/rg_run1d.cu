@@ -10,8 +10,8 @@
 // of its cells and of one more on either side (so no flux travels), and after
 // the fold writes its edge cells into the neighbours' copies and its smallest
 // CFL candidates into every block's through distributed shared memory: one
-// cluster barrier a step.  A (cell, side) pair is one thread's work, a warp's
-// pairs are of one side.  Same functions on the same operands in the same
+// cluster barrier a step.  A (cell, side) pair is one thread's work, lower sides
+// first: the warps but the one where the sides meet have one side each.  Same functions on the same operands in the same
 // order as the level kernels, so the same bits.
 #include <cooperative_groups.h>
 
@@ -24,7 +24,7 @@ namespace {
 
 constexpr int kCta = 8;          // the portable cluster size
 constexpr int kLineHalo = 3;     // a cell's new state reaches three cells to either side
-constexpr int kLineThreads = 288;
+constexpr int kLineThreads = 288;  // nine warps: the 260 pairs of a 1024-cell line's piece in one round
 constexpr int kLineWarps = kLineThreads / 32;
 
 // Is the level one periodic line in list order?  Site i = 2 k + ic - 1 of the

@@ -502,8 +502,8 @@ def test_host_substeps_move_only_the_level(ctx_factory, oracle, memory):
 def test_level_run_matches_host_loop(ctx_factory, case):
     """rg_level_run against the host loop `while t < t_end: t += level_substep()`:
     same state bits, same time, same step count.  sod1d (1024 cells, the Sod
-    run of config 1 to t = 0.245) and sedov3d_small (8^3 = 512 cells) take the
-    single-block kernel; sedov3d (32^3) the graph with a device-side WHILE loop."""
+    run of config 1 to t = 0.245) takes the cluster kernel, sedov3d_small (8^3 =
+    512 cells) the single-block one; sedov3d (32^3) the graph with a device-side WHILE loop."""
     if case == "sedov3d_small":
         ndim, L, params, cap, t_end = 3, 3, make_params(3, slope_type=2, riemann="hllc"), False, 0.3
         g = rg_tree.build_uniform(3, L)

@@ -239,7 +239,7 @@ __device__ __forceinline__ bool step_brick(const PlanView& P, const BrickGeom& G
 // the pressure floor: 686 with both, 1065 with the plain forms behind those
 // without floors).  In the others the floors are a few comparisons, and what a
 // second copy does to the first one's registers costs more (LLF 456 with both,
-// 430 with floors everywhere).
+// 413 with floors everywhere).
 template <int RS, bool BOXED>
 __device__ __noinline__ void step_brick_floor(const PlanView& P, BrickGeom G, const int* lat_id, const int* lat_ord,
                                               int kind, double* prim0, double* prim1, size_t ncell, double* uold,

@@ -158,8 +158,8 @@ __device__ __forceinline__ void trace_fast(const double* q, const double* ql, co
         C.up(dq[IP]);
     }
     C.num(dq[IP]);
-    double cs2 = div_by(gamma * p, r, y);
-    if (FLOOR) cs2 = smax(cs2, 1e-20);
+    // (the floor of cs2, 1e-20, cannot act on a pressure of 1e-20 r or more: gamma - 1 is above 2^-20)
+    const double cs2 = div_by(gamma * p, r, y);
     const double ru = dq[1] * r;
     const double b[3] = {S.hdt * (-u * dq[0] - ru), S.hdt * (-u * dq[1] - div_by(dq[IP], r, y)),
                          S.hdt * (-u * dq[IP] - ru * cs2)};

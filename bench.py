@@ -41,7 +41,7 @@ Keys besides the contract's:
   the same window;
 - `parity`: the GPU run's uold and son after W+2 coarse steps against the
   reference's (SHA-1 digest, computed in the CPU baseline's process);
-- `sedov128` (config 2: the uniform 128^3 level, brick face kernel, its own
+- `sedov128` (config 2: the uniform 128^3 level, brick step kernel, its own
   rooflines), `newton` (config 5), `ensemble` (config 4), `amr_dropin`
   (the reference's own AmrGrid/TreeUpdater step with the GPU hydro drop-in),
   `sod1d` (config 1).
@@ -824,7 +824,7 @@ def _ensemble_box_oracle(index, steps):
 def ensemble_parity(local_rank, nbox=32, steps=3):
     """Config 4's parity check on a seeded, edge-stratified subset of the 512
     boxes (about the same number of boxes of every edge): the subset stepped
-    together on the GPU (per-box CFL, brick face kernel over the boxes'
+    together on the GPU (per-box CFL, brick step kernel over the boxes'
     lattices) against each box stepped alone by the C oracle, per-box state
     digests and dt bits compared."""
     import multiprocessing as mp
@@ -868,7 +868,7 @@ def ensemble_parity(local_rank, nbox=32, steps=3):
         same_dt += all(float(dts[k][i]) == want[s.index][1][k] for k in range(steps))
     return {"boxes": nbox, "edges": {str(e): sum(1 for s in subset if s.edge == e) for e in edges},
             "substeps": steps, "cells": int(f.cells), "bit_identical_boxes": same_state, "same_dt_boxes": same_dt,
-            "check": "GPU forest of the subset (brick face kernel, per-box CFL) against each box alone by the C oracle"}
+            "check": "GPU forest of the subset (brick step kernel, per-box CFL) against each box alone by the C oracle"}
 
 
 def amr_sample(variant, steps, lmin=7, lmax=10, ngridmax=400000):

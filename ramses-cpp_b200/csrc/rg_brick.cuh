@@ -38,16 +38,16 @@ struct BrickGeom {
 };
 
 // The two fluxes of one cell and direction in the plain forms, one trace of the
-// cell for both; sides in `none` (bit per side) carry no flux.  Returns the
-// Newton updates.  In line in the kernels without branch-free forms, a call
+// cell for both; sides in `none` (bit per side) carry no flux.  put(side, flux)
+// takes each as it is known.  Returns the Newton updates.  In line in the kernels without branch-free forms, a call
 // where those do not cover a cell: one per direction (a call per face formed
 // the cell's trace twice and took 1.3 times the two-kernel step's time where
 // every cell went that way), and without the forms with floors in it (what the
 // call may overwrite costs the loop around it also where it is not made: with
 // them k_brick_step took 474 instead of 434 us at 128^3).
-template <int RS, int SITES>
+template <int RS, int SITES, class Put>
 __device__ __forceinline__ unsigned brick_dir(const double* sq, int site, int idim, int stride, unsigned none, bool ghost,
-                                              double dt, const DxDiv& D, const StepK& K, double* f) {
+                                              double dt, const DxDiv& D, const StepK& K, Put put) {
     constexpr int NV = 5;
     const BrickPlanes<SITES> B(idim);
     double qc[NV], ql[NV], qr[NV], qmo[NV], qpo[NV];
@@ -62,7 +62,8 @@ __device__ __forceinline__ unsigned brick_dir(const double* sq, int site, int id
         double qn[NV], qfar[NV], qm[NV], qp[NV], g[NV];
         if ((none >> side) & 1u) {
 #pragma unroll
-            for (int iv = 0; iv < NV; ++iv) f[side * NV + iv] = 0.0;
+            for (int iv = 0; iv < NV; ++iv) g[iv] = 0.0;
+            put(side, g);
             continue;
         }
         B.load(sq, side ? site + stride : site - stride, qn);
@@ -73,15 +74,17 @@ __device__ __forceinline__ unsigned brick_dir(const double* sq, int site, int id
         else own_trace<3>(qn, qnl, qnr, dt, D, K, qm, qp);
         it += side == 0 ? riemann<3, RS>(qm, qpo, g, K) : riemann<3, RS>(qmo, qp, g, K);
         rot_swap<3>(g, idim);
-#pragma unroll
-        for (int iv = 0; iv < NV; ++iv) f[side * NV + iv] = g[iv];
+        put(side, g);
     }
     return it;
 }
 template <int RS, int SITES>
 __device__ __noinline__ unsigned brick_dir_plain(const double* sq, int site, int idim, int stride, unsigned none,
                                                  bool ghost, double dt, const DxDiv& D, const StepK& K, double* f) {
-    return brick_dir<RS, SITES>(sq, site, idim, stride, none, ghost, dt, D, K, f);
+    return brick_dir<RS, SITES>(sq, site, idim, stride, none, ghost, dt, D, K, [&](int side, const double* g) {
+#pragma unroll
+        for (int iv = 0; iv < 5; ++iv) f[side * 5 + iv] = g[iv];
+    });
 }
 
 // The flux of one cell through one face in the plain forms; `stride` is the

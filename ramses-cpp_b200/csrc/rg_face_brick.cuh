@@ -42,12 +42,12 @@ __device__ __forceinline__ void brick_cell(const double* sq, int site, int p, in
     for (int iv = 0; iv < NV; ++iv) fs[iv] = 0.0;
 #pragma unroll 1
     for (int idim = 0; idim < 3; ++idim) {
-        double f[2][NV];
         double* out = flux + (size_t)(2 * idim * NV) * nc + p;
         unsigned it = 0;
         const int stride = idim == 0 ? 1 : (idim == 1 ? BSIDE : BSIDE * BSIDE);
-        const unsigned none = (zero >> (2 * idim)) & 3u;
         if constexpr (FORMS) {
+            const unsigned none = (zero >> (2 * idim)) & 3u;
+            double f[2][NV];
             bool ok = false;
             if (fast) ok = brick_dir_fast<RS, POW2, FLOOR, BSITES, CHK>(sq, site, idim, stride, S, Sc, K, f[0], f[1], it);
             if (!ok || none) {
@@ -56,14 +56,21 @@ __device__ __forceinline__ void brick_cell(const double* sq, int site, int p, in
 #pragma unroll
                 for (int k = 0; k < 2 * NV; ++k) f[k / NV][k % NV] = g[k];
             }
+#pragma unroll
+            for (int k = 0; k < 2 * NV; ++k) out[(size_t)k * nc] = f[k / NV][k % NV];
+#pragma unroll
+            for (int iv = 0; iv < NV; ++iv) fs[iv] = (fs[iv] + f[0][iv]) - f[1][iv];
         } else {
-            it = brick_dir<RS, BSITES>(sq, site, idim, stride, 0u, ghost, dt, D, K, f[0]);
+            // each flux is stored before the next is solved: its registers are free then
+            it = brick_dir<RS, BSITES>(sq, site, idim, stride, 0u, ghost, dt, D, K, [&](int side, const double* g) {
+#pragma unroll
+                for (int iv = 0; iv < NV; ++iv) {
+                    out[(size_t)(side * NV + iv) * nc] = g[iv];
+                    fs[iv] = side ? fs[iv] - g[iv] : fs[iv] + g[iv];
+                }
+            });
         }
-#pragma unroll
-        for (int k = 0; k < 2 * NV; ++k) out[(size_t)k * nc] = f[k / NV][k % NV];
         iters += it;
-#pragma unroll
-        for (int iv = 0; iv < NV; ++iv) fs[iv] = (fs[iv] + f[0][iv]) - f[1][iv];
     }
 #pragma unroll
     for (int iv = 0; iv < NV; ++iv) fsum[(size_t)iv * nc + p] = fs[iv];
